@@ -245,7 +245,7 @@ __host__ __device__ __forceinline__ void sb_block_geom(int b, int& x, int& y, in
   const int sq = b / 5, kind = b % 5;
   const int level = sq >= 21 ? 3 : sq >= 5 ? 2 : sq >= 1 ? 1 : 0;
   const int idx = sq - sb_level_offset(level), n = 1 << level, size = 64 >> level, half = size / 2;
-  const int sx = (idx % n) * size, sy = (idx / n) * size;
+  const int sx = (idx & (n - 1)) * size, sy = (idx >> level) * size;
   x = sx, y = sy, w = size, h = size;
   if (kind == 1 || kind == 2) h = half, y = sy + (kind == 2 ? half : 0);
   if (kind == 3 || kind == 4) w = half, x = sx + (kind == 4 ? half : 0);

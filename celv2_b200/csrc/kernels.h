@@ -62,7 +62,8 @@ void launch_me_level(const FrameJob* jobs, const WorkList& w, int level, int cel
 int refine_units(int nrefs, int cols, int rows);
 void launch_me_refine(const FrameJob* jobs, const WorkList& w, cudaStream_t st);
 
-// Intra SATDs of every candidate block and mode. Units: sb_cols * sb_rows per job.
+// Intra SATDs of every candidate block and mode. Units: sb_cols * sb_rows per job (split further by the
+// launcher where they are few).
 void launch_intra(const FrameJob* jobs, const WorkList& w, cudaStream_t st);
 
 // Each reference's best candidate MV per candidate block, the distinct MVs of a superblock taken
