@@ -258,8 +258,10 @@ struct celv2_engine {
   // batch's records to cross PCIe); copied[p] marks buffer set p's copies done.
   cudaStream_t copy_st = nullptr;
   cudaStream_t up_st = nullptr;  // celv2_upload's stream (frame-store uploads)
+  cudaStream_t fin_st = nullptr;  // the finalize of a batch in slices (high priority; st waits for it)
+  cudaEvent_t slice_ready[8] = {}, slice_done[8] = {};  // per slice (kMaxSlices)
   static constexpr int kRecordSets = 3;
-  cudaEvent_t stages_done = nullptr, copied[kRecordSets] = {};
+  cudaEvent_t copied[kRecordSets] = {};
   bool copy_pending[kRecordSets] = {};
   int group_parity = 0;
   long long kernel_launches = 0;
@@ -274,9 +276,10 @@ struct celv2_engine {
   double stage_ms[kStages] = {};
   long long stage_n[kStages] = {};
   unsigned long long* stats = nullptr;  // device work counters (kStats), while timing
-  // stage work queues (device counters): [0..4] motion search levels, [5] intra, [6] inter,
-  // [7] finalize, [8] level 0's refinement, [9] inter by regions, of the main stream; [15]
-  // prepare's intra
+  // stage work queues (device counters): prepare's intra (its own stream); the motion-search levels
+  // and the refinement; per slice its intra, inter, inter by regions and finalize
+  static constexpr int kQueuePrep = 0, kQueueMe = 1, kQueueRefine = kQueueMe + kLevels, kQueueSlice = kQueueRefine + 1;
+  static constexpr int kMaxSlices = 8, kQueues = kQueueSlice + 4 * kMaxSlices;
   unsigned* queues = nullptr;
   bool persistent = true;      // the queue-draining persistent stage kernels (else one CTA per unit)
   unsigned persistent_off = 0; // stages (bit i: queue i) that run one CTA per unit anyway
@@ -338,6 +341,7 @@ struct celv2_engine {
     if (prep_st) cudaStreamSynchronize(prep_st);
     if (copy_st) cudaStreamSynchronize(copy_st);
     if (up_st) cudaStreamSynchronize(up_st);
+    if (fin_st) cudaStreamSynchronize(fin_st);
     free_graphs();
     for (Slot* s : store) free_slot(s);
     for (Slot& s : srcs) cudaFree(s.mem);
@@ -363,13 +367,17 @@ struct celv2_engine {
     for (cudaEvent_t e : ring_done)
       if (e) cudaEventDestroy(e);
     if (prep_done) cudaEventDestroy(prep_done);
-    if (stages_done) cudaEventDestroy(stages_done);
+    for (int i = 0; i < kMaxSlices; i++) {
+      if (slice_ready[i]) cudaEventDestroy(slice_ready[i]);
+      if (slice_done[i]) cudaEventDestroy(slice_done[i]);
+    }
     for (cudaEvent_t e : copied)
       if (e) cudaEventDestroy(e);
     if (st) cudaStreamDestroy(st);
     if (prep_st) cudaStreamDestroy(prep_st);
     if (copy_st) cudaStreamDestroy(copy_st);
     if (up_st) cudaStreamDestroy(up_st);
+    if (fin_st) cudaStreamDestroy(fin_st);
   }
 
   static void free_slot(Slot* s) {
@@ -413,10 +421,16 @@ struct celv2_engine {
     CK(cudaEventCreateWithFlags(&prep_done, cudaEventDisableTiming));
     CK(cudaStreamCreateWithFlags(&copy_st, cudaStreamNonBlocking));
     CK(cudaStreamCreateWithFlags(&up_st, cudaStreamNonBlocking));
-    CK(cudaEventCreateWithFlags(&stages_done, cudaEventDisableTiming));
     for (cudaEvent_t& e : copied) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     CK(cudaMalloc(&djobs, kRingJobs * sizeof(FrameJob)));
-    CK(cudaMalloc(&queues, 16 * sizeof(unsigned)));
+    CK(cudaMalloc(&queues, kQueues * sizeof(unsigned)));
+    int least = 0, greatest = 0;
+    CK(cudaDeviceGetStreamPriorityRange(&least, &greatest));
+    CK(cudaStreamCreateWithPriority(&fin_st, cudaStreamNonBlocking, greatest));
+    for (int i = 0; i < kMaxSlices; i++) {
+      CK(cudaEventCreateWithFlags(&slice_ready[i], cudaEventDisableTiming));
+      CK(cudaEventCreateWithFlags(&slice_done[i], cudaEventDisableTiming));
+    }
     CK(cudaMallocHost(&ring, (size_t)kRing * kRingJobs * sizeof(FrameJob)));
     for (cudaEvent_t& e : ring_done) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     alloc_buffers(single, false);
@@ -598,22 +612,73 @@ struct celv2_engine {
     ring_pending[i] = true;
   }
 
-  // Queues the stage kernels of the jobs whose descriptors are in djobs (intra for all of them
-  // or none); returns the kernels launched.
-  int enqueue_stages(const std::vector<FrameJob>& jobs, bool with_intra, cudaStream_t stream,
-                     const std::vector<NetJob>& nets) {
+  // ---- the stages of a batch ----
+  // Superblocks decided, and copied to the host, together (see run()).
+  struct Slice {
+    std::vector<SbRange> parts;
+    int sbs = 0;
+  };
+
+  // Rows of superblocks in decision order, cut into slices for the records' way to the host. A
+  // batch's records leave at PCIe speed only once its last stage has run, so a launch of many
+  // superblocks has its inter stage and finalize run slice by slice, the copies of one behind the
+  // stages of the next. A slice is worth it from kSliceSbs superblocks on: 5 MB, ~90 us of copy,
+  // against the ~30 us that the drained ends of its launches cost. Five 1080p leaves of 7 references
+  // in 1 / 2 / 3 / 5 / 8 slices: 7.81 / 7.78 / 7.25 / 6.83 / 6.70 ms; one masked 4K frame 3.30 / 3.17
+  // / 3.12 / 3.09 / 3.09; one 1080p frame of 7 references (4 slices at most) 2.27 / 2.11 / 2.15 /
+  // 2.17 / 2.15.
+  static constexpr int kSliceSbs = 128;
+  static std::vector<Slice> cut(const std::vector<SbRange>& rows, bool to_host) {
+    int total = 0;
+    for (const SbRange& r : rows) total += r.sbs;
+    const int n = to_host ? std::max(1, std::min(kMaxSlices, total / kSliceSbs)) : 1;
+    std::vector<Slice> out(1);
+    int done = 0;
+    for (const SbRange& r : rows) {
+      Slice* s = &out.back();
+      const bool joins = !s->parts.empty() && s->parts.back().job == r.job && s->parts.back().sb0 + s->parts.back().sbs == r.sb0;
+      if ((long long)done * n >= (long long)total * (long long)out.size() || (!joins && (int)s->parts.size() == kMaxJobs)) {
+        out.emplace_back();
+        s = &out.back();
+        s->parts.push_back(r);
+      } else if (joins) {
+        s->parts.back().sbs += r.sbs;
+      } else {
+        s->parts.push_back(r);
+      }
+      s->sbs += r.sbs, done += r.sbs;
+    }
+    return out;
+  }
+
+  // The rows of every job, job after job.
+  static std::vector<SbRange> rows_of(const std::vector<FrameJob>& jobs) {
+    std::vector<SbRange> rows;
+    for (int j = 0; j < (int)jobs.size(); j++)
+      for (int r = 0; r < jobs[j].sb_rows; r++) rows.push_back(SbRange{j, r * jobs[j].sb_cols, jobs[j].sb_cols});
+    return rows;
+  }
+
+  unsigned* queue(int stage_bit, int index) const {
+    return persistent && !(persistent_off >> stage_bit & 1) ? queues + index : nullptr;
+  }
+
+  // Queues the stages that come before the superblock stages, for the jobs whose descriptors are in
+  // djobs: motion search, the pruner between its levels 1 and 0, refinement; returns the kernels
+  // launched. Zeroes the work queues of the whole batch.
+  int enqueue_search(const std::vector<FrameJob>& jobs, cudaStream_t stream, const std::vector<NetJob>& nets) {
     const int n = (int)jobs.size();
     int launched = 0;
-    if (persistent) CK(cudaMemsetAsync(queues, 0, 10 * sizeof(unsigned), stream));
-    auto q = [&](int i) { return persistent && !(persistent_off >> i & 1) ? queues + i : nullptr; };
+    if (persistent) CK(cudaMemsetAsync(queues + kQueueMe, 0, (kQueues - kQueueMe) * sizeof(unsigned), stream));
     WorkList w{};
-    w.njobs = n;
+    w.nparts = n;
+    for (int j = 0; j < n; j++) w.part[j] = SbRange{j, 0, jobs[j].sb_cols * jobs[j].sb_rows};
     for (int l = kLevels - 1; l >= 0; l--) {
       for (int j = 0; j < n; j++)
         w.prefix[j + 1] = w.prefix[j] + me_units(jobs[j].nrefs, jobs[j].fcols[l], jobs[j].frows[l], me_cells[l]);
       if (l == 0 && !nets.empty())  // the learned pruner, from the level-1 motion search
         stage(kStPruner, stream, [&] { launched += enqueue_pruner(jobs, nets, stream); });
-      w.queue = q(l);
+      w.queue = queue(l, kQueueMe + l);
       if (w.prefix[n] > 0) {
         stage(kStMe0 - l, stream, [&] { launch_me_level(djobs, w, l, me_cells[l], stream); });
         launched++;
@@ -621,31 +686,48 @@ struct celv2_engine {
     }
     for (int j = 0; j < n; j++)
       w.prefix[j + 1] = w.prefix[j] + refine_units(jobs[j].nrefs, jobs[j].fcols[0], jobs[j].frows[0]);
-    w.queue = q(8);
+    w.queue = queue(8, kQueueRefine);
     if (w.prefix[n] > 0) {
       stage(kStRefine, stream, [&] { launch_me_refine(djobs, w, stream); });
       launched++;
     }
-    if (with_intra) {
-      for (int j = 0; j < n; j++) w.prefix[j + 1] = w.prefix[j] + jobs[j].sb_cols * jobs[j].sb_rows;
-      w.queue = q(5);
-      stage(kStIntra, stream, [&] { launch_intra(djobs, w, stream); });
-      launched++;
-    }
-    for (int j = 0; j < n; j++) w.prefix[j + 1] = w.prefix[j] + jobs[j].nrefs * jobs[j].sb_cols * jobs[j].sb_rows;
-    w.queue = q(6);
-    if (w.prefix[n] > 0) {
-      bool any_keep = false;
-      for (const FrameJob& jb : jobs) any_keep |= jb.keep != nullptr;
-      stage(kStInter, stream, [&] { launch_inter(djobs, w, inter_chunk, any_keep, q(9), stream); });
-      launched++;
-    }
-    for (int j = 0; j < n; j++) w.prefix[j + 1] = w.prefix[j] + jobs[j].sb_cols * jobs[j].sb_rows;
-    w.queue = q(7);
-    stage(kStFinalize, stream, [&] { launch_finalize(djobs, w, stream); });
-    launched++;
     CK(cudaGetLastError());
     return launched;
+  }
+
+  // The work list of a slice (a unit per superblock; inter: per superblock and reference).
+  static WorkList slice_list(const std::vector<FrameJob>& jobs, const Slice& s, bool per_ref, unsigned* q) {
+    WorkList w{};
+    w.nparts = (int)s.parts.size();
+    for (int p = 0; p < w.nparts; p++) {
+      w.part[p] = s.parts[p];
+      w.prefix[p + 1] = w.prefix[p] + s.parts[p].sbs * (per_ref ? jobs[s.parts[p].job].nrefs : 1);
+    }
+    w.queue = q;
+    return w;
+  }
+
+  // Slice i's intra, inter and finalize; each returns the kernels launched.
+  int enqueue_intra(const std::vector<FrameJob>& jobs, const Slice& s, int i, cudaStream_t stream) {
+    const WorkList w = slice_list(jobs, s, false, queue(5, kQueueSlice + 4 * i));
+    stage(kStIntra, stream, [&] { launch_intra(djobs, w, stream); });
+    return 1;
+  }
+  int enqueue_inter(const std::vector<FrameJob>& jobs, const Slice& s, int i, cudaStream_t stream) {
+    const WorkList w = slice_list(jobs, s, true, queue(6, kQueueSlice + 4 * i + 1));
+    if (w.prefix[w.nparts] <= 0) return 0;
+    bool any_keep = false;
+    for (const SbRange& r : s.parts) any_keep |= jobs[r.job].keep != nullptr;
+    stage(kStInter, stream, [&] {
+      launch_inter(djobs, w, inter_chunk, any_keep, queue(6, kQueueSlice + 4 * i + 2), stream);
+    });
+    return 1;
+  }
+  int enqueue_finalize(const std::vector<FrameJob>& jobs, const Slice& s, int i, cudaStream_t stream) {
+    const WorkList w = slice_list(jobs, s, false, queue(7, kQueueSlice + 4 * i + 3));
+    stage(kStFinalize, stream, [&] { launch_finalize(djobs, w, stream); });
+    CK(cudaGetLastError());
+    return 1;
   }
 
   // The pruner's features per job, then per job one kernel running the network on each
@@ -667,11 +749,57 @@ struct celv2_engine {
     return launched;
   }
 
-  // The stage kernels of the jobs, their descriptors sent through the pinned ring.
-  void run_stages(const std::vector<FrameJob>& jobs, bool with_intra, cudaStream_t stream,
-                  const std::vector<NetJob>& nets = {}) {
-    put_jobs(jobs.data(), (int)jobs.size(), djobs, stream);
-    kernel_launches += enqueue_stages(jobs, with_intra, stream, nets);
+  // Everything of a batch up to its slices: motion search, refinement, and intra (with_intra) unless
+  // the slices run it; of a batch in one slice also its inter stage and finalize. A batch without
+  // references has its intra in the slices: it is all the work there is before the records.
+  int enqueue_front(const std::vector<FrameJob>& jobs, bool with_intra, const std::vector<NetJob>& nets,
+                    const std::vector<Slice>& slices) {
+    int launched = enqueue_search(jobs, st, nets);
+    const bool whole = slices.size() == 1;
+    if (with_intra && (whole || any_refs(jobs))) {
+      Slice all;
+      for (int j = 0; j < (int)jobs.size(); j++) all.parts.push_back(SbRange{j, 0, jobs[j].sb_cols * jobs[j].sb_rows});
+      launched += enqueue_intra(jobs, all, 0, st);
+    }
+    if (whole) launched += enqueue_inter(jobs, slices[0], 0, st) + enqueue_finalize(jobs, slices[0], 0, st);
+    return launched;
+  }
+  static bool any_refs(const std::vector<FrameJob>& jobs) {
+    for (const FrameJob& j : jobs)
+      if (j.nrefs > 0) return true;
+    return false;
+  }
+
+  // The stages of a batch on st, its descriptors sent through the pinned ring (graph: the part up to
+  // the slices replayed as a CUDA graph). done(i, stream) is called once slice i's records are queued
+  // on `stream` -- to queue their copies. Several slices: the inter stage of one runs while the
+  // finalize of the one before it, on a stream of higher priority, takes the SMs the drained inter
+  // launch leaves; st waits for the last finalize.
+  template <typename F>
+  void run(const std::vector<FrameJob>& jobs, bool with_intra, const std::vector<NetJob>& nets,
+           const std::vector<Slice>& slices, bool graph, F&& done) {
+    if (graph) {
+      launch_graph(jobs, with_intra, nets, slices);
+    } else {
+      put_jobs(jobs.data(), (int)jobs.size(), djobs, st);
+      kernel_launches += enqueue_front(jobs, with_intra, nets, slices);
+    }
+    const int n = (int)slices.size();
+    if (n == 1) {
+      done(0, st);
+      return;
+    }
+    const bool intra_here = with_intra && !any_refs(jobs);
+    for (int i = 0; i < n; i++) {
+      if (intra_here) kernel_launches += enqueue_intra(jobs, slices[i], i, st);
+      kernel_launches += enqueue_inter(jobs, slices[i], i, st);
+      CK(cudaEventRecord(slice_ready[i], st));
+      CK(cudaStreamWaitEvent(fin_st, slice_ready[i], 0));
+      kernel_launches += enqueue_finalize(jobs, slices[i], i, fin_st);
+      CK(cudaEventRecord(slice_done[i], fin_st));
+      done(i, fin_st);
+    }
+    CK(cudaStreamWaitEvent(st, slice_done[n - 1], 0));
   }
 
   void wait_idle() {
@@ -731,26 +859,42 @@ struct celv2_engine {
       jobs[0].keep = put_keep(keep0, single, st);
       const std::vector<NetJob> nets{net_for(jobs[0], single, !keep0.empty())};
       if (nets[0].net) jobs[0].keep = single.keep;
-      run_stages(jobs, !prepared, st, nets);
-      mark_used(used, nrefs, st);
-      last_nrefs = nrefs;
       // rows back to the host in row-stream order
       const int streams = std::max(1, std::min(row_streams, g.sb_rows));
-      const int run = (g.sb_rows + streams - 1) / streams;
+      const int per = (g.sb_rows + streams - 1) / streams;
       order.clear();
-      for (int i = 0; i < run; i++)
+      for (int i = 0; i < per; i++)
         for (int s = 0; s < streams; s++)
-          if (s * run + i < g.sb_rows) order.push_back(s * run + i);
-      for (int r : order) {
-        const size_t first = (size_t)r * g.sb_cols;
-        CK(cudaMemcpyAsync(dest + first, single.out + first, g.sb_cols * sizeof(celv2_sb_out),
-                           cudaMemcpyDeviceToHost, st));
-        CK(cudaEventRecord(row_done[r], st));
-      }
+          if (s * per + i < g.sb_rows) order.push_back(s * per + i);
+      std::vector<SbRange> rows;
+      for (int r : order) rows.push_back(SbRange{0, r * g.sb_cols, g.sb_cols});
+      std::vector<Slice> slices = cut(rows, true);
+      if ((int)slices.size() > kMaxSlices) slices.assign(1, Slice{});
+      if (slices.size() == 1) slices[0].parts.assign(1, SbRange{0, 0, g.nsb}), slices[0].sbs = g.nsb;
+      size_t next = 0;  // the next row of `order` to copy
+      run(jobs, !prepared, nets, slices, false, [&](int i, cudaStream_t ready) {
+        // one slice: the copies follow on st; several: on copy_st, beside the next slices' stages
+        cudaStream_t cs = st;
+        if (ready != st) {
+          cs = copy_st;
+          CK(cudaStreamWaitEvent(cs, slice_done[i], 0));
+        }
+        for (int left = slices[i].sbs; left > 0; left -= g.sb_cols) {
+          const int r = order[next++];
+          const size_t first = (size_t)r * g.sb_cols;
+          CK(cudaMemcpyAsync(dest + first, single.out + first, g.sb_cols * sizeof(celv2_sb_out), cudaMemcpyDeviceToHost,
+                             cs));
+          CK(cudaEventRecord(row_done[r], cs));
+        }
+      });
+      mark_used(used, nrefs, st);
+      last_nrefs = nrefs;
       last_out = dest;
       pending = true;
     } catch (...) {
       cudaStreamSynchronize(st);  // a failure leaves no work running
+      cudaStreamSynchronize(fin_st);
+      cudaStreamSynchronize(copy_st);
       cudaStreamSynchronize(prep_st);
       pending = false;
       throw;
@@ -771,11 +915,12 @@ struct celv2_engine {
     FrameJob* dprep = djobs + kRingJobs - 1;
     put_jobs(jobs.data(), 1, dprep, prep_st);
     WorkList w{};
-    w.njobs = 1;
+    w.nparts = 1;
     w.prefix[1] = g.nsb;
+    w.part[0] = SbRange{0, 0, g.nsb};
     if (persistent) {
-      CK(cudaMemsetAsync(queues + 15, 0, sizeof(unsigned), prep_st));
-      w.queue = queues + 15;
+      CK(cudaMemsetAsync(queues + kQueuePrep, 0, sizeof(unsigned), prep_st));
+      w.queue = queues + kQueuePrep;
     }
     stage(kStIntra, prep_st, [&] { launch_intra(dprep, w, prep_st); });
     kernel_launches++;
@@ -931,27 +1076,35 @@ struct celv2_engine {
     }
     const int par = take_parity(st);
     for (int j = 0; j < njobs; j++) jobs[j].out = group[j].records(par);
-    if (use_graphs && !timing)
-      launch_graph(jobs, nets);
-    else
-      run_stages(jobs, true, st, nets);
+    for (int j = 0; j < njobs; j++)
+      group_out[j] = !to_host ? nullptr : dests[j] ? dests[j] : group_host + (size_t)j * g.nsb;
+    const std::vector<Slice> slices = cut(rows_of(jobs), to_host);
+    run(jobs, true, nets, slices, use_graphs && !timing, [&](int i, cudaStream_t ready) {
+      if (!to_host) return;  // records left on the device
+      copy_slice(slices[i], i, ready, [&](int j) { return std::make_pair(jobs[j].out, group_out[j]); });
+    });
     mark_used(reads.data(), (int)reads.size(), st);
     if (to_host) {
-      CK(cudaEventRecord(stages_done, st));
-      CK(cudaStreamWaitEvent(copy_st, stages_done, 0));
-      for (int j = 0; j < njobs; j++) {
-        group_out[j] = dests[j] ? dests[j] : group_host + (size_t)j * g.nsb;
-        CK(cudaMemcpyAsync(group_out[j], jobs[j].out, g.nsb * sizeof(celv2_sb_out), cudaMemcpyDeviceToHost, copy_st));
-      }
       CK(cudaEventRecord(copied[par], copy_st));
       copy_pending[par] = true;
-    } else {
-      for (int j = 0; j < njobs; j++) group_out[j] = nullptr;  // records left on the device
     }
     group_jobs = njobs;
     ++launches;
     launches_group = launches;
     pending = true;
+  }
+
+  // Queues the copies of slice i's records on copy_st, once `ready` has them: of(job) gives a job's
+  // records on the device and on the host.
+  template <typename F>
+  void copy_slice(const Slice& s, int i, cudaStream_t ready, F&& of) {
+    if (ready == st) CK(cudaEventRecord(slice_done[i], st));  // else recorded by run()
+    CK(cudaStreamWaitEvent(copy_st, slice_done[i], 0));
+    for (const SbRange& r : s.parts) {
+      const std::pair<const celv2_sb_out*, celv2_sb_out*> rec = of(r.job);
+      CK(cudaMemcpyAsync(rec.second + r.sb0, rec.first + r.sb0, r.sbs * sizeof(celv2_sb_out), cudaMemcpyDeviceToHost,
+                         copy_st));
+    }
   }
 
   // ---- CUDA graphs: a batch's whole stage sequence captured once per shape, then replayed ----
@@ -972,10 +1125,13 @@ struct celv2_engine {
     graphs.clear();
   }
 
-  void launch_graph(const std::vector<FrameJob>& jobs, const std::vector<NetJob>& nets) {
-    // the shape: per job its reference count, whether it has keep words (which decides whether the
-    // region pass of the inter stage is launched at all), features and the network
-    std::vector<int> key;
+  // The batch up to its slices (enqueue_front), replayed.
+  void launch_graph(const std::vector<FrameJob>& jobs, bool with_intra, const std::vector<NetJob>& nets,
+                    const std::vector<Slice>& slices) {
+    // the shape: whether its superblock stages are in the graph or follow in slices; per job its
+    // reference count, whether it has keep words (which decides whether the region pass of the inter
+    // stage is launched at all), features and the network
+    std::vector<int> key{slices.size() == 1};
     for (size_t j = 0; j < jobs.size(); j++)
       key.push_back(jobs[j].nrefs * 8 + (jobs[j].keep ? 4 : 0) + (nets[j].feats ? 2 : 0) + (nets[j].net ? 1 : 0));
     Graph* gr = nullptr;
@@ -989,7 +1145,7 @@ struct celv2_engine {
       cudaGraph_t graph = nullptr;
       CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
       try {
-        gr->kernels = enqueue_stages(jobs, true, st, nets);
+        gr->kernels = enqueue_front(jobs, with_intra, nets, slices);
       } catch (...) {
         cudaStreamEndCapture(st, &graph);
         if (graph) cudaGraphDestroy(graph);
@@ -1100,21 +1256,18 @@ void launch_multi(int njobs, celv2_engine* const* engines, const long long* src_
   std::vector<FrameJob> jobs;
   std::vector<NetJob> nets;
   for (const Entry& en : entries) jobs.push_back(en.job), nets.push_back(en.net);
-  lead->run_stages(jobs, true, lead->st, nets);
+  for (Entry& en : entries) {
+    if (!to_host) en.dest = nullptr;  // records left on the device
+    else if (!en.dest) en.dest = en.e->group_host + (size_t)en.slot * en.e->g.nsb;
+    en.e->group_out[en.slot] = en.dest;
+  }
+  // the records on the lead's copy stream, overlapping later work
+  const std::vector<celv2_engine::Slice> slices = celv2_engine::cut(celv2_engine::rows_of(jobs), to_host);
+  lead->run(jobs, true, nets, slices, false, [&](int i, cudaStream_t ready) {
+    if (!to_host) return;
+    lead->copy_slice(slices[i], i, ready, [&](int j) { return std::make_pair(jobs[j].out, entries[j].dest); });
+  });
   for (size_t i = 0; i < uniq.size(); i++) uniq[i]->mark_used(reads[i].data(), (int)reads[i].size(), lead->st);
-  if (to_host) {  // on the lead's copy stream, overlapping later work
-    CK(cudaEventRecord(lead->stages_done, lead->st));
-    CK(cudaStreamWaitEvent(lead->copy_st, lead->stages_done, 0));
-  }
-  for (const Entry& en : entries) {
-    if (!to_host) {
-      en.e->group_out[en.slot] = nullptr;  // records left on the device
-      continue;
-    }
-    celv2_sb_out* d = en.dest ? en.dest : en.e->group_host + (size_t)en.slot * en.e->g.nsb;
-    en.e->group_out[en.slot] = d;
-    CK(cudaMemcpyAsync(d, en.job.out, en.e->g.nsb * sizeof(celv2_sb_out), cudaMemcpyDeviceToHost, lead->copy_st));
-  }
   if (to_host)
     for (size_t i = 0; i < uniq.size(); i++) {
       celv2_engine* e = uniq[i];

@@ -44,9 +44,9 @@ __global__ void __launch_bounds__(kFinThreads, 4) k_finalize(const FrameJob* __r
   const int tid = threadIdx.x;
   int unit, iter = 0;
   while (take_unit(w, unit, iter, &unit_slot)) {
-  const int jb = job_of(w, unit);
-  const FrameJob& job = jobs[jb];
-  const int sb = unit - w.prefix[jb], sby = sb / job.sb_cols, sbx = sb - sby * job.sb_cols;
+  const int jb = part_of(w, unit);
+  const FrameJob& job = jobs[w.part[jb].job];
+  const int sb = w.part[jb].sb0 + unit - w.prefix[jb], sby = sb / job.sb_cols, sbx = sb - sby * job.sb_cols;
   const int ox = sbx * 64, oy = sby * 64;
   const int nrefs = job.nrefs;
   const long long lam = job.lam;
@@ -264,7 +264,7 @@ __global__ void __launch_bounds__(kFinThreads, 4) k_finalize(const FrameJob* __r
 }
 
 void launch_finalize(const FrameJob* jobs, const WorkList& w, cudaStream_t st) {
-  const int units = w.prefix[w.njobs];
+  const int units = w.prefix[w.nparts];
   if (units <= 0) return;
   const int grid = w.queue ? persistent_grid((const void*)k_finalize, kFinThreads, sizeof(FinSmem), units) : units;
   k_finalize<<<grid, kFinThreads, sizeof(FinSmem), st>>>(jobs, w);

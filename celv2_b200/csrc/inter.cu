@@ -186,11 +186,11 @@ __global__ void __launch_bounds__(kInterThreads, 4) k_inter(const FrameJob* __re
   const int tid = threadIdx.x, lane = tid & 31;
   int unit, iter = 0;
   while (take_unit(w, unit, iter, &unit_slot)) {
-  const int jb = job_of(w, unit);
-  const FrameJob& job = jobs[jb];
-  const int nsb = job.sb_cols * job.sb_rows;
+  const int jb = part_of(w, unit);
+  const FrameJob& job = jobs[w.part[jb].job];
+  const int nsb = w.part[jb].sbs;
   const int u = unit - w.prefix[jb];
-  const int r = u / nsb, sb = u - r * nsb, sby = sb / job.sb_cols, sbx = sb - sby * job.sb_cols;
+  const int r = u / nsb, sb = w.part[jb].sb0 + u - r * nsb, sby = sb / job.sb_cols, sbx = sb - sby * job.sb_cols;
   const unsigned keep = keep_mask(job, sb);
   // a pruned (superblock, reference) is not scored; without 64-level blocks k_inter_regions scores it
   if (!(keep >> r & 1u) || !(keep & CELV2_KEEP_LEVEL(0))) continue;
@@ -509,11 +509,11 @@ __global__ void __launch_bounds__(kInterThreads, 4) k_inter_regions(const FrameJ
   __shared__ int unit_slot;
   int unit, iter = 0;
   while (take_unit(w, unit, iter, &unit_slot)) {
-    const int jb = job_of(w, unit);
-    const FrameJob& job = jobs[jb];
-    const int nsb = job.sb_cols * job.sb_rows;
+    const int jb = part_of(w, unit);
+    const FrameJob& job = jobs[w.part[jb].job];
+    const int nsb = w.part[jb].sbs;
     const int u = unit - w.prefix[jb];
-    const int r = u / nsb, sb = u - r * nsb, sby = sb / job.sb_cols, sbx = sb - sby * job.sb_cols;
+    const int r = u / nsb, sb = w.part[jb].sb0 + u - r * nsb, sby = sb / job.sb_cols, sbx = sb - sby * job.sb_cols;
     const unsigned keep = keep_mask(job, sb);
     // a pruned (superblock, reference) is not scored; with 64-level blocks k_inter scores it
     if (!(keep >> r & 1u) || (keep & CELV2_KEEP_LEVEL(0))) continue;
@@ -527,7 +527,7 @@ __global__ void __launch_bounds__(kInterThreads, 4) k_inter_regions(const FrameJ
 
 void launch_inter(const FrameJob* jobs, const WorkList& w, int chunk, bool regions, unsigned* region_queue,
                   cudaStream_t st) {
-  const int units = w.prefix[w.njobs];
+  const int units = w.prefix[w.nparts];
   if (units <= 0) return;
   chunk = chunk < 8 ? 8 : chunk > kChunk ? kChunk : chunk;
   const int grid = w.queue ? persistent_grid((const void*)k_inter, kInterThreads, sizeof(WholeSmem), units) : units;

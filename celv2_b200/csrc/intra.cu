@@ -152,9 +152,9 @@ __global__ void __launch_bounds__(kIntraThreads, 4) k_intra(const FrameJob* __re
   const int tid = threadIdx.x;
   int unit, iter = 0;
   while (take_unit(w, unit, iter, &unit_slot)) {
-  const int jb = job_of(w, unit);
-  const FrameJob& job = jobs[jb];
-  const int u = unit - w.prefix[jb], sb = u / parts, part = u - sb * parts;
+  const int jb = part_of(w, unit);
+  const FrameJob& job = jobs[w.part[jb].job];
+  const int u = unit - w.prefix[jb], usb = u / parts, part = u - usb * parts, sb = w.part[jb].sb0 + usb;
   const int sby = sb / job.sb_cols, sbx = sb - sby * job.sb_cols;
   const unsigned keep = keep_mask(job, sb);
   if (!(keep & CELV2_KEEP_INTRA)) continue;  // intra pruned for this superblock
@@ -505,12 +505,12 @@ __global__ void __launch_bounds__(kIntraThreads, 4) k_intra(const FrameJob* __re
 static int intra_parts(int sbs, int full) { return sbs * 9 <= full ? 9 : sbs <= full ? 3 : 1; }
 
 void launch_intra(const FrameJob* jobs, const WorkList& w, cudaStream_t st) {
-  const int sbs = w.prefix[w.njobs];
+  const int sbs = w.prefix[w.nparts];
   if (sbs <= 0) return;
   const int full = persistent_grid((const void*)k_intra, kIntraThreads, sizeof(IntraSmem), INT_MAX);
   const int parts = intra_parts(sbs, full), units = sbs * parts;
   WorkList wp = w;
-  for (int j = 1; j <= w.njobs; j++) wp.prefix[j] = w.prefix[j] * parts;
+  for (int j = 1; j <= w.nparts; j++) wp.prefix[j] = w.prefix[j] * parts;
   k_intra<<<w.queue ? std::min(full, units) : units, kIntraThreads, sizeof(IntraSmem), st>>>(jobs, wp, parts);
 }
 

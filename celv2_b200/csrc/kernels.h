@@ -12,12 +12,19 @@ namespace celv2cu {
 
 constexpr int kMaxJobs = 32;
 
-// Units of one stage per job, as prefix sums: job j owns units [prefix[j], prefix[j + 1]).
+// The superblocks [sb0, sb0 + sbs) of a job.
+struct SbRange {
+  int job, sb0, sbs;
+};
+
+// Units of one stage as prefix sums: part p -- a job, or in the superblock stages (intra, inter,
+// finalize) a range of its superblocks -- owns units [prefix[p], prefix[p + 1]).
 // queue: the stage's work queue in device memory (zero before the launch) -- a persistent grid's
 // CTAs take units from it in order until it runs dry; null: one CTA per unit (blockIdx.x).
 struct WorkList {
-  int njobs;
+  int nparts;
   int prefix[kMaxJobs + 1];
+  SbRange part[kMaxJobs];
   unsigned* queue;
 };
 
@@ -25,7 +32,7 @@ struct WorkList {
 // Starts with a barrier, so the previous unit's shared state is free for the next one. No CTA
 // ever waits for another: a drained queue simply ends the loop.
 __device__ __forceinline__ bool take_unit(const WorkList& w, int& unit, int& iter, int* slot) {
-  const int total = w.prefix[w.njobs];
+  const int total = w.prefix[w.nparts];
   if (!w.queue) {
     if (iter++) return false;
     unit = blockIdx.x;
@@ -41,10 +48,10 @@ __device__ __forceinline__ bool take_unit(const WorkList& w, int& unit, int& ite
 // CTAs of a persistent grid for a kernel: the SM count times the CTAs an SM holds, at most units.
 int persistent_grid(const void* kernel, int threads, size_t smem, int units);
 
-// Unit u's job (a linear scan: at most kMaxJobs jobs).
-__device__ __forceinline__ int job_of(const WorkList& w, int u) {
+// Unit u's part (a linear scan: at most kMaxJobs parts).
+__device__ __forceinline__ int part_of(const WorkList& w, int u) {
   int j = 0;
-  while (j + 1 < w.njobs && u >= w.prefix[j + 1]) j++;
+  while (j + 1 < w.nparts && u >= w.prefix[j + 1]) j++;
   return j;
 }
 
@@ -62,18 +69,18 @@ void launch_me_level(const FrameJob* jobs, const WorkList& w, int level, int cel
 int refine_units(int nrefs, int cols, int rows);
 void launch_me_refine(const FrameJob* jobs, const WorkList& w, cudaStream_t st);
 
-// Intra SATDs of every candidate block and mode. Units: sb_cols * sb_rows per job (split further by the
+// Intra SATDs of every candidate block and mode. Units: the parts' superblocks (split further by the
 // launcher where they are few).
 void launch_intra(const FrameJob* jobs, const WorkList& w, cudaStream_t st);
 
 // Each reference's best candidate MV per candidate block, the distinct MVs of a superblock taken
-// in chunks of at most `chunk` (<= 64). Units: nrefs * sb_cols * sb_rows per job. Units that keep
+// in chunks of at most `chunk` (<= 64). Units: nrefs times the parts' superblocks. Units that keep
 // their 64-level blocks are scored whole (k_inter); with `regions` (some job has keep words) a
 // second kernel scores the others region by region, draining `region_queue` (zero beforehand).
 void launch_inter(const FrameJob* jobs, const WorkList& w, int chunk, bool regions, unsigned* region_queue,
                   cudaStream_t st);
 
-// Per-block choice, compound, partition choice and the decision records. Units: superblocks.
+// Per-block choice, compound, partition choice and the decision records. Units: the parts' superblocks.
 void launch_finalize(const FrameJob* jobs, const WorkList& w, cudaStream_t st);
 
 // The learned pruner (pruner.cu): one job's features (nsb x CELV2_PRUNER_FEATURES), the network's

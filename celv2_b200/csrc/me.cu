@@ -119,8 +119,8 @@ __global__ void __launch_bounds__(kMeThreads, 4) k_me_level(const FrameJob* __re
   const int tid = threadIdx.x;
   int unit, iter = 0;
   while (take_unit(w, unit, iter, &unit_slot)) {
-  const int jb = job_of(w, unit);
-  const FrameJob& job = jobs[jb];
+  const int jb = part_of(w, unit);
+  const FrameJob& job = jobs[w.part[jb].job];
   const int cols = job.fcols[level], rows = job.frows[level], ncell = cols * rows;
   const int groups = (ncell + kMeCells - 1) / kMeCells;
   const int u = unit - w.prefix[jb];
@@ -359,8 +359,8 @@ __global__ void __launch_bounds__(kRefineThreads, 8) k_me_refine(const FrameJob*
   const int tid = threadIdx.x, c = tid & 31, t = tid >> 5;
   int unit, iter = 0;
   while (take_unit(w, unit, iter, &unit_slot)) {
-  const int jb = job_of(w, unit);
-  const FrameJob& job = jobs[jb];
+  const int jb = part_of(w, unit);
+  const FrameJob& job = jobs[w.part[jb].job];
   const int cols = job.fcols[0], ncell = cols * job.frows[0];
   const int groups = (ncell + kRefineCells - 1) / kRefineCells;
   const int u = unit - w.prefix[jb];
@@ -454,7 +454,7 @@ __global__ void __launch_bounds__(kRefineThreads, 8) k_me_refine(const FrameJob*
 int refine_units(int nrefs, int cols, int rows) { return nrefs * ((cols * rows + kRefineCells - 1) / kRefineCells); }
 
 void launch_me_refine(const FrameJob* jobs, const WorkList& w, cudaStream_t st) {
-  const int units = w.prefix[w.njobs];
+  const int units = w.prefix[w.nparts];
   if (units <= 0) return;
   const int grid = w.queue ? persistent_grid((const void*)k_me_refine, kRefineThreads, 0, units) : units;
   k_me_refine<<<grid, kRefineThreads, 0, st>>>(jobs, w);
@@ -464,14 +464,14 @@ int me_units(int nrefs, int cols, int rows, int cells) { return nrefs * ((cols *
 
 template <int CELLS>
 static void launch_cells(const FrameJob* jobs, const WorkList& w, int level, cudaStream_t st) {
-  const int units = w.prefix[w.njobs];
+  const int units = w.prefix[w.nparts];
   const size_t smem = sizeof(MeSmem<CELLS>);
   const int grid = w.queue ? persistent_grid((const void*)k_me_level<CELLS>, kMeThreads, smem, units) : units;
   k_me_level<CELLS><<<grid, kMeThreads, smem, st>>>(jobs, w, level);
 }
 
 void launch_me_level(const FrameJob* jobs, const WorkList& w, int level, int cells, cudaStream_t st) {
-  if (w.prefix[w.njobs] <= 0) return;
+  if (w.prefix[w.nparts] <= 0) return;
   if (cells == 15)
     launch_cells<15>(jobs, w, level, st);
   else

@@ -137,8 +137,9 @@ extern "C" int celv2_decide_key_noalloc(const uint8_t* luma, int width, int heig
   e = cudaGetLastError();
   if (e == cudaSuccess) {
     WorkList w{};
-    w.njobs = 1;
+    w.nparts = 1;
     w.prefix[1] = sb_cols * sb_rows;
+    w.part[0] = SbRange{0, 0, sb_cols * sb_rows};
     launch_intra(djob, w, st);
     launch_finalize(djob, w, st);
     e = cudaGetLastError();
