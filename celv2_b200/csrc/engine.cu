@@ -173,7 +173,9 @@ struct Stage {
   void* dev = nullptr;
   size_t bytes = 0;
   cudaEvent_t done = nullptr;
-  bool pending = false;
+  bool pending = false;      // `done` recorded after the last use
+  bool taken = false;        // in use, `done` not recorded yet
+  unsigned long long turn = 0;  // when it was taken last
 };
 
 // Stages timed by CUDA events when stage timing is on (celv2_stage_timing).
@@ -213,14 +215,15 @@ struct celv2_engine {
   int device = 0;
   Geometry g;
   cudaStream_t st = nullptr, prep_st = nullptr;
-  cudaEvent_t prep_done = nullptr;
+  cudaEvent_t src_up = nullptr, prep_done = nullptr;  // prepare's stream: the planes made, the intra SATDs made
+  static constexpr size_t kCopyPiece = 512 << 10;  // bytes of a plane copied on the host before they go to the GPU
   std::vector<Slot*> store;      // keyed frames (references, resident frames)
   Slot srcs[2];                  // sources of launch / prepare
   int cur_src = 0;
   long long launches = 0;
   long long launches_group = -1;  // the value of `launches` after the last group launch
   std::vector<Stage> stages;
-  int next_stage = 0;
+  unsigned long long stage_turn = 0;
   JobBuffers single;             // the launch() path
   int* intra_prep[2] = {nullptr, nullptr};  // intra SATDs per source slot
   celv2_sb_out* host_out = nullptr;          // pinned, nsb records
@@ -366,6 +369,7 @@ struct celv2_engine {
     cudaFreeHost(ring);
     for (cudaEvent_t e : ring_done)
       if (e) cudaEventDestroy(e);
+    if (src_up) cudaEventDestroy(src_up);
     if (prep_done) cudaEventDestroy(prep_done);
     for (int i = 0; i < kMaxSlices; i++) {
       if (slice_ready[i]) cudaEventDestroy(slice_ready[i]);
@@ -418,19 +422,14 @@ struct celv2_engine {
     g.set(width, height);
     CK(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
     CK(cudaStreamCreateWithFlags(&prep_st, cudaStreamNonBlocking));
+    CK(cudaEventCreateWithFlags(&src_up, cudaEventDisableTiming));
     CK(cudaEventCreateWithFlags(&prep_done, cudaEventDisableTiming));
     CK(cudaStreamCreateWithFlags(&copy_st, cudaStreamNonBlocking));
     CK(cudaStreamCreateWithFlags(&up_st, cudaStreamNonBlocking));
     for (cudaEvent_t& e : copied) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    CK(cudaEventCreateWithFlags(&slice_done[0], cudaEventDisableTiming));
     CK(cudaMalloc(&djobs, kRingJobs * sizeof(FrameJob)));
     CK(cudaMalloc(&queues, kQueues * sizeof(unsigned)));
-    int least = 0, greatest = 0;
-    CK(cudaDeviceGetStreamPriorityRange(&least, &greatest));
-    CK(cudaStreamCreateWithPriority(&fin_st, cudaStreamNonBlocking, greatest));
-    for (int i = 0; i < kMaxSlices; i++) {
-      CK(cudaEventCreateWithFlags(&slice_ready[i], cudaEventDisableTiming));
-      CK(cudaEventCreateWithFlags(&slice_done[i], cudaEventDisableTiming));
-    }
     CK(cudaMallocHost(&ring, (size_t)kRing * kRingJobs * sizeof(FrameJob)));
     for (cudaEvent_t& e : ring_done) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     alloc_buffers(single, false);
@@ -464,19 +463,48 @@ struct celv2_engine {
     s.phases = false;
   }
 
+  // A staging buffer of at least `bytes`: the first one whose last use is over, so that few of them
+  // are ever allocated and their pages stay in the host's cache (in turn, sixteen planes' worth did
+  // not: a 1080p 16-bit plane's copy 0.43 ms against 0.3); with none free the one taken longest ago.
   Stage& take_stage(size_t bytes) {
-    Stage& s = stages[next_stage];
-    next_stage = (next_stage + 1) % (int)stages.size();
+    Stage *pick = nullptr, *oldest = nullptr;
+    for (Stage& s : stages) {
+      if (s.taken) continue;
+      if (s.pending && cudaEventQuery(s.done) == cudaSuccess) s.pending = false;
+      if (!s.pending && (!pick || pick->bytes < bytes)) pick = &s;
+      if (pick && pick->bytes >= bytes) break;
+      if (!oldest || s.turn < oldest->turn) oldest = &s;
+    }
+    if (!pick) pick = oldest;
+    if (!pick) throw Error(CELV2_ESTATE, "no staging buffer left");
+    Stage& s = *pick;
     if (s.pending) CK(cudaEventSynchronize(s.done)), s.pending = false;
     if (s.bytes < bytes) {
       if (s.host) CK(cudaFreeHost(s.host));
       if (s.dev) CK(cudaFree(s.dev));
       s.host = s.dev = nullptr;
+      s.bytes = 0;
       CK(cudaMallocHost(&s.host, bytes));
       CK(cudaMalloc(&s.dev, bytes));
       s.bytes = bytes;
     }
+    s.taken = true;
+    s.turn = ++stage_turn;
     return s;
+  }
+  // s's last use ends where `stream` now stands.
+  void give_stage(Stage& s, cudaStream_t stream) {
+    CK(cudaEventRecord(s.done, stream));
+    s.pending = true, s.taken = false;
+  }
+  // Staging buffers a failed call left taken: free once what it queued is over.
+  void recover_stages() {
+    for (Stage& s : stages)
+      if (s.taken) {
+        for (cudaStream_t t : {st, prep_st, up_st}) cudaStreamSynchronize(t);
+        for (Stage& x : stages) x.taken = false;
+        return;
+      }
   }
 
   void check_frame(const celv2_frame* f, const char* what) {
@@ -488,15 +516,19 @@ struct celv2_engine {
     if (f->pitch && f->pitch < g.pw) invalid(std::string(what) + ": pitch below the padded width");
   }
 
-  // Copies f's luma into pinned memory (synchronously: the caller may change it afterwards), then
-  // queues its upload, the 8-bit level 0, the pyramid and (phases) the quarter-pel planes.
-  // Uploads f into s on `stream`: 8-bit level 0 and pyramid, the phase planes too when `phases`
-  // (room for them when `room`).
+  // A frame on its way into a slot: its samples in the staging buffer's device half.
+  struct Incoming {
+    Slot* s;
+    Stage* sg;
+    PlaneIn in;
+  };
+
+  // Copies f's luma into pinned memory (synchronously: the caller may change it afterwards) and queues
+  // its upload into a staging buffer of s's on `stream` (room: s gets room for the phase planes).
   // direct: the plane is page-locked and stays unchanged until the upload ran (DMA from it, no
   // staging copy on the host).
-  void upload(const celv2_frame* f, Slot& s, bool phases, cudaStream_t stream, bool room = false,
-              bool direct = false) {
-    alloc_slot(s, phases || room || s.phases);
+  Incoming bring(const celv2_frame* f, Slot& s, cudaStream_t stream, bool room, bool direct = false) {
+    alloc_slot(s, room || s.phases);
     const bool wide = f->y == nullptr;
     const int pitch = f->pitch ? f->pitch : g.pw;
     const size_t row = (size_t)g.pw * (wide ? 2 : 1);
@@ -506,32 +538,53 @@ struct celv2_engine {
     if (direct) {
       CK(cudaMemcpy2DAsync(sg.dev, row, src, spitch, row, g.ph, cudaMemcpyHostToDevice, stream));
     } else {
-      if (spitch == row) {
-        std::memcpy(sg.host, src, row * g.ph);
-      } else {
-        for (int r = 0; r < g.ph; r++) std::memcpy((uint8_t*)sg.host + r * row, src + r * spitch, row);
+      // piece by piece, so a large plane's upload runs beside its own copy
+      const int step = (int)std::max<size_t>(1, kCopyPiece / row);
+      for (int r = 0; r < g.ph; r += step) {
+        const int n = std::min(step, g.ph - r);
+        uint8_t* h = static_cast<uint8_t*>(sg.host) + r * row;
+        if (spitch == row) {
+          std::memcpy(h, src + r * row, n * row);
+        } else {
+          for (int k = 0; k < n; k++) std::memcpy(h + k * row, src + (r + k) * spitch, row);
+        }
+        CK(cudaMemcpyAsync(static_cast<uint8_t*>(sg.dev) + r * row, h, n * row, cudaMemcpyHostToDevice, stream));
       }
-      CK(cudaMemcpyAsync(sg.dev, sg.host, row * g.ph, cudaMemcpyHostToDevice, stream));
     }
-    stage(kStUpload, stream, [&] {
-      if (wide)
-        launch_expand_u16((const uint16_t*)sg.dev, g.pw, f->bit_depth, s.pyr.lv[0], stream);
-      else
-        launch_expand_u8((const uint8_t*)sg.dev, g.pw, s.pyr.lv[0], stream);
-    });
-    CK(cudaEventRecord(sg.done, stream));
-    sg.pending = true;
-    stage(kStUpload, stream, [&] { launch_pyramid(s.pyr, stream); });
-    kernel_launches += 1 + (kLevels - 1);
     s.phases = false;
-    if (phases) make_phases(s, stream);
+    return Incoming{&s, &sg, PlaneIn{sg.dev, wide ? f->bit_depth - 8 : -1, s.pyr}};
   }
 
-  void make_phases(Slot& s, cudaStream_t stream) {
-    if (s.phases) return;
-    stage(kStPhases, stream, [&] { launch_phases(s.pyr.lv[0], stream); });
-    kernel_launches++;
-    s.phases = true;
+  // Queues level 0 and the pyramid of every frame brought in on `stream`, one launch for all of them.
+  void make_planes(const std::vector<Incoming>& in, cudaStream_t stream) {
+    for (size_t i = 0; i < in.size();) {
+      PlaneSet set{};
+      const size_t first = i;
+      for (; i < in.size() && set.n <= kMaxRefs; i++) set.p[set.n++] = in[i].in;
+      stage(kStUpload, stream, [&] { launch_pyramid(set, stream); });
+      kernel_launches++;
+      for (size_t k = first; k < i; k++) {
+        give_stage(*in[k].sg, stream);
+      }
+    }
+  }
+
+  // Queues the phase planes of those of the slots that have none yet.
+  void make_phases(Slot* const* slots, int n, cudaStream_t stream) {
+    PlaneSet set{};
+    auto flush = [&] {
+      if (!set.n) return;
+      stage(kStPhases, stream, [&] { launch_phases(set, stream); });
+      kernel_launches++;
+      set.n = 0;
+    };
+    for (int i = 0; i < n; i++) {
+      if (slots[i]->phases) continue;
+      if (set.n > kMaxRefs) flush();
+      set.p[set.n++].pyr = slots[i]->pyr;
+      slots[i]->phases = true;
+    }
+    flush();
   }
 
   // The store's slot for `key` (keys of this launch are protected), else a free or new one.
@@ -595,8 +648,7 @@ struct celv2_engine {
     Stage& sg = take_stage(bytes);
     std::memcpy(sg.host, k.data(), bytes);
     CK(cudaMemcpyAsync(b.keep, sg.host, bytes, cudaMemcpyHostToDevice, stream));
-    CK(cudaEventRecord(sg.done, stream));
-    sg.pending = true;
+    give_stage(sg, stream);
     return b.keep;
   }
 
@@ -749,19 +801,24 @@ struct celv2_engine {
     return launched;
   }
 
-  // Everything of a batch up to its slices: motion search, refinement, and intra (with_intra) unless
-  // the slices run it; of a batch in one slice also its inter stage and finalize. A batch without
-  // references has its intra in the slices: it is all the work there is before the records.
-  int enqueue_front(const std::vector<FrameJob>& jobs, bool with_intra, const std::vector<NetJob>& nets,
+  // Everything of a batch up to its slices: motion search, refinement, and intra (unless it runs on
+  // another stream, which records intra_done) where the slices do not run it; of a batch in one slice
+  // also its inter stage and finalize. A batch without references has its intra in the slices: it is
+  // all the work there is before the records.
+  int enqueue_front(const std::vector<FrameJob>& jobs, cudaEvent_t intra_done, const std::vector<NetJob>& nets,
                     const std::vector<Slice>& slices) {
     int launched = enqueue_search(jobs, st, nets);
     const bool whole = slices.size() == 1;
-    if (with_intra && (whole || any_refs(jobs))) {
+    if (!intra_done && (whole || any_refs(jobs))) {
       Slice all;
       for (int j = 0; j < (int)jobs.size(); j++) all.parts.push_back(SbRange{j, 0, jobs[j].sb_cols * jobs[j].sb_rows});
       launched += enqueue_intra(jobs, all, 0, st);
     }
-    if (whole) launched += enqueue_inter(jobs, slices[0], 0, st) + enqueue_finalize(jobs, slices[0], 0, st);
+    if (whole) {
+      launched += enqueue_inter(jobs, slices[0], 0, st);
+      if (intra_done) CK(cudaStreamWaitEvent(st, intra_done, 0));
+      launched += enqueue_finalize(jobs, slices[0], 0, st);
+    }
     return launched;
   }
   static bool any_refs(const std::vector<FrameJob>& jobs) {
@@ -770,26 +827,40 @@ struct celv2_engine {
     return false;
   }
 
+  // What batches in several slices need, made with the first of them.
+  void make_fin_stream() {
+    if (fin_st) return;
+    int least = 0, greatest = 0;
+    CK(cudaDeviceGetStreamPriorityRange(&least, &greatest));
+    for (int i = 0; i < kMaxSlices; i++)
+      if (!slice_ready[i]) CK(cudaEventCreateWithFlags(&slice_ready[i], cudaEventDisableTiming));
+    for (int i = 1; i < kMaxSlices; i++)
+      if (!slice_done[i]) CK(cudaEventCreateWithFlags(&slice_done[i], cudaEventDisableTiming));
+    CK(cudaStreamCreateWithPriority(&fin_st, cudaStreamNonBlocking, greatest));
+  }
+
   // The stages of a batch on st, its descriptors sent through the pinned ring (graph: the part up to
   // the slices replayed as a CUDA graph). done(i, stream) is called once slice i's records are queued
   // on `stream` -- to queue their copies. Several slices: the inter stage of one runs while the
   // finalize of the one before it, on a stream of higher priority, takes the SMs the drained inter
   // launch leaves; st waits for the last finalize.
   template <typename F>
-  void run(const std::vector<FrameJob>& jobs, bool with_intra, const std::vector<NetJob>& nets,
+  void run(const std::vector<FrameJob>& jobs, cudaEvent_t intra_done, const std::vector<NetJob>& nets,
            const std::vector<Slice>& slices, bool graph, F&& done) {
-    if (graph) {
-      launch_graph(jobs, with_intra, nets, slices);
+    if (graph) {  // (never with intra on another stream)
+      launch_graph(jobs, nets, slices);
     } else {
       put_jobs(jobs.data(), (int)jobs.size(), djobs, st);
-      kernel_launches += enqueue_front(jobs, with_intra, nets, slices);
+      kernel_launches += enqueue_front(jobs, intra_done, nets, slices);
     }
     const int n = (int)slices.size();
     if (n == 1) {
       done(0, st);
       return;
     }
-    const bool intra_here = with_intra && !any_refs(jobs);
+    make_fin_stream();
+    const bool intra_here = !intra_done && !any_refs(jobs);
+    if (intra_done) CK(cudaStreamWaitEvent(fin_st, intra_done, 0));
     for (int i = 0; i < n; i++) {
       if (intra_here) kernel_launches += enqueue_intra(jobs, slices[i], i, st);
       kernel_launches += enqueue_inter(jobs, slices[i], i, st);
@@ -823,37 +894,44 @@ struct celv2_engine {
     for (int r = 0; r < nrefs; r++) check_frame(&refs[r], "reference");
     if (nrefs > 0 && (g.pw < 16 || g.ph < 16)) invalid("CudaEngine: inter frames need at least 9x9 pixels");
     if (pending) wait_idle();
+    recover_stages();
     try {
-      // the prepared source, else an upload into the other slot
+      // the prepared source, else an upload into the other slot: with the intra stage beside the
+      // references' uploads and the motion search, on prepare's stream, where nothing decides it anew
+      // (no keep words; a KEY frame has nothing to run beside)
       int use = -1;
       for (int i = 0; i < 2; i++)
         if (src_key >= 0 && srcs[i].key == src_key) use = i;
-      const bool prepared = use >= 0;
-      if (prepared) {
-        CK(cudaStreamWaitEvent(st, prep_done, 0));
-      } else {
+      bool prepared = use >= 0;
+      if (!prepared) {
         use = 1 - cur_src;
         CK(cudaStreamSynchronize(prep_st));  // a prepare() into this slot may still run
-        upload(src, srcs[use], false, st);
+        if (nrefs > 0 && keep0.empty() && !pruner_params) {
+          start_source(src, use);
+          prepared = true;
+        } else {
+          make_planes({bring(src, srcs[use], st, false)}, st);
+        }
       }
+      if (prepared) CK(cudaStreamWaitEvent(st, src_up, 0));
       srcs[use].key = -1;  // used: a later prepare() may overwrite it
       cur_src = use;
       const long long now = ++launches;
       Slot* used[kMaxRefs];
+      std::vector<Incoming> fresh_refs;
       for (int r = 0; r < nrefs; r++) {
         bool fresh;
         Slot* s = ref_slot(keys ? keys[r] : -1, keys, keys ? nrefs : 0, now, fresh);
+        wait_ready(*s, st);  // a frame of the store; a dropped one's upload may still run
         if (fresh) {
-          wait_ready(*s, st);  // a dropped store frame's upload may still run
-          upload(&refs[r], *s, true, st);
+          fresh_refs.push_back(bring(&refs[r], *s, st, true));
           s->key = keys ? keys[r] : -1;
-        } else {
-          wait_ready(*s, st);  // a frame of the store
-          make_phases(*s, st);
         }
         s->used = now;
         used[r] = s;
       }
+      make_planes(fresh_refs, st);
+      make_phases(used, nrefs, st);
       std::vector<FrameJob> jobs(1);
       fill_job(jobs[0], srcs[use].pyr, used, nrefs, single, intra_prep[use], lam);
       jobs[0].keep = put_keep(keep0, single, st);
@@ -872,7 +950,7 @@ struct celv2_engine {
       if ((int)slices.size() > kMaxSlices) slices.assign(1, Slice{});
       if (slices.size() == 1) slices[0].parts.assign(1, SbRange{0, 0, g.nsb}), slices[0].sbs = g.nsb;
       size_t next = 0;  // the next row of `order` to copy
-      run(jobs, !prepared, nets, slices, false, [&](int i, cudaStream_t ready) {
+      run(jobs, prepared ? prep_done : nullptr, nets, slices, false, [&](int i, cudaStream_t ready) {
         // one slice: the copies follow on st; several: on copy_st, beside the next slices' stages
         cudaStream_t cs = st;
         if (ready != st) {
@@ -893,7 +971,7 @@ struct celv2_engine {
       pending = true;
     } catch (...) {
       cudaStreamSynchronize(st);  // a failure leaves no work running
-      cudaStreamSynchronize(fin_st);
+      if (fin_st) cudaStreamSynchronize(fin_st);
       cudaStreamSynchronize(copy_st);
       cudaStreamSynchronize(prep_st);
       pending = false;
@@ -904,13 +982,22 @@ struct celv2_engine {
   void prepare(const celv2_frame* next, long long key) {
     if (key < 0 || !next || next->width != g.width || next->height != g.height) return;
     check_frame(next, "next frame");
-    Slot& s = srcs[1 - cur_src];
-    s.key = -1;
+    recover_stages();
     // the slot's previous use (two launches back) was collected; the current launch uses the other
-    upload(next, s, false, prep_st);
+    srcs[1 - cur_src].key = -1;
+    start_source(next, 1 - cur_src);
+    srcs[1 - cur_src].key = key;
+  }
+
+  // A source's work that needs no reference, on prepare's stream: planes (src_up) and intra SATDs of
+  // every superblock (prep_done) of source slot i.
+  void start_source(const celv2_frame* f, int i) {
+    Slot& s = srcs[i];
+    make_planes({bring(f, s, prep_st, false)}, prep_st);
+    CK(cudaEventRecord(src_up, prep_st));
     std::vector<FrameJob> jobs(1);
     JobBuffers none{};
-    fill_job(jobs[0], s.pyr, nullptr, 0, none, intra_prep[1 - cur_src], 0);
+    fill_job(jobs[0], s.pyr, nullptr, 0, none, intra_prep[i], 0);
     // the intra stage alone, from a descriptor area of its own (the main stream owns djobs[0..])
     FrameJob* dprep = djobs + kRingJobs - 1;
     put_jobs(jobs.data(), 1, dprep, prep_st);
@@ -926,7 +1013,6 @@ struct celv2_engine {
     kernel_launches++;
     CK(cudaGetLastError());
     CK(cudaEventRecord(prep_done, prep_st));
-    s.key = key;
   }
 
   const celv2_sb_out* wait_row(int row) {
@@ -983,6 +1069,7 @@ struct celv2_engine {
   void upload_store(const celv2_frame* f, long long key, bool direct = false) {
     check_frame(f, "frame");
     if (key < 0) invalid("store keys must be >= 0");
+    recover_stages();
     // No wait for queued work: it runs on this stream, ahead of the upload.
     Slot* s = find(key);
     if (!s) {
@@ -1010,7 +1097,7 @@ struct celv2_engine {
     // planes are made by the first launch that uses the frame as a reference
     if (s->use_pending) CK(cudaStreamWaitEvent(up_st, s->last_use, 0));
     s->use_pending = false;
-    upload(f, *s, false, up_st, true, direct);
+    make_planes({bring(f, *s, up_st, true, direct)}, up_st);
     CK(cudaEventRecord(s->ready, up_st));
     s->ready_pending = true;
     s->key = key;
@@ -1063,9 +1150,9 @@ struct celv2_engine {
       reads.push_back(cur);
       for (int r = 0; r < nrefs[j]; r++) {
         wait_ready(*refs[r], st);
-        make_phases(*refs[r], st);
         reads.push_back(refs[r]);
       }
+      make_phases(refs, nrefs[j], st);
       fill_job(jobs[j], cur->pyr, refs, nrefs[j], group[j], group[j].intra, lams[j]);
     }
     std::vector<NetJob> nets(njobs);
@@ -1079,7 +1166,7 @@ struct celv2_engine {
     for (int j = 0; j < njobs; j++)
       group_out[j] = !to_host ? nullptr : dests[j] ? dests[j] : group_host + (size_t)j * g.nsb;
     const std::vector<Slice> slices = cut(rows_of(jobs), to_host);
-    run(jobs, true, nets, slices, use_graphs && !timing, [&](int i, cudaStream_t ready) {
+    run(jobs, nullptr, nets, slices, use_graphs && !timing, [&](int i, cudaStream_t ready) {
       if (!to_host) return;  // records left on the device
       copy_slice(slices[i], i, ready, [&](int j) { return std::make_pair(jobs[j].out, group_out[j]); });
     });
@@ -1126,7 +1213,7 @@ struct celv2_engine {
   }
 
   // The batch up to its slices (enqueue_front), replayed.
-  void launch_graph(const std::vector<FrameJob>& jobs, bool with_intra, const std::vector<NetJob>& nets,
+  void launch_graph(const std::vector<FrameJob>& jobs, const std::vector<NetJob>& nets,
                     const std::vector<Slice>& slices) {
     // the shape: whether its superblock stages are in the graph or follow in slices; per job its
     // reference count, whether it has keep words (which decides whether the region pass of the inter
@@ -1145,7 +1232,7 @@ struct celv2_engine {
       cudaGraph_t graph = nullptr;
       CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
       try {
-        gr->kernels = enqueue_front(jobs, with_intra, nets, slices);
+        gr->kernels = enqueue_front(jobs, nullptr, nets, slices);
       } catch (...) {
         cudaStreamEndCapture(st, &graph);
         if (graph) cudaGraphDestroy(graph);
@@ -1239,9 +1326,9 @@ void launch_multi(int njobs, celv2_engine* const* engines, const long long* src_
     reads[ei].push_back(cur);
     for (int r = 0; r < nrefs[j]; r++) {
       e->wait_ready(*refs[r], lead->st);
-      e->make_phases(*refs[r], lead->st);
       reads[ei].push_back(refs[r]);
     }
+    e->make_phases(refs, nrefs[j], lead->st);
     Entry en;
     e->fill_job(en.job, cur->pyr, refs, nrefs[j], e->group[slot], e->group[slot].intra, lams[j]);
     en.job.keep = e->put_keep(keeps[ei][slot], e->group[slot], lead->st);
@@ -1263,7 +1350,7 @@ void launch_multi(int njobs, celv2_engine* const* engines, const long long* src_
   }
   // the records on the lead's copy stream, overlapping later work
   const std::vector<celv2_engine::Slice> slices = celv2_engine::cut(celv2_engine::rows_of(jobs), to_host);
-  lead->run(jobs, true, nets, slices, false, [&](int i, cudaStream_t ready) {
+  lead->run(jobs, nullptr, nets, slices, false, [&](int i, cudaStream_t ready) {
     if (!to_host) return;
     lead->copy_slice(slices[i], i, ready, [&](int j) { return std::make_pair(jobs[j].out, entries[j].dest); });
   });

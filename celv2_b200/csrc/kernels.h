@@ -55,10 +55,21 @@ __device__ __forceinline__ int part_of(const WorkList& w, int u) {
   return j;
 }
 
-void launch_expand_u8(const uint8_t* raw, int pitch, const DevPlane& lv0, cudaStream_t st);
-void launch_expand_u16(const uint16_t* raw, int pitch, int bit_depth, const DevPlane& lv0, cudaStream_t st);
-void launch_pyramid(const DevPyramid& pyr, cudaStream_t st);
-void launch_phases(const DevPlane& lv0, cudaStream_t st);
+// A plane to make from its uploaded samples (packed rows of the padded width): its pyramid with
+// margins. shift: bit depth - 8 of 16-bit samples, -1: 8-bit samples.
+struct PlaneIn {
+  const void* raw;
+  int shift;
+  DevPyramid pyr;
+};
+struct PlaneSet {
+  int n;
+  PlaneIn p[kMaxRefs + 1];
+};
+// Level 0 with its margin and the pyramid of every plane of the set, from their samples.
+void launch_pyramid(const PlaneSet& s, cudaStream_t st);
+// The quarter-pel phase planes of every plane of the set (pyr.lv[0] alone is read).
+void launch_phases(const PlaneSet& s, cudaStream_t st);
 
 // Motion search of one pyramid level for every (job, reference, 8x8 cell), whole-pel (level 0's
 // field in quarter pels). Units: me_units(nrefs, fcols[level], frows[level], cells) per job (groups
