@@ -1,10 +1,14 @@
 // pruner.cu: the learned partition / mode pruner -- its features, its network (forward and
 // backward), loss and optimiser, and the masks it proposes (include/celv2_pruner.h).
 //
-// The network is small (55,080 parameters, ~1 MFLOP per superblock); every layer is an im2col
-// (convolutions) plus one GEMM on the tensor cores: operands rounded to BF16, mma.sync m16n8k16
-// with FP32 accumulators, bias and ReLU in the epilogue. The backward pass is the same GEMM with
-// transposed strides, a gather col2im, ReLU masks and column sums for the biases.
+// The network is small (56,120 parameters, ~1 MFLOP per superblock), so training is bound by what
+// moves between its layers. The forward pass runs all three convolutions of two samples in one CTA,
+// the backward pass all three of one: the activations' BF16 copies sit in shared memory and a
+// convolution's column matrix exists only as the row addresses ldmatrix is given (a zero row for the
+// padding); weight gradients stay in the CTA's accumulators over all its samples. Operands are rounded
+// to BF16, mma.sync m16n8k16 with FP32 accumulators, bias, ReLU and masks on the FP32 values, which is
+// what the cache between the passes holds. A step on 4,096 samples 2.33 -> 0.28 ms against column
+// matrices written out and read back for every layer (390 MB) and weight gradients of a few CTAs.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
@@ -24,194 +28,558 @@ constexpr int kF = CELV2_PRUNER_FEATURES, kOut = CELV2_PRUNER_OUTPUTS;
 constexpr int kW1 = 0, kB1 = kW1 + 16 * 9, kW2 = kB1 + 16, kB2 = kW2 + 32 * 144, kW3 = kB2 + 32, kB3 = kW3 + 32 * 288,
               kW4 = kB3 + 32, kB4 = kW4 + 64 * 632, kW5 = kB4 + 64, kB5 = kW5 + kOut * 64, kParams = kB5 + kOut;
 static_assert(kParams == CELV2_PRUNER_PARAMS, "parameter count");
-// forward cache, floats per sample, in this order
-constexpr int kCols1 = 256 * 9, kA1 = 256 * 16, kCols2 = 64 * 144, kA2 = 64 * 32, kCols3 = 16 * 288, kA3 = 16 * 32,
-              kH0 = 632, kA4 = 64, kLogits = kOut;
-static_assert(kCols1 + kA1 + kCols2 + kA2 + kCols3 + kA3 + kH0 + kA4 + kLogits == CELV2_PRUNER_ACTS, "cache size");
-// backward workspace, floats per sample
-constexpr int kDz4 = 64, kDh0 = 512, kDcols3 = 4608, kDz2 = 2048, kDcols2 = 9216, kDz1 = 4096;
-static_assert(kDz4 + kDh0 + kDcols3 + kDz2 + kDcols2 + kDz1 == CELV2_PRUNER_WORK, "workspace size");
+// forward cache, floats per sample: the image, the convolutions' outputs (the last with the other
+// features behind it), the hidden layer; the logits are the buffer's last
+constexpr int kXs = 256, kA1 = 256 * 16, kA2 = 64 * 32, kH0 = 632, kA4 = 64, kLogits = kOut;
+static_assert(kXs + kA1 + kA2 + kH0 + kA4 + kLogits + 4 <= CELV2_PRUNER_ACTS, "cache size");
+// backward workspace, floats per sample: gradients at the hidden layer and at the last convolution
+constexpr int kDz4 = 64, kDz3 = 512;
+static_assert(kDz4 + kDz3 + 4 <= CELV2_PRUNER_WORK, "workspace size");
 
+// The caller's buffers are floats at any address: the segments start at the first 16-byte boundary.
+template <typename T>
+T* aligned16(T* p) {
+  return reinterpret_cast<T*>((reinterpret_cast<uintptr_t>(p) + 15) & ~uintptr_t(15));
+}
 struct Cache {  // the forward cache of a batch, segment by segment
-  float *cols1, *a1, *cols2, *a2, *cols3, *a3, *h0, *a4, *logits;
+  float *xs, *a1, *a2, *h0, *a4, *logits;
   Cache(float* base, long long b) {
-    cols1 = base;
-    a1 = cols1 + b * kCols1;
-    cols2 = a1 + b * kA1;
-    a2 = cols2 + b * kCols2;
-    cols3 = a2 + b * kA2;
-    a3 = cols3 + b * kCols3;
-    h0 = a3 + b * kA3;
+    xs = aligned16(base);
+    a1 = xs + b * kXs;
+    a2 = a1 + b * kA1;
+    h0 = a2 + b * kA2;
     a4 = h0 + b * kH0;
-    logits = a4 + b * kA4;
+    logits = base + b * (CELV2_PRUNER_ACTS - kLogits);
   }
 };
 
-// ---- GEMM: C[m][n] = act(sum_k bf16(A[m][k]) * bf16(B[k][n]) + bias[n]) (+ C if accumulate) ----
-// Element (m, k) of A at A[m * a_sm + k * a_sk], (k, n) of B at B[k * b_sk + n * b_sn], (m, n) of C
-// at C[m * c_sm + n * c_sn]: transposes are strides. CTA tile 64 x 64, four warps of 32 x 32, K in
-// steps of 16 staged as BF16 in shared memory; out-of-range elements load as zero.
-constexpr int kTm = 64, kTn = 64, kTk = 16, kPad = 8;
+using bf16 = __nv_bfloat16;
 
-// Split K (gridDim.z > 1): CTA z takes K range [z * kc, (z + 1) * kc) and adds its partial sums
-// atomically into C (zero beforehand; no ReLU; the bias comes from z == 0).
-__global__ void __launch_bounds__(128) k_gemm(int M, int N, int K, const float* __restrict__ A, long long a_sm,
-                                              long long a_sk, const float* __restrict__ B, long long b_sk,
-                                              long long b_sn, float* C, long long c_sm, long long c_sn,
-                                              const float* __restrict__ bias, int relu, int accumulate, int kc) {
-  __shared__ __align__(16) __nv_bfloat16 As[kTm][kTk + kPad];  // [m][k]
-  __shared__ __align__(16) __nv_bfloat16 Bs[kTn][kTk + kPad];  // [n][k]
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int m0 = blockIdx.x * kTm, n0 = blockIdx.y * kTn;
-  const int kbeg = blockIdx.z * kc, kend = min(K, kbeg + kc);
-  const int wm = (warp >> 1) * 32, wn = (warp & 1) * 32;
-  const int g = lane >> 2, t = lane & 3;
-  float acc[2][4][4];
-#pragma unroll
-  for (int i = 0; i < 2; i++)
-#pragma unroll
-    for (int j = 0; j < 4; j++)
-#pragma unroll
-      for (int q = 0; q < 4; q++) acc[i][j][q] = 0.f;
-  for (int k0 = kbeg; k0 < kend; k0 += kTk) {
-#pragma unroll
-    for (int e = tid; e < kTm * kTk; e += 128) {
-      const int r = e / kTk, c = e % kTk, m = m0 + r, k = k0 + c;
-      As[r][c] = __float2bfloat16_rn(m < M && k < kend ? A[m * a_sm + k * a_sk] : 0.f);
-    }
-#pragma unroll
-    for (int e = tid; e < kTn * kTk; e += 128) {
-      const int r = e / kTk, c = e % kTk, n = n0 + r, k = k0 + c;
-      Bs[r][c] = __float2bfloat16_rn(n < N && k < kend ? B[k * b_sk + n * b_sn] : 0.f);
+__device__ __forceinline__ uint32_t pack2(float lo, float hi) {
+  const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
+  return *reinterpret_cast<const uint32_t*>(&v);
+}
+__device__ __forceinline__ float rbf(float v) { return __bfloat162float(__float2bfloat16_rn(v)); }
+
+__device__ __forceinline__ void mma16816(float* d, const uint32_t* a, uint32_t b0, uint32_t b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+
+// Four 8x8 matrices from shared memory, lane i giving the address of row i % 8 of matrix i / 8; T: each
+// transposed on the way.
+template <bool T>
+__device__ __forceinline__ void ldsm4(uint32_t* r, const bf16* p) {
+  const unsigned a = (unsigned)__cvta_generic_to_shared(p);
+  if (T)
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a) : "memory");
+  else
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(a) : "memory");
+}
+template <bool T>
+__device__ __forceinline__ void ldsm2(uint32_t* r, const bf16* p) {  // two, lanes 0-15's addresses
+  const unsigned a = (unsigned)__cvta_generic_to_shared(p);
+  if (T)
+    asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0,%1}, [%2];" : "=r"(r[0]), "=r"(r[1]) : "r"(a) : "memory");
+  else
+    asm volatile("ldmatrix.sync.aligned.m8n8.x2.shared.b16 {%0,%1}, [%2];" : "=r"(r[0]), "=r"(r[1]) : "r"(a) : "memory");
+}
+
+constexpr int kNnThreads = 256;
+// Row strides in shared memory, elements: 16 bytes more than the row, so that eight rows of a matrix
+// fall into different banks (or two by two where a stride-2 convolution skips rows).
+constexpr int kS1 = 24, kS2 = 40, kSw2 = 152, kSw3 = 296;
+
+// BF16 copies of the strided convolutions' weights, all threads; the caller's barrier follows.
+__device__ __forceinline__ void stage_conv_weights(const float* P, bf16* w2, bf16* w3) {
+  for (int i = threadIdx.x; i < 32 * 144; i += kNnThreads) w2[i / 144 * kSw2 + i % 144] = __float2bfloat16_rn(P[kW2 + i]);
+  for (int i = threadIdx.x; i < 32 * 288; i += kNnThreads) w3[i / 288 * kSw3 + i % 288] = __float2bfloat16_rn(P[kW3 + i]);
+}
+
+// The input position that tap (ky, kx) of a stride-2 convolution reads at output (oy, ox), as a row of
+// the H x H activation in shared memory; its row H * H is zero and stands for the padding.
+template <int H>
+__device__ __forceinline__ int tap_row(int oy, int ox, int ky, int kx) {
+  const int y = 2 * oy + ky - 1, x = 2 * ox + kx - 1;
+  return y >= 0 && y < H && x >= 0 && x < H ? y * H + x : H * H;
+}
+
+// ---- forward: the convolutions, two samples at a time ----
+struct FwdSmem {
+  bf16 w2[32 * kSw2], w3[32 * kSw3];
+  float w1[9][16], b1[16], b2[32], b3[32];
+  float x[2][18][18];        // the images, BF16-rounded, with a border of zeros
+  bf16 a1[2][257][kS1], a2[2][65][kS2];
+};
+
+__global__ void __launch_bounds__(kNnThreads, 3) k_conv_forward(const float* __restrict__ P, const float* __restrict__ X,
+                                                                int batch, float* xs, float* a1g, float* a2g, float* h0) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  FwdSmem& S = *reinterpret_cast<FwdSmem*>(smem_raw);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+  stage_conv_weights(P, S.w2, S.w3);
+  if (tid < 144) S.w1[tid % 9][tid / 9] = rbf(P[kW1 + tid]);
+  if (tid < 16) S.b1[tid] = P[kB1 + tid];
+  if (tid < 32) S.b2[tid] = P[kB2 + tid], S.b3[tid] = P[kB3 + tid];
+  for (int i = tid; i < 2 * 18 * 18; i += kNnThreads) (&S.x[0][0][0])[i] = 0.f;
+  if (tid < 2 * kS1) S.a1[tid / kS1][256][tid % kS1] = __float2bfloat16_rn(0.f);
+  if (tid < 2 * kS2) S.a2[tid / kS2][64][tid % kS2] = __float2bfloat16_rn(0.f);
+  __syncthreads();
+  for (int b0 = 2 * blockIdx.x; b0 < batch; b0 += 2 * gridDim.x) {
+    const int nb = min(2, batch - b0);
+    for (int i = tid; i < nb * kF; i += kNnThreads) {
+      const int s = i / kF, k = i - s * kF;
+      const float v = X[(long long)(b0 + s) * kF + k];
+      if (k < 256) {
+        xs[(long long)(b0 + s) * kXs + k] = v;
+        S.x[s][1 + (k >> 4)][1 + (k & 15)] = rbf(v);
+      } else {
+        h0[(long long)(b0 + s) * kH0 + 256 + k] = v;  // features 256 .. 375 behind the 512 of the convolution
+      }
     }
     __syncthreads();
-    uint32_t af[2][4], bfr[4][2];
+    {  // 3x3, 1 -> 16: a thread a position, its nine samples against all sixteen channels
+      const int y = tid >> 4, x = tid & 15;
+#pragma unroll 1
+      for (int s = 0; s < 2; s++) {
+        float acc[16];
 #pragma unroll
-    for (int i = 0; i < 2; i++) {
-      const int r = wm + i * 16 + g;
-      af[i][0] = *reinterpret_cast<const uint32_t*>(&As[r][2 * t]);
-      af[i][1] = *reinterpret_cast<const uint32_t*>(&As[r + 8][2 * t]);
-      af[i][2] = *reinterpret_cast<const uint32_t*>(&As[r][2 * t + 8]);
-      af[i][3] = *reinterpret_cast<const uint32_t*>(&As[r + 8][2 * t + 8]);
+        for (int c = 0; c < 16; c++) acc[c] = 0.f;
+#pragma unroll 1
+        for (int ky = 0; ky < 3; ky++)
+#pragma unroll
+          for (int kx = 0; kx < 3; kx++) {
+            const float v = S.x[s][y + ky][x + kx];
+#pragma unroll
+            for (int c = 0; c < 16; c++) acc[c] += v * S.w1[3 * ky + kx][c];
+          }
+        uint32_t h[8];
+#pragma unroll
+        for (int c = 0; c < 16; c++) acc[c] = fmaxf(acc[c] + S.b1[c], 0.f);
+#pragma unroll
+        for (int c = 0; c < 8; c++) h[c] = pack2(acc[2 * c], acc[2 * c + 1]);
+        uint4* row = reinterpret_cast<uint4*>(S.a1[s][tid]);
+        row[0] = make_uint4(h[0], h[1], h[2], h[3]), row[1] = make_uint4(h[4], h[5], h[6], h[7]);
+        if (s < nb) {
+          float4* o = reinterpret_cast<float4*>(a1g + (long long)(b0 + s) * kA1 + tid * 16);
+#pragma unroll
+          for (int c = 0; c < 4; c++) o[c] = make_float4(acc[4 * c], acc[4 * c + 1], acc[4 * c + 2], acc[4 * c + 3]);
+        }
+      }
     }
+    __syncthreads();
+    const int s = warp >> 2, q = warp & 3;  // the warp's sample, and its quarter of the work
+    {  // 3x3 stride 2, 16 -> 32: 16 output positions a warp
+      float acc[4][4] = {};
+      const int pos = q * 16 + (lane & 15), kc = (lane >> 4) * 8;
+      for (int k = 0; k < 9; k++) {
+        uint32_t a[4], w[8];
+        ldsm4<false>(a, &S.a1[s][tap_row<16>(pos >> 3, pos & 7, k / 3, k % 3)][kc]);
+        const bf16* wp = S.w2 + ((lane & 7) + (lane >> 4) * 8) * kSw2 + k * 16 + ((lane >> 3) & 1) * 8;
+        ldsm4<false>(w, wp);
+        ldsm4<false>(w + 4, wp + 16 * kSw2);
 #pragma unroll
-    for (int j = 0; j < 4; j++) {
-      const int n = wn + j * 8 + g;
-      bfr[j][0] = *reinterpret_cast<const uint32_t*>(&Bs[n][2 * t]);
-      bfr[j][1] = *reinterpret_cast<const uint32_t*>(&Bs[n][2 * t + 8]);
-    }
-#pragma unroll
-    for (int i = 0; i < 2; i++)
+        for (int j = 0; j < 4; j++) mma16816(acc[j], a, w[2 * j], w[2 * j + 1]);
+      }
 #pragma unroll
       for (int j = 0; j < 4; j++)
-        asm volatile(
-            "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
-            "{%0,%1,%2,%3};"
-            : "+f"(acc[i][j][0]), "+f"(acc[i][j][1]), "+f"(acc[i][j][2]), "+f"(acc[i][j][3])
-            : "r"(af[i][0]), "r"(af[i][1]), "r"(af[i][2]), "r"(af[i][3]), "r"(bfr[j][0]), "r"(bfr[j][1]));
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+          const int r = q * 16 + g + 8 * h, n = j * 8 + 2 * t;
+          const float v0 = fmaxf(acc[j][2 * h] + S.b2[n], 0.f), v1 = fmaxf(acc[j][2 * h + 1] + S.b2[n + 1], 0.f);
+          *reinterpret_cast<uint32_t*>(&S.a2[s][r][n]) = pack2(v0, v1);
+          if (s < nb) *reinterpret_cast<float2*>(a2g + (long long)(b0 + s) * kA2 + r * 32 + n) = make_float2(v0, v1);
+        }
+    }
     __syncthreads();
+    {  // 3x3 stride 2, 32 -> 32: eight channels a warp
+      float acc[4] = {};
+      const int pos = lane & 15, kc = (lane >> 4) * 8;
+      for (int k = 0; k < 9; k++) {
+        uint32_t a[4], w[4];
+        const bf16* row = S.a2[s][tap_row<8>(pos >> 2, pos & 3, k / 3, k % 3)];
+        ldsm4<false>(w, S.w3 + (q * 8 + (lane & 7)) * kSw3 + k * 32 + (lane >> 3) * 8);
+        ldsm4<false>(a, row + kc);
+        mma16816(acc, a, w[0], w[1]);
+        ldsm4<false>(a, row + 16 + kc);
+        mma16816(acc, a, w[2], w[3]);
+      }
+      if (s < nb) {
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+          const int r = g + 8 * h, n = q * 8 + 2 * t;
+          *reinterpret_cast<float2*>(h0 + (long long)(b0 + s) * kH0 + r * 32 + n) =
+              make_float2(fmaxf(acc[2 * h] + S.b3[n], 0.f), fmaxf(acc[2 * h + 1] + S.b3[n + 1], 0.f));
+        }
+      }
+    }
+  }
+}
+
+// ---- forward: the dense layers, 32 samples a CTA ----
+constexpr int kRows = 32, kKc = 128;  // samples a CTA; the first layer's inputs a step
+struct DenseSmem {
+  bf16 h0[kRows][648];         // inputs 632 .. 639 zero
+  bf16 w4[64][kKc + 8];
+  bf16 a4[kRows][72], w5[24][72];
+};
+
+__global__ void __launch_bounds__(kNnThreads) k_dense_forward(const float* __restrict__ P, const float* __restrict__ h0,
+                                                              int batch, float* a4g, float* logits) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  DenseSmem& S = *reinterpret_cast<DenseSmem*>(smem_raw);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+  const int b0 = blockIdx.x * kRows, mt = warp & 1, np = warp >> 1;  // the warp's 16 samples, 16 outputs
+#pragma unroll 5
+  for (int i = tid; i < kRows * 160; i += kNnThreads) {  // four inputs at a time (h0's rows are 16-byte aligned)
+    const int r = i / 160, k = 4 * (i - r * 160);
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (b0 + r < batch && k < kH0) v = *reinterpret_cast<const float4*>(h0 + (long long)(b0 + r) * kH0 + k);
+    *reinterpret_cast<uint2*>(&S.h0[r][k]) = make_uint2(pack2(v.x, v.y), pack2(v.z, v.w));
+  }
+  for (int i = tid; i < 24 * 64; i += kNnThreads) S.w5[i >> 6][i & 63] = __float2bfloat16_rn(P[kW5 + i]);
+  float acc[2][4] = {};
+  for (int k0 = 0; k0 < 640; k0 += kKc) {
+    __syncthreads();
+#pragma unroll 16
+    for (int i = tid; i < 64 * kKc; i += kNnThreads) {
+      const int o = i / kKc, k = i - o * kKc;
+      S.w4[o][k] = __float2bfloat16_rn(k0 + k < kH0 ? P[kW4 + o * kH0 + k0 + k] : 0.f);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < kKc; k += 16) {
+      uint32_t a[4], w[4];
+      ldsm4<false>(a, &S.h0[mt * 16 + (lane & 15)][k0 + k + (lane >> 4) * 8]);
+      ldsm4<false>(w, &S.w4[np * 16 + (lane & 7) + (lane >> 4) * 8][k + ((lane >> 3) & 1) * 8]);
+      mma16816(acc[0], a, w[0], w[1]);
+      mma16816(acc[1], a, w[2], w[3]);
+    }
   }
 #pragma unroll
-  for (int i = 0; i < 2; i++)
+  for (int j = 0; j < 2; j++)
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+      const int r = mt * 16 + g + 8 * h, n = np * 16 + j * 8 + 2 * t;
+      const float v0 = fmaxf(acc[j][2 * h] + P[kB4 + n], 0.f), v1 = fmaxf(acc[j][2 * h + 1] + P[kB4 + n + 1], 0.f);
+      *reinterpret_cast<uint32_t*>(&S.a4[r][n]) = pack2(v0, v1);
+      if (b0 + r < batch) *reinterpret_cast<float2*>(a4g + (long long)(b0 + r) * kA4 + n) = make_float2(v0, v1);
+    }
+  __syncthreads();
+  if (np < 3) {  // 64 -> 24
+    float z[4] = {};
+#pragma unroll
+    for (int k = 0; k < 64; k += 16) {
+      uint32_t a[4], w[2];
+      ldsm4<false>(a, &S.a4[mt * 16 + (lane & 15)][k + (lane >> 4) * 8]);
+      ldsm2<false>(w, &S.w5[np * 8 + (lane & 7)][k + ((lane >> 3) & 1) * 8]);
+      mma16816(z, a, w[0], w[1]);
+    }
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      const int r = b0 + mt * 16 + g + (q >> 1) * 8, n = np * 8 + 2 * t + (q & 1);
+      if (r < batch) logits[(long long)r * kOut + n] = z[q] + P[kB5 + n];
+    }
+  }
+}
+
+// ---- backward: the dense layers' input gradients, 32 samples a CTA ----
+struct DenseBackSmem {
+  bf16 dl[kRows][40], w5[32][72];  // outputs 24 .. 31 zero
+  bf16 dz4[kRows][72], w4[64][kKc + 8];
+};
+
+// dz4 = dlogits W5 where the hidden unit is positive; dz3 = dz4 W4 (its first 512 inputs) where the
+// convolution's output is.
+__global__ void __launch_bounds__(kNnThreads) k_dense_backward(const float* __restrict__ P, const float* __restrict__ dlogits,
+                                                               const float* __restrict__ a4g, const float* __restrict__ h0,
+                                                               int batch, float* dz4g, float* dz3g) {
+  __shared__ __align__(16) DenseBackSmem S;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+  const int b0 = blockIdx.x * kRows, mt = warp & 1, np = warp >> 1;
+  for (int i = tid; i < kRows * 32; i += kNnThreads) {
+    const int r = i >> 5, k = i & 31;
+    S.dl[r][k] = __float2bfloat16_rn(b0 + r < batch && k < kOut ? dlogits[(long long)(b0 + r) * kOut + k] : 0.f);
+  }
+  for (int i = tid; i < 32 * 64; i += kNnThreads) S.w5[i >> 6][i & 63] = __float2bfloat16_rn(i < kOut * 64 ? P[kW5 + i] : 0.f);
+  __syncthreads();
+  {
+    float acc[2][4] = {};
+#pragma unroll
+    for (int k = 0; k < 32; k += 16) {
+      uint32_t a[4], w[4];
+      ldsm4<false>(a, &S.dl[mt * 16 + (lane & 15)][k + (lane >> 4) * 8]);
+      ldsm4<true>(w, &S.w5[k + (lane & 15)][np * 16 + (lane >> 4) * 8]);
+      mma16816(acc[0], a, w[0], w[1]);
+      mma16816(acc[1], a, w[2], w[3]);
+    }
+#pragma unroll
+    for (int j = 0; j < 2; j++)
+#pragma unroll
+      for (int h = 0; h < 2; h++) {
+        const int r = mt * 16 + g + 8 * h, n = np * 16 + j * 8 + 2 * t;
+        float2 m = make_float2(0.f, 0.f);
+        const long long o = (long long)(b0 + r) * kA4 + n;
+        if (b0 + r < batch) m = *reinterpret_cast<const float2*>(a4g + o);
+        const float v0 = m.x > 0.f ? acc[j][2 * h] : 0.f, v1 = m.y > 0.f ? acc[j][2 * h + 1] : 0.f;
+        *reinterpret_cast<uint32_t*>(&S.dz4[r][n]) = pack2(v0, v1);
+        if (b0 + r < batch) *reinterpret_cast<float2*>(dz4g + o) = make_float2(v0, v1);
+      }
+  }
+  for (int n0 = 0; n0 < 512; n0 += kKc) {
+    __syncthreads();
+#pragma unroll 16
+    for (int i = tid; i < 64 * kKc; i += kNnThreads) {
+      const int o = i / kKc, k = i - o * kKc;
+      S.w4[o][k] = __float2bfloat16_rn(P[kW4 + o * kH0 + n0 + k]);
+    }
+    __syncthreads();
+    float acc[4][4] = {};
+#pragma unroll
+    for (int k = 0; k < 64; k += 16) {
+      uint32_t a[4], w[8];
+      ldsm4<false>(a, &S.dz4[mt * 16 + (lane & 15)][k + (lane >> 4) * 8]);
+      const bf16* wp = &S.w4[k + (lane & 15)][np * 32 + (lane >> 4) * 8];
+      ldsm4<true>(w, wp);
+      ldsm4<true>(w + 4, wp + 16);
+#pragma unroll
+      for (int j = 0; j < 4; j++) mma16816(acc[j], a, w[2 * j], w[2 * j + 1]);
+    }
 #pragma unroll
     for (int j = 0; j < 4; j++)
 #pragma unroll
-      for (int q = 0; q < 4; q++) {
-        const int m = m0 + wm + i * 16 + g + (q >> 1) * 8, n = n0 + wn + j * 8 + 2 * t + (q & 1);
-        if (m >= M || n >= N) continue;
-        float v = acc[i][j][q] + (bias && blockIdx.z == 0 ? bias[n] : 0.f);
-        float* dst = C + m * c_sm + n * c_sn;
-        if (gridDim.z > 1) {
-          atomicAdd(dst, v);
-          continue;
-        }
-        if (relu) v = fmaxf(v, 0.f);
-        *dst = accumulate ? *dst + v : v;
+      for (int h = 0; h < 2; h++) {
+        const int r = b0 + mt * 16 + g + 8 * h, n = n0 + np * 32 + j * 8 + 2 * t;
+        if (r >= batch) continue;
+        const float2 m = *reinterpret_cast<const float2*>(h0 + (long long)r * kH0 + n);
+        *reinterpret_cast<float2*>(dz3g + (long long)r * kDz3 + n) =
+            make_float2(m.x > 0.f ? acc[j][2 * h] : 0.f, m.y > 0.f ? acc[j][2 * h + 1] : 0.f);
       }
-}
-
-// split > 1: C must hold zeros (or the sum to add to), and no ReLU.
-void gemm(int M, int N, int K, const float* A, long long a_sm, long long a_sk, const float* B, long long b_sk,
-          long long b_sn, float* C, long long c_sm, long long c_sn, const float* bias, bool relu, bool accumulate,
-          cudaStream_t st, int split = 1) {
-  const int kc = ((K + split - 1) / split + kTk - 1) / kTk * kTk;
-  const dim3 grid((M + kTm - 1) / kTm, (N + kTn - 1) / kTn, (K + kc - 1) / kc);
-  k_gemm<<<grid, 128, 0, st>>>(M, N, K, A, a_sm, a_sk, B, b_sk, b_sn, C, c_sm, c_sn, bias, relu, accumulate, kc);
-}
-
-// The K split of a weight-gradient GEMM (long K = batch x positions, small M x N): ~2048 per CTA.
-int wsplit(long long K) {
-  const long long s = (K + 2047) / 2048;
-  return (int)(s < 1 ? 1 : s > 1024 ? 1024 : s);
-}
-
-// ---- im2col / col2im for 3x3 convolutions, padding 1, NHWC activations ----
-// cols[(b * Ho + oy) * Wo + ox][(ky * 3 + kx) * C + c] = X[b][oy * s + ky - 1][ox * s + kx - 1][c]
-__global__ void k_im2col(const float* __restrict__ X, long long sample_stride, int H, int W, int C, int s,
-                         float* __restrict__ cols, long long total) {
-  const int Ho = (H - 1) / s + 1, Wo = (W - 1) / s + 1, K = 9 * C;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
-    const long long row = i / K;
-    const int col = (int)(i - row * K), tap = col / C, c = col - tap * C, ky = tap / 3, kx = tap - ky * 3;
-    const long long b = row / (Ho * Wo);
-    const int p = (int)(row - b * Ho * Wo), oy = p / Wo, ox = p - oy * Wo;
-    const int y = oy * s + ky - 1, x = ox * s + kx - 1;
-    cols[i] = (y >= 0 && y < H && x >= 0 && x < W) ? X[b * sample_stride + ((long long)y * W + x) * C + c] : 0.f;
   }
 }
 
-// dX[b][y][x][c] = sum of dcols over the (output position, tap) pairs that read (y, x)
-__global__ void k_col2im(const float* __restrict__ dcols, int H, int W, int C, int s, float* __restrict__ dX,
-                         long long total) {
-  const int Ho = (H - 1) / s + 1, Wo = (W - 1) / s + 1, K = 9 * C;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
-    const long long b = i / ((long long)H * W * C);
-    const int r = (int)(i - b * H * W * C), c = r % C, px = r / C, y = px / W, x = px - y * W;
-    float sum = 0.f;
-    for (int ky = 0; ky < 3; ky++) {
-      const int ty = y + 1 - ky;
-      if (ty < 0 || ty % s) continue;
-      const int oy = ty / s;
-      if (oy >= Ho) continue;
-      for (int kx = 0; kx < 3; kx++) {
-        const int tx = x + 1 - kx;
-        if (tx < 0 || tx % s) continue;
-        const int ox = tx / s;
-        if (ox >= Wo) continue;
-        sum += dcols[((b * Ho + oy) * Wo + ox) * K + (ky * 3 + kx) * C + c];
+// ---- backward: a dense layer's weight and bias gradients ----
+// G[m][n] += sum over samples b of D[b][m] H[b][n] (m < M <= 64, n < N), B[m] += sum of D[b][m] (FP32). CTA
+// (x, y): columns 64 x .., samples y * per ..
+__global__ void __launch_bounds__(kNnThreads) k_dense_weights(const float* __restrict__ D, int M, const float* __restrict__ H,
+                                                              int N, int batch, int per, float* G, float* B) {
+  __shared__ __align__(16) bf16 Ds[64][72], Hs[64][72];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+  const int n0 = blockIdx.x * 64, b1 = min(batch, (int)(blockIdx.y + 1) * per), mt = warp & 3, nh = warp >> 2;
+  const int col = tid & 63;
+  float acc[4][4] = {}, bias = 0.f;
+  for (int b0 = blockIdx.y * per; b0 < b1; b0 += 64) {
+    __syncthreads();
+#pragma unroll 8
+    for (int r = tid >> 6; r < 64; r += 4) {
+      const long long b = b0 + r;
+      const float d = b < b1 && col < M ? D[b * M + col] : 0.f;
+      Ds[r][col] = __float2bfloat16_rn(d);
+      Hs[r][col] = __float2bfloat16_rn(b < b1 && n0 + col < N ? H[b * N + n0 + col] : 0.f);
+      bias += d;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < 64; k += 16) {
+      uint32_t a[4], w[8];
+      ldsm4<true>(a, &Ds[k + (lane & 7) + (lane >> 4) * 8][mt * 16 + ((lane >> 3) & 1) * 8]);
+      const bf16* wp = &Hs[k + (lane & 15)][nh * 32 + (lane >> 4) * 8];
+      ldsm4<true>(w, wp);
+      ldsm4<true>(w + 4, wp + 16);
+#pragma unroll
+      for (int j = 0; j < 4; j++) mma16816(acc[j], a, w[2 * j], w[2 * j + 1]);
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < 4; j++)
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+      const int m = mt * 16 + g + (q >> 1) * 8, n = n0 + nh * 32 + j * 8 + 2 * t + (q & 1);
+      if (m < M && n < N) atomicAdd(G + m * N + n, acc[j][q]);
+    }
+  if (blockIdx.x == 0 && col < M) atomicAdd(B + col, bias);
+}
+
+// ---- backward: the convolutions, a sample at a time, their weight gradients over a CTA's samples ----
+struct BackSmem {
+  bf16 w2[32 * kSw2], w3[32 * kSw3];
+  bf16 a1[257][kS1], a2[65][kS2], dz3[17][kS2], dz2[65][kS2], dz1[256][kS1];
+  bf16 cols[256][kS1];      // the first convolution's columns (nine taps, then zeros)
+  float x[18][18];
+  float bias[16 + 32 + 32];
+};
+
+__global__ void __launch_bounds__(kNnThreads, 2) k_conv_backward(const float* __restrict__ P, const float* __restrict__ xs,
+                                                                 const float* __restrict__ a1g, const float* __restrict__ a2g,
+                                                                 const float* __restrict__ dz3g, int batch, float* G) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  BackSmem& S = *reinterpret_cast<BackSmem*>(smem_raw);
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+  stage_conv_weights(P, S.w2, S.w3);
+  const bf16 zero = __float2bfloat16_rn(0.f);
+  if (tid < kS1) S.a1[256][tid] = zero;
+  if (tid < kS2) S.a2[64][tid] = S.dz3[16][tid] = S.dz2[64][tid] = zero;
+  if (tid < 80) S.bias[tid] = 0.f;
+  for (int i = tid; i < 18 * 18; i += kNnThreads) (&S.x[0][0])[i] = 0.f;
+  for (int i = tid; i < 256 * 16; i += kNnThreads) S.cols[i >> 4][i & 15] = zero;
+  // this warp's share: weight gradients of 16 output channels (m2) and a run of 8-column tiles
+  const int m2 = warp & 1, q = warp >> 1, t2 = q < 2 ? 5 * q : 10 + 4 * (q - 2), n2 = q < 2 ? 5 : 4;
+  float g3[9][4] = {}, g2[5][4] = {}, g1[2][4] = {};
+  float s3[2] = {}, s2[2] = {}, s1[4] = {};  // bias sums
+  for (int b = blockIdx.x; b < batch; b += gridDim.x) {
+    __syncthreads();  // the sample before is done with
+    {
+      const float4* v = reinterpret_cast<const float4*>(a1g + (long long)b * kA1);
+#pragma unroll
+      for (int i = 0; i < 4; i++) {
+        const int e = tid + i * kNnThreads;
+        const float4 f = v[e];
+        *reinterpret_cast<uint2*>(&S.a1[e >> 2][(e & 3) * 4]) = make_uint2(pack2(f.x, f.y), pack2(f.z, f.w));
+      }
+      const float4* u = reinterpret_cast<const float4*>(a2g + (long long)b * kA2);
+#pragma unroll
+      for (int i = 0; i < 2; i++) {
+        const int e = tid + i * kNnThreads;
+        const float4 f = u[e];
+        *reinterpret_cast<uint2*>(&S.a2[e >> 3][(e & 7) * 4]) = make_uint2(pack2(f.x, f.y), pack2(f.z, f.w));
+      }
+      const float2 d = reinterpret_cast<const float2*>(dz3g + (long long)b * kDz3)[tid];
+      *reinterpret_cast<uint32_t*>(&S.dz3[tid >> 4][(tid & 15) * 2]) = pack2(d.x, d.y);
+      s3[0] += d.x, s3[1] += d.y;
+      S.x[1 + (tid >> 4)][1 + (tid & 15)] = xs[(long long)b * kXs + tid];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < 9; k++) S.cols[tid][k] = __float2bfloat16_rn(S.x[(tid >> 4) + k / 3][(tid & 15) + k % 3]);
+    {  // W3's gradient: dz3^T (32 x 16 positions) against the columns of a2, nine tiles a warp
+      uint32_t a[4];
+      ldsm4<true>(a, &S.dz3[(lane & 7) + (lane >> 4) * 8][m2 * 16 + ((lane >> 3) & 1) * 8]);
+      const int pos = lane & 15;
+#pragma unroll
+      for (int j = 0; j < 9; j++) {
+        const int n = q * 9 + j, k = n >> 2;
+        uint32_t w[2];
+        ldsm2<true>(w, &S.a2[tap_row<8>(pos >> 2, pos & 3, k / 3, k % 3)][(n & 3) * 8]);
+        mma16816(g3[j], a, w[0], w[1]);
       }
     }
-    dX[i] = sum;
+    // dz2: the gradient at a2, eight channels a warp. A position of the 8 x 8 map is read by the taps
+    // whose parity is its own: even rows by ky = 1 alone, odd ones by ky = 0 (from the output below) and
+    // 2 (from the one above), columns likewise -- four classes of 16 positions with 1, 2, 2 and 4 taps,
+    // the last to one half of the warps, the others to the other half
+    {
+      const int nt = warp & 3, r = lane & 15, cy = r >> 2, cx = r & 3;
+      for (int c = warp < 4 ? 3 : 0; c < (warp < 4 ? 4 : 3); c++) {
+        const int py = c >> 1, px = c & 1;
+        float acc[4] = {};
+        for (int i = 0; i <= py; i++)
+          for (int j = 0; j <= px; j++) {
+            // output (cy + dy, cx + dx): the tap's own for an even position, for an odd one 0 -> below / right
+            const int ky = py ? 2 * i : 1, kx = px ? 2 * j : 1, oy = cy + (py && i == 0), ox = cx + (px && j == 0);
+            const bf16* row = S.dz3[oy < 4 && ox < 4 ? oy * 4 + ox : 16];
+            const bf16* wp = S.w3 + (lane & 15) * kSw3 + (ky * 3 + kx) * 32 + nt * 8;
+            uint32_t a[4], w[2];
+            ldsm4<false>(a, row + (lane >> 4) * 8);
+            ldsm2<true>(w, wp);
+            mma16816(acc, a, w[0], w[1]);
+            ldsm4<false>(a, row + 16 + (lane >> 4) * 8);
+            ldsm2<true>(w, wp + 16 * kSw3);
+            mma16816(acc, a, w[0], w[1]);
+          }
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+          const int pr = g + 8 * h, p = (2 * (pr >> 2) + py) * 8 + 2 * (pr & 3) + px, n = nt * 8 + 2 * t;
+          const uint32_t m = *reinterpret_cast<const uint32_t*>(&S.a2[p][n]);  // (ReLU outputs: positive or zero)
+          const float v0 = m & 0xffffu ? acc[2 * h] : 0.f, v1 = m >> 16 ? acc[2 * h + 1] : 0.f;
+          *reinterpret_cast<uint32_t*>(&S.dz2[p][n]) = pack2(v0, v1);
+          s2[0] += v0, s2[1] += v1;
+        }
+      }
+    }
+    __syncthreads();
+    // W2's gradient: dz2^T (32 x 64 positions) against the columns of a1
+#pragma unroll
+    for (int kk = 0; kk < 4; kk++) {
+      uint32_t a[4];
+      ldsm4<true>(a, &S.dz2[kk * 16 + (lane & 7) + (lane >> 4) * 8][m2 * 16 + ((lane >> 3) & 1) * 8]);
+      const int pos = kk * 16 + (lane & 15);
+#pragma unroll
+      for (int j = 0; j < 5; j++) {
+        if (j >= n2) break;
+        const int n = t2 + j, k = n >> 1;
+        uint32_t w[2];
+        ldsm2<true>(w, &S.a1[tap_row<16>(pos >> 3, pos & 7, k / 3, k % 3)][(n & 1) * 8]);
+        mma16816(g2[j], a, w[0], w[1]);
+      }
+    }
+    // dz1: the gradient at a1, 16 positions of a class (two of its eight rows) and all 16 channels a warp
+    {
+      const int mt = warp & 3, r = mt * 16 + (lane & 15), cy = r >> 3, cx = r & 7;
+      for (int c = warp < 4 ? 3 : 0; c < (warp < 4 ? 4 : 3); c++) {
+        const int py = c >> 1, px = c & 1;
+        float acc[2][4] = {};
+        for (int i = 0; i <= py; i++)
+          for (int j = 0; j <= px; j++) {
+            const int ky = py ? 2 * i : 1, kx = px ? 2 * j : 1, oy = cy + (py && i == 0), ox = cx + (px && j == 0);
+            const bf16* row = S.dz2[oy < 8 && ox < 8 ? oy * 8 + ox : 64];
+            const bf16* wp = S.w2 + (lane & 15) * kSw2 + (ky * 3 + kx) * 16 + (lane >> 4) * 8;
+            uint32_t a[4], w[4];
+#pragma unroll
+            for (int k = 0; k < 32; k += 16) {
+              ldsm4<false>(a, row + k + (lane >> 4) * 8);
+              ldsm4<true>(w, wp + k * kSw2);
+              mma16816(acc[0], a, w[0], w[1]);
+              mma16816(acc[1], a, w[2], w[3]);
+            }
+          }
+#pragma unroll
+        for (int j = 0; j < 2; j++)
+#pragma unroll
+          for (int h = 0; h < 2; h++) {
+            const int pr = mt * 16 + g + 8 * h, p = (2 * (pr >> 3) + py) * 16 + 2 * (pr & 7) + px, n = j * 8 + 2 * t;
+            const uint32_t m = *reinterpret_cast<const uint32_t*>(&S.a1[p][n]);
+            const float v0 = m & 0xffffu ? acc[j][2 * h] : 0.f, v1 = m >> 16 ? acc[j][2 * h + 1] : 0.f;
+            *reinterpret_cast<uint32_t*>(&S.dz1[p][n]) = pack2(v0, v1);
+            s1[2 * j] += v0, s1[2 * j + 1] += v1;
+          }
+      }
+    }
+    __syncthreads();
+    // W1's gradient: dz1^T (16 x 256 positions) against the image's columns, 32 positions a warp
+#pragma unroll
+    for (int kk = 2 * warp; kk < 2 * warp + 2; kk++) {
+      uint32_t a[4], w[4];
+      ldsm4<true>(a, &S.dz1[kk * 16 + (lane & 7) + (lane >> 4) * 8][((lane >> 3) & 1) * 8]);
+      ldsm4<true>(w, &S.cols[kk * 16 + (lane & 15)][(lane >> 4) * 8]);
+      mma16816(g1[0], a, w[0], w[1]);
+      mma16816(g1[1], a, w[2], w[3]);
+    }
   }
-}
-
-// h0[b] = a3[b] (512) ++ x[b][256 .. 376)
-__global__ void k_concat(const float* __restrict__ a3, const float* __restrict__ x, float* __restrict__ h0, long long total) {
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
-    const long long b = i / kH0;
-    const int k = (int)(i - b * kH0);
-    h0[i] = k < 512 ? a3[b * 512 + k] : x[b * kF + 256 + (k - 512)];
+  __syncthreads();
+  // everything into the gradient vector
+#pragma unroll
+  for (int e = 0; e < 4; e++) {
+    const int m = m2 * 16 + g + (e >> 1) * 8, c = 2 * t + (e & 1);
+#pragma unroll
+    for (int j = 0; j < 9; j++) atomicAdd(G + kW3 + m * 288 + (q * 9 + j) * 8 + c, g3[j][e]);
+#pragma unroll
+    for (int j = 0; j < 5; j++)
+      if (j < n2) atomicAdd(G + kW2 + m * 144 + (t2 + j) * 8 + c, g2[j][e]);
+    const int m1 = g + (e >> 1) * 8;
+    atomicAdd(G + kW1 + m1 * 9 + c, g1[0][e]);
+    if (c == 0) atomicAdd(G + kW1 + m1 * 9 + 8, g1[1][e]);
   }
-}
-
-__global__ void k_relu(float* a, long long n) {
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-    a[i] = fmaxf(a[i], 0.f);
-}
-
-// dz = da where the activation is positive (ReLU backward; in place allowed)
-__global__ void k_relu_bwd(const float* __restrict__ act, const float* da, float* dz, long long n) {
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-    dz[i] = act[i] > 0.f ? da[i] : 0.f;
-}
-
-// db[n] += sum over rows of dz[m][n] (N <= 64 columns, one thread each; blocks take row strides)
-__global__ void k_colsum(const float* __restrict__ dz, long long M, int N, float* db) {
-  const int n = threadIdx.x;
-  if (n >= N) return;
-  float s = 0.f;
-  for (long long m = blockIdx.x; m < M; m += gridDim.x) s += dz[m * N + n];
-  atomicAdd(db + n, s);
+  atomicAdd(&S.bias[48 + 2 * (tid & 15)], s3[0]), atomicAdd(&S.bias[48 + 2 * (tid & 15) + 1], s3[1]);
+  atomicAdd(&S.bias[16 + (warp & 3) * 8 + 2 * t], s2[0]), atomicAdd(&S.bias[16 + (warp & 3) * 8 + 2 * t + 1], s2[1]);
+#pragma unroll
+  for (int j = 0; j < 4; j++) atomicAdd(&S.bias[(j >> 1) * 8 + 2 * t + (j & 1)], s1[j]);
+  __syncthreads();
+  if (tid < 16) atomicAdd(G + kB1 + tid, S.bias[tid]);
+  if (tid < 32) atomicAdd(G + kB2 + tid, S.bias[16 + tid]), atomicAdd(G + kB3 + tid, S.bias[48 + tid]);
 }
 
 __global__ void k_bce(const float* __restrict__ z, const float* __restrict__ y, const float* __restrict__ w, int n,
@@ -248,59 +616,37 @@ int grid_for(long long n) {
   return (int)(g < 148 * 16 ? (g < 1 ? 1 : g) : 148 * 16);
 }
 
+// CTAs of a kernel that loops over its samples: as many as the GPU holds, at most `units`.
+template <typename K>
+int resident(K kernel, size_t smem, int units) {
+  cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  return persistent_grid((const void*)kernel, kNnThreads, smem, units);
+}
+
 void forward(const float* P, const float* x, int batch, float* acts, cudaStream_t st) {
-  const long long b = batch;
-  Cache c(acts, b);
-  k_im2col<<<grid_for(b * kCols1), 256, 0, st>>>(x, kF, 16, 16, 1, 1, c.cols1, b * kCols1);
-  gemm((int)(b * 256), 16, 9, c.cols1, 9, 1, P + kW1, 1, 9, c.a1, 16, 1, P + kB1, true, false, st);
-  k_im2col<<<grid_for(b * kCols2), 256, 0, st>>>(c.a1, kA1, 16, 16, 16, 2, c.cols2, b * kCols2);
-  gemm((int)(b * 64), 32, 144, c.cols2, 144, 1, P + kW2, 1, 144, c.a2, 32, 1, P + kB2, true, false, st);
-  k_im2col<<<grid_for(b * kCols3), 256, 0, st>>>(c.a2, kA2, 8, 8, 32, 2, c.cols3, b * kCols3);
-  gemm((int)(b * 16), 32, 288, c.cols3, 288, 1, P + kW3, 1, 288, c.a3, 32, 1, P + kB3, true, false, st);
-  k_concat<<<grid_for(b * kH0), 256, 0, st>>>(c.a3, x, c.h0, b * kH0);
-  // the dense layer's K (632) in 8 slices on separate CTAs (few rows, many columns of K), then ReLU
-  cudaMemsetAsync(c.a4, 0, (size_t)b * kA4 * sizeof(float), st);
-  gemm(batch, 64, 632, c.h0, 632, 1, P + kW4, 1, 632, c.a4, 64, 1, P + kB4, false, false, st, 8);
-  k_relu<<<grid_for(b * kA4), 256, 0, st>>>(c.a4, b * kA4);
-  gemm(batch, kOut, 64, c.a4, 64, 1, P + kW5, 1, 64, c.logits, kOut, 1, P + kB5, false, false, st);
+  Cache c(acts, batch);
+  const int grid = resident(k_conv_forward, sizeof(FwdSmem), (batch + 1) / 2);
+  k_conv_forward<<<grid, kNnThreads, sizeof(FwdSmem), st>>>(P, x, batch, c.xs, c.a1, c.a2, c.h0);
+  const int blocks = (batch + kRows - 1) / kRows;
+  resident(k_dense_forward, sizeof(DenseSmem), blocks);
+  k_dense_forward<<<blocks, kNnThreads, sizeof(DenseSmem), st>>>(P, c.h0, batch, c.a4, c.logits);
 }
 
 void backward(const float* P, int batch, const float* acts, const float* dlogits, float* work, float* G,
               cudaStream_t st) {
-  const long long b = batch;
-  Cache c(const_cast<float*>(acts), b);
-  float* dz4 = work;
-  float* dh0 = dz4 + b * kDz4;
-  float* dcols3 = dh0 + b * kDh0;
-  float* dz2 = dcols3 + b * kDcols3;
-  float* dcols2 = dz2 + b * kDz2;
-  float* dz1 = dcols2 + b * kDcols2;
-  cudaMemsetAsync(G, 0, kParams * sizeof(float), st);  // the bias sums accumulate
-  // dense 64 -> kOut
-  gemm(kOut, 64, batch, dlogits, 1, kOut, c.a4, 64, 1, G + kW5, 64, 1, nullptr, false, false, st, wsplit(b));
-  k_colsum<<<grid_for(b), 64, 0, st>>>(dlogits, b, kOut, G + kB5);
-  gemm(batch, 64, kOut, dlogits, kOut, 1, P + kW5, 64, 1, dz4, 64, 1, nullptr, false, false, st);
-  k_relu_bwd<<<grid_for(b * 64), 256, 0, st>>>(c.a4, dz4, dz4, b * 64);
-  // dense 632 -> 64 (the gradient reaches only the convolution part of its input)
-  gemm(64, 632, batch, dz4, 1, 64, c.h0, 632, 1, G + kW4, 632, 1, nullptr, false, false, st, wsplit(b));
-  k_colsum<<<grid_for(b), 64, 0, st>>>(dz4, b, 64, G + kB4);
-  gemm(batch, 512, 64, dz4, 64, 1, P + kW4, 632, 1, dh0, 512, 1, nullptr, false, false, st);
-  k_relu_bwd<<<grid_for(b * 512), 256, 0, st>>>(c.a3, dh0, dh0, b * 512);  // dz3, (b * 16) x 32
-  // conv 32 -> 32, stride 2
-  gemm(32, 288, (int)(b * 16), dh0, 1, 32, c.cols3, 288, 1, G + kW3, 288, 1, nullptr, false, false, st, wsplit(b * 16));
-  k_colsum<<<grid_for(b * 16), 64, 0, st>>>(dh0, b * 16, 32, G + kB3);
-  gemm((int)(b * 16), 288, 32, dh0, 32, 1, P + kW3, 288, 1, dcols3, 288, 1, nullptr, false, false, st);
-  k_col2im<<<grid_for(b * kDz2), 256, 0, st>>>(dcols3, 8, 8, 32, 2, dz2, b * kDz2);
-  k_relu_bwd<<<grid_for(b * kDz2), 256, 0, st>>>(c.a2, dz2, dz2, b * kDz2);
-  // conv 16 -> 32, stride 2
-  gemm(32, 144, (int)(b * 64), dz2, 1, 32, c.cols2, 144, 1, G + kW2, 144, 1, nullptr, false, false, st, wsplit(b * 64));
-  k_colsum<<<grid_for(b * 64), 64, 0, st>>>(dz2, b * 64, 32, G + kB2);
-  gemm((int)(b * 64), 144, 32, dz2, 32, 1, P + kW2, 144, 1, dcols2, 144, 1, nullptr, false, false, st);
-  k_col2im<<<grid_for(b * kDz1), 256, 0, st>>>(dcols2, 16, 16, 16, 2, dz1, b * kDz1);
-  k_relu_bwd<<<grid_for(b * kDz1), 256, 0, st>>>(c.a1, dz1, dz1, b * kDz1);
-  // conv 1 -> 16
-  gemm(16, 9, (int)(b * 256), dz1, 1, 16, c.cols1, 9, 1, G + kW1, 9, 1, nullptr, false, false, st, wsplit(b * 256));
-  k_colsum<<<grid_for(b * 256), 64, 0, st>>>(dz1, b * 256, 16, G + kB1);
+  Cache c(const_cast<float*>(acts), batch);
+  float* dz4 = aligned16(work);
+  float* dz3 = dz4 + (long long)batch * kDz4;
+  cudaMemsetAsync(G, 0, kParams * sizeof(float), st);  // every gradient is a sum of CTAs' sums
+  const int blocks = (batch + kRows - 1) / kRows;
+  k_dense_backward<<<blocks, kNnThreads, 0, st>>>(P, dlogits, c.a4, c.h0, batch, dz4, dz3);
+  // the dense layers' weights: 256 samples a CTA for the first (ten column tiles), 64 for the second
+  k_dense_weights<<<dim3((kH0 + 63) / 64, (batch + 255) / 256), kNnThreads, 0, st>>>(dz4, 64, c.h0, kH0, batch, 256,
+                                                                                     G + kW4, G + kB4);
+  k_dense_weights<<<dim3(1, (batch + 63) / 64), kNnThreads, 0, st>>>(dlogits, kOut, c.a4, 64, batch, 64, G + kW5,
+                                                                      G + kB5);
+  const int grid = resident(k_conv_backward, sizeof(BackSmem), batch);
+  k_conv_backward<<<grid, kNnThreads, sizeof(BackSmem), st>>>(P, c.xs, c.a1, c.a2, dz3, batch, G);
 }
 
 }  // namespace nn
@@ -422,15 +768,6 @@ __global__ void k_infer_weights(const float* __restrict__ P, __nv_bfloat16* __re
     }
     Wb[i] = __float2bfloat16_rn(v);
   }
-}
-
-__device__ __forceinline__ float rbf(float v) { return __bfloat162float(__float2bfloat16_rn(v)); }
-
-__device__ __forceinline__ void mma16816(float* d, const uint32_t* a, uint32_t b0, uint32_t b1) {
-  asm volatile(
-      "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
 __global__ void __launch_bounds__(128) k_infer(const float* __restrict__ P, const __nv_bfloat16* __restrict__ Wb,
