@@ -15,6 +15,8 @@
 //    pinned memory before it returns (the reference requires that the inputs may change at once,
 //    decision_engine.h:12-16).
 // No CPU fallback: every decision is made by the kernels; a missing GPU is an error.
+#include <cuda.h>
+#include <cudaTypedefs.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -117,6 +119,33 @@ void init_device(int dev) {
 
 size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
+// The phase planes at `mem` -- rows of `stride` bytes, `rows` a plane, planes `plane` bytes apart -- as a
+// tensor whose boxes are the inter stage's windows (inter_window). cuTensorMapEncodeTiled is the driver's,
+// looked up once (the library links the runtime alone).
+TensorMap phase_map(void* mem, int stride, int rows, size_t plane) {
+  static const PFN_cuTensorMapEncodeTiled_v12000 encode = [] {
+    void* f = nullptr;
+    cudaDriverEntryPointQueryResult q = cudaDriverEntryPointSymbolNotFound;
+    if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &f, 12000, cudaEnableDefault, &q) != cudaSuccess ||
+        q != cudaDriverEntryPointSuccess)
+      f = nullptr;
+    return reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(f);
+  }();
+  if (!encode) throw Error(CELV2_ECUDA, "cuTensorMapEncodeTiled: not in this driver");
+  const cuuint64_t dim[3] = {(cuuint64_t)stride, (cuuint64_t)rows, (cuuint64_t)kPhases};
+  const cuuint64_t bytes[2] = {(cuuint64_t)stride, (cuuint64_t)plane};
+  cuuint32_t box[3] = {0, 0, 1}, step[3] = {1, 1, 1};
+  inter_window(box[0], box[1]);
+  CUtensorMap m;
+  const CUresult r = encode(&m, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, mem, dim, bytes, box, step, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                            CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) throw Error(CELV2_ECUDA, "cuTensorMapEncodeTiled: error " + std::to_string((int)r));
+  TensorMap t;
+  static_assert(sizeof t == sizeof m, "a tensor map is 128 bytes");
+  std::memcpy(&t, &m, sizeof t);
+  return t;
+}
+
 // Geometry of one frame size: padded luma, pyramid levels, fields, superblocks.
 struct Geometry {
   int width = 0, height = 0, pw = 0, ph = 0;
@@ -165,6 +194,7 @@ struct Slot {
   uint8_t* mem = nullptr;
   size_t bytes = 0;
   DevPyramid pyr{};
+  TensorMap map{};  // its phase planes (room for them), box k_inter's window
 };
 
 // One pinned staging buffer with its device copy (an upload in flight).
@@ -262,7 +292,8 @@ struct celv2_engine {
   cudaStream_t copy_st = nullptr;
   cudaStream_t up_st = nullptr;  // celv2_upload's stream (frame-store uploads)
   cudaStream_t fin_st = nullptr;  // the finalize of a batch in slices (high priority; st waits for it)
-  cudaEvent_t slice_ready[8] = {}, slice_done[8] = {};  // per slice (kMaxSlices)
+  cudaStream_t side_st = nullptr;  // every other slice's inter stage
+  cudaEvent_t front_done = nullptr, slice_ready[8] = {}, slice_done[8] = {};  // per slice (kMaxSlices)
   static constexpr int kRecordSets = 3;
   cudaEvent_t copied[kRecordSets] = {};
   bool copy_pending[kRecordSets] = {};
@@ -284,6 +315,7 @@ struct celv2_engine {
   static constexpr int kQueuePrep = 0, kQueueMe = 1, kQueueRefine = kQueueMe + kLevels, kQueueSlice = kQueueRefine + 1;
   static constexpr int kMaxSlices = 8, kQueues = kQueueSlice + 4 * kMaxSlices;
   unsigned* queues = nullptr;
+  int* fault = nullptr;  // behind the ring, page-locked: set by a kernel whose wait for its copies ran out
   bool persistent = true;      // the queue-draining persistent stage kernels (else one CTA per unit)
   unsigned persistent_off = 0; // stages (bit i: queue i) that run one CTA per unit anyway
   int me_cells[kLevels] = {30, 30, 30, 30, 30};
@@ -344,6 +376,7 @@ struct celv2_engine {
     if (prep_st) cudaStreamSynchronize(prep_st);
     if (copy_st) cudaStreamSynchronize(copy_st);
     if (up_st) cudaStreamSynchronize(up_st);
+    if (side_st) cudaStreamSynchronize(side_st);
     if (fin_st) cudaStreamSynchronize(fin_st);
     free_graphs();
     for (Slot* s : store) free_slot(s);
@@ -381,7 +414,9 @@ struct celv2_engine {
     if (prep_st) cudaStreamDestroy(prep_st);
     if (copy_st) cudaStreamDestroy(copy_st);
     if (up_st) cudaStreamDestroy(up_st);
+    if (side_st) cudaStreamDestroy(side_st);
     if (fin_st) cudaStreamDestroy(fin_st);
+    if (front_done) cudaEventDestroy(front_done);
   }
 
   static void free_slot(Slot* s) {
@@ -430,7 +465,9 @@ struct celv2_engine {
     CK(cudaEventCreateWithFlags(&slice_done[0], cudaEventDisableTiming));
     CK(cudaMalloc(&djobs, kRingJobs * sizeof(FrameJob)));
     CK(cudaMalloc(&queues, kQueues * sizeof(unsigned)));
-    CK(cudaMallocHost(&ring, (size_t)kRing * kRingJobs * sizeof(FrameJob)));
+    CK(cudaMallocHost(&ring, (size_t)kRing * kRingJobs * sizeof(FrameJob) + sizeof(int)));
+    fault = reinterpret_cast<int*>(ring + (size_t)kRing * kRingJobs);
+    *fault = 0;
     for (cudaEvent_t& e : ring_done) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     alloc_buffers(single, false);
     for (int*& p : intra_prep) CK(cudaMalloc(&p, (size_t)g.nsb * kBlocks * kModes * sizeof(int)));
@@ -461,6 +498,7 @@ struct celv2_engine {
       p.phase = l == 0 && phases ? (long long)g.level_bytes[0] : 0;
     }
     s.phases = false;
+    if (phases) s.map = phase_map(s.mem, g.stride[0], g.h[0] + 2 * g.margin[0], g.level_bytes[0]);
   }
 
   // A staging buffer of at least `bytes`: the first one whose last use is over, so that few of them
@@ -614,7 +652,8 @@ struct celv2_engine {
                 const int* intra, long long lam) {
     std::memset(&job, 0, sizeof job);
     job.cur = cur;
-    for (int r = 0; r < nrefs; r++) job.ref[r] = refs[r]->pyr;
+    for (int r = 0; r < nrefs; r++) job.ref[r] = refs[r]->pyr, job.map[r] = refs[r]->map;
+    job.fault = fault;
     job.nrefs = nrefs;
     job.pw = g.pw, job.ph = g.ph;
     job.sb_cols = g.sb_cols, job.sb_rows = g.sb_rows;
@@ -676,9 +715,8 @@ struct celv2_engine {
   // superblocks has its inter stage and finalize run slice by slice, the copies of one behind the
   // stages of the next. A slice is worth it from kSliceSbs superblocks on: 5 MB, ~90 us of copy,
   // against the ~30 us that the drained ends of its launches cost. Five 1080p leaves of 7 references
-  // in 1 / 2 / 3 / 5 / 8 slices: 7.81 / 7.78 / 7.25 / 6.83 / 6.70 ms; one masked 4K frame 3.30 / 3.17
-  // / 3.12 / 3.09 / 3.09; one 1080p frame of 7 references (4 slices at most) 2.27 / 2.11 / 2.15 /
-  // 2.17 / 2.15.
+  // in 2 / 4 / 8 slices: 7.29 / 6.47 / 6.08 ms; ten 720p leaves of 2 3.90 / 3.64 / 3.54; one masked 4K
+  // frame 3.24 / 3.17 / 3.17; a 1080p frame of the encoder's loop (3 at most) 2.01 / 1.94 / 2.0.
   static constexpr int kSliceSbs = 128;
   static std::vector<Slice> cut(const std::vector<SbRange>& rows, bool to_host) {
     int total = 0;
@@ -836,14 +874,17 @@ struct celv2_engine {
       if (!slice_ready[i]) CK(cudaEventCreateWithFlags(&slice_ready[i], cudaEventDisableTiming));
     for (int i = 1; i < kMaxSlices; i++)
       if (!slice_done[i]) CK(cudaEventCreateWithFlags(&slice_done[i], cudaEventDisableTiming));
+    if (!front_done) CK(cudaEventCreateWithFlags(&front_done, cudaEventDisableTiming));
+    if (!side_st) CK(cudaStreamCreateWithFlags(&side_st, cudaStreamNonBlocking));
     CK(cudaStreamCreateWithPriority(&fin_st, cudaStreamNonBlocking, greatest));
   }
 
   // The stages of a batch on st, its descriptors sent through the pinned ring (graph: the part up to
   // the slices replayed as a CUDA graph). done(i, stream) is called once slice i's records are queued
-  // on `stream` -- to queue their copies. Several slices: the inter stage of one runs while the
-  // finalize of the one before it, on a stream of higher priority, takes the SMs the drained inter
-  // launch leaves; st waits for the last finalize.
+  // on `stream` -- to queue their copies. Several slices: their inter stages go to two streams in turn, so
+  // one's CTAs take the SMs that the drained launch before it leaves (in one stream eight slices of five
+  // 1080p leaves spent 2.07 ms in the stage that takes 1.60 in one launch), and their finalize to a third
+  // of higher priority; st waits for the last finalize.
   template <typename F>
   void run(const std::vector<FrameJob>& jobs, cudaEvent_t intra_done, const std::vector<NetJob>& nets,
            const std::vector<Slice>& slices, bool graph, F&& done) {
@@ -861,10 +902,13 @@ struct celv2_engine {
     make_fin_stream();
     const bool intra_here = !intra_done && !any_refs(jobs);
     if (intra_done) CK(cudaStreamWaitEvent(fin_st, intra_done, 0));
+    CK(cudaEventRecord(front_done, st));
+    CK(cudaStreamWaitEvent(side_st, front_done, 0));
     for (int i = 0; i < n; i++) {
-      if (intra_here) kernel_launches += enqueue_intra(jobs, slices[i], i, st);
-      kernel_launches += enqueue_inter(jobs, slices[i], i, st);
-      CK(cudaEventRecord(slice_ready[i], st));
+      cudaStream_t s = i & 1 ? side_st : st;
+      if (intra_here) kernel_launches += enqueue_intra(jobs, slices[i], i, s);
+      kernel_launches += enqueue_inter(jobs, slices[i], i, s);
+      CK(cudaEventRecord(slice_ready[i], s));
       CK(cudaStreamWaitEvent(fin_st, slice_ready[i], 0));
       kernel_launches += enqueue_finalize(jobs, slices[i], i, fin_st);
       CK(cudaEventRecord(slice_done[i], fin_st));
@@ -881,6 +925,10 @@ struct celv2_engine {
     if (!timed.empty()) {
       CK(cudaStreamSynchronize(prep_st));
       harvest();
+    }
+    if (*static_cast<volatile int*>(fault)) {
+      *fault = 0;
+      throw Error(CELV2_ECUDA, "a kernel's wait for its copies ran out: the last batch is not decided");
     }
   }
 
@@ -971,6 +1019,7 @@ struct celv2_engine {
       pending = true;
     } catch (...) {
       cudaStreamSynchronize(st);  // a failure leaves no work running
+      if (side_st) cudaStreamSynchronize(side_st);
       if (fin_st) cudaStreamSynchronize(fin_st);
       cudaStreamSynchronize(copy_st);
       cudaStreamSynchronize(prep_st);

@@ -91,6 +91,9 @@ void launch_intra(const FrameJob* jobs, const WorkList& w, cudaStream_t st);
 void launch_inter(const FrameJob* jobs, const WorkList& w, int chunk, bool regions, unsigned* region_queue,
                   cudaStream_t st);
 
+// The window the inter stage loads of a phase plane for a motion vector (its box): bytes, rows.
+void inter_window(unsigned& bytes, unsigned& rows);
+
 // Per-block choice, compound, partition choice and the decision records. Units: the parts' superblocks.
 void launch_finalize(const FrameJob* jobs, const WorkList& w, cudaStream_t st);
 

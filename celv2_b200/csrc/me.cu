@@ -354,7 +354,9 @@ __global__ void __launch_bounds__(kMeThreads, 4) k_me_level(const FrameJob* __re
 constexpr int kRefineCells = 32, kRefineTiles = 4, kRefineThreads = 32 * kRefineTiles;
 
 __global__ void __launch_bounds__(kRefineThreads, 8) k_me_refine(const FrameJob* __restrict__ jobs, WorkList w) {
-  __shared__ int sat[2][9][kRefineTiles][kRefineCells];  // [step][position][tile][cell]
+  // [step][pair][tile][cell]: the SATDs of positions 2 pair + 1 and 2 pair + 2 in halfwords (a cell's four
+  // tiles sum to at most 65,280), and of the first step's centre
+  __shared__ uint32_t sat[2][4][kRefineTiles][kRefineCells], sat0[kRefineTiles][kRefineCells];
   __shared__ int unit_slot;
   const int tid = threadIdx.x, c = tid & 31, t = tid >> 5;
   int unit, iter = 0;
@@ -397,53 +399,66 @@ __global__ void __launch_bounds__(kRefineThreads, 8) k_me_refine(const FrameJob*
       uint32_t pr[5], lf[5], rt[5];
 #pragma unroll
       for (int i = 0; i < 4; i++) pr[i] = load4(p00 + i * rs);
-      sat[0][0][t][c] = satd4_rows(C, pr);  // the centre, phase (0, 0)
+      sat0[t][c] = (uint32_t)satd4_rows(C, pr);  // the centre, phase (0, 0)
       const uint8_t* p20 = p00 + 8 * ref.phase;  // phase (2, 0): rows Y - 1 .. Y + 3
 #pragma unroll
       for (int i = 0; i < 5; i++) pr[i] = load4(p20 + (i - 1) * rs);
-      sat[0][2][t][c] = satd4_rows(C, pr);      // (0, -1/2)
-      sat[0][7][t][c] = satd4_rows(C, pr + 1);  // (0, +1/2)
+      const uint32_t v27 = satd4_pair(C, pr, pr + 1);  // positions 2 and 7: (0, -1/2), (0, +1/2)
       const uint8_t* p02 = p00 + 2 * ref.phase - 1;  // phase (0, 2): columns X - 1 .. X + 3
 #pragma unroll
       for (int i = 0; i < 4; i++) load_pair(p02 + i * rs, lf[i], rt[i]);
-      sat[0][4][t][c] = satd4_rows(C, lf);  // (-1/2, 0)
-      sat[0][5][t][c] = satd4_rows(C, rt);  // (+1/2, 0)
+      const uint32_t v45 = satd4_pair(C, lf, rt);  // 4 and 5: (-1/2, 0), (+1/2, 0)
       const uint8_t* p22 = p00 + 10 * ref.phase - 1;  // phase (2, 2): both
 #pragma unroll
       for (int i = 0; i < 5; i++) load_pair(p22 + (i - 1) * rs, lf[i], rt[i]);
-      sat[0][1][t][c] = satd4_rows(C, lf);      // (-1/2, -1/2)
-      sat[0][3][t][c] = satd4_rows(C, rt);      // (+1/2, -1/2)
-      sat[0][6][t][c] = satd4_rows(C, lf + 1);  // (-1/2, +1/2)
-      sat[0][8][t][c] = satd4_rows(C, rt + 1);  // (+1/2, +1/2)
+      const uint32_t v13 = satd4_pair(C, lf, rt);          // 1 and 3: (-1/2, -1/2), (+1/2, -1/2)
+      const uint32_t v68 = satd4_pair(C, lf + 1, rt + 1);  // 6 and 8: (-1/2, +1/2), (+1/2, +1/2)
+      sat[0][0][t][c] = __byte_perm(v13, v27, 0x5410);
+      sat[0][1][t][c] = __byte_perm(v13, v45, 0x5432);
+      sat[0][2][t][c] = __byte_perm(v45, v68, 0x5432);
+      sat[0][3][t][c] = __byte_perm(v27, v68, 0x7632);
     } else {
+      // four rows at position k (the second step's centre, k = 0, is the first step's winner)
+      auto rows_at = [&](int k, uint32_t* pr) {
+        const int n = refine_pos(k);
+        const int qx = cx + (n % 3 - 1) * step, qy = cy + (n / 3 - 1) * step;
+        DevPlane ph = ref;
+        ph.p = ref.p + (long long)((qy & 3) * 4 + (qx & 3)) * ref.phase;
+        const int x = ox + (qx >> 2), y = oy + (qy >> 2);
+        if (inside(ph, x, y, 4, 4)) {
+          const uint8_t* p = ph.p + (long long)y * ph.stride + x;
 #pragma unroll
-    for (int k = s; k < 9; k++) {  // the second step's centre (k = 0) is the first step's winner
-      const int n = refine_pos(k);
-      const int qx = cx + (n % 3 - 1) * step, qy = cy + (n / 3 - 1) * step;
-      DevPlane ph = ref;
-      ph.p = ref.p + (long long)((qy & 3) * 4 + (qx & 3)) * ref.phase;
-      const int x = ox + (qx >> 2), y = oy + (qy >> 2);
-      uint32_t pr[4];
-      if (inside(ph, x, y, 4, 4)) {
-        const uint8_t* p = ph.p + (long long)y * ph.stride + x;
+          for (int i = 0; i < 4; i++) pr[i] = load4(p + (long long)i * ph.stride);
+        } else {
 #pragma unroll
-        for (int i = 0; i < 4; i++) pr[i] = load4(p + (long long)i * ph.stride);
-      } else {
-#pragma unroll
-        for (int i = 0; i < 4; i++) pr[i] = row4(ph, x, y + i);
+          for (int i = 0; i < 4; i++) pr[i] = row4(ph, x, y + i);
+        }
+      };
+      if (s == 0) {
+        uint32_t pr[4];
+        rows_at(0, pr);
+        sat0[t][c] = (uint32_t)satd4_rows(C, pr);
       }
-      sat[s][k][t][c] = satd4_rows(C, pr);
-    }
+#pragma unroll
+      for (int k = 0; k < 4; k++) {
+        uint32_t pa[4], pb[4];
+        rows_at(2 * k + 1, pa);
+        rows_at(2 * k + 2, pb);
+        sat[s][k][t][c] = satd4_pair(C, pa, pb);
+      }
     }
     __syncthreads();
     // the cell's choice (me_refine: the centre first, a move must save kSubpelPenalty)
-    int best = s == 0 ? sat[0][0][0][c] + sat[0][0][1][c] + sat[0][0][2][c] + sat[0][0][3][c] : centre;
+    int best = s == 0 ? (int)(sat0[0][c] + sat0[1][c] + sat0[2][c] + sat0[3][c]) : centre;
     int raw = best, nx = cx, ny = cy;
 #pragma unroll
-    for (int k = 1; k < 9; k++) {
-      const int v = sat[s][k][0][c] + sat[s][k][1][c] + sat[s][k][2][c] + sat[s][k][3][c];
-      const int n = refine_pos(k);
-      if (v + kSubpelPenalty < best) best = v + kSubpelPenalty, raw = v, nx = cx + (n % 3 - 1) * step, ny = cy + (n / 3 - 1) * step;
+    for (int k = 0; k < 4; k++) {
+      const uint32_t two = sat[s][k][0][c] + sat[s][k][1][c] + sat[s][k][2][c] + sat[s][k][3][c];
+#pragma unroll
+      for (int h = 0; h < 2; h++) {
+        const int v = (int)(h ? two >> 16 : two & 0xffffu), n = refine_pos(2 * k + 1 + h);
+        if (v + kSubpelPenalty < best) best = v + kSubpelPenalty, raw = v, nx = cx + (n % 3 - 1) * step, ny = cy + (n / 3 - 1) * step;
+      }
     }
     centre = raw, cx = nx, cy = ny;
   }
