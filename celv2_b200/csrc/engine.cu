@@ -764,13 +764,16 @@ struct celv2_engine {
     w.nparts = n;
     for (int j = 0; j < n; j++) w.part[j] = SbRange{j, 0, jobs[j].sb_cols * jobs[j].sb_rows};
     for (int l = kLevels - 1; l >= 0; l--) {
+      long long total = 0;
+      for (const FrameJob& jb : jobs) total += (long long)jb.nrefs * jb.fcols[l] * jb.frows[l];
+      const int cells = me_level_cells(total, me_cells[l]);
       for (int j = 0; j < n; j++)
-        w.prefix[j + 1] = w.prefix[j] + me_units(jobs[j].nrefs, jobs[j].fcols[l], jobs[j].frows[l], me_cells[l]);
+        w.prefix[j + 1] = w.prefix[j] + me_units(jobs[j].nrefs, jobs[j].fcols[l], jobs[j].frows[l], cells);
       if (l == 0 && !nets.empty())  // the learned pruner, from the level-1 motion search
         stage(kStPruner, stream, [&] { launched += enqueue_pruner(jobs, nets, stream); });
       w.queue = queue(l, kQueueMe + l);
       if (w.prefix[n] > 0) {
-        stage(kStMe0 - l, stream, [&] { launch_me_level(djobs, w, l, me_cells[l], stream); });
+        stage(kStMe0 - l, stream, [&] { launch_me_level(djobs, w, l, cells, stream); });
         launched++;
       }
     }

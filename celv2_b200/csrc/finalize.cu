@@ -40,10 +40,10 @@ struct FinSmem {
 __global__ void __launch_bounds__(kFinThreads, 4) k_finalize(const FrameJob* __restrict__ jobs, WorkList w) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   FinSmem& S = *reinterpret_cast<FinSmem*>(smem_raw);
-  __shared__ int unit_slot;
+  __shared__ int unit_slot[2];
   const int tid = threadIdx.x;
   int unit, iter = 0;
-  while (take_unit(w, unit, iter, &unit_slot)) {
+  while (take_unit(w, unit, iter, unit_slot)) {
   const int jb = part_of(w, unit);
   const FrameJob& job = jobs[w.part[jb].job];
   const int sb = w.part[jb].sb0 + unit - w.prefix[jb], sby = sb / job.sb_cols, sbx = sb - sby * job.sb_cols;

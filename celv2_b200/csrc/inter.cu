@@ -282,7 +282,7 @@ __global__ void __launch_bounds__(kInterThreads* G, 4 / G) k_inter(const FrameJo
   PassSums Q;
   Q.cell = reinterpret_cast<uint2 (*)[64]>(ring + kRing * M * kWin);
   Q.sum16 = reinterpret_cast<int (*)[20]>(ring + kRing * M * kWin + pass * 512);
-  __shared__ int unit_slot;
+  __shared__ int unit_slot[2];
   const int tid = threadIdx.x, lane = tid & 31, half = tid >> 7, px = tid & 7, ty = (tid & 127) >> 3;
   const unsigned ring_s = (unsigned)__cvta_generic_to_shared(ring);
   const unsigned full_s = (unsigned)__cvta_generic_to_shared(S.full), empty_s = (unsigned)__cvta_generic_to_shared(S.empty);
@@ -293,7 +293,7 @@ __global__ void __launch_bounds__(kInterThreads* G, 4 / G) k_inter(const FrameJo
   __syncthreads();
   unsigned parity = 0;  // per ring slot: the parity of its next step's round (bit; over all units)
   int unit, iter = 0;
-  while (take_unit(w, unit, iter, &unit_slot)) {
+  while (take_unit(w, unit, iter, unit_slot)) {
   const int jb = part_of(w, unit);
   const FrameJob& job = jobs[w.part[jb].job];
   const int nsb = w.part[jb].sbs;
@@ -686,9 +686,9 @@ __global__ void __launch_bounds__(kInterThreads, 4) k_inter_regions(const FrameJ
   extern __shared__ __align__(16) unsigned char smem_raw[];
   RegionSmem& S = *reinterpret_cast<RegionSmem*>(smem_raw);
   const ChunkSums Q = chunk_sums(smem_raw, chunk);
-  __shared__ int unit_slot;
+  __shared__ int unit_slot[2];
   int unit, iter = 0;
-  while (take_unit(w, unit, iter, &unit_slot)) {
+  while (take_unit(w, unit, iter, unit_slot)) {
     const int jb = part_of(w, unit);
     const FrameJob& job = jobs[w.part[jb].job];
     const int nsb = w.part[jb].sbs;

@@ -148,10 +148,10 @@ __device__ __forceinline__ uint32_t z2_left(const uint32_t* tr, int l, int r0, i
 __global__ void __launch_bounds__(kIntraThreads, 4) k_intra(const FrameJob* __restrict__ jobs, WorkList w, int parts) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   IntraSmem& S = *reinterpret_cast<IntraSmem*>(smem_raw);
-  __shared__ int unit_slot;
+  __shared__ int unit_slot[2];
   const int tid = threadIdx.x;
   int unit, iter = 0;
-  while (take_unit(w, unit, iter, &unit_slot)) {
+  while (take_unit(w, unit, iter, unit_slot)) {
   const int jb = part_of(w, unit);
   const FrameJob& job = jobs[w.part[jb].job];
   const int u = unit - w.prefix[jb], usb = u / parts, part = u - usb * parts, sb = w.part[jb].sb0 + usb;

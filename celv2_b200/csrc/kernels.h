@@ -29,8 +29,8 @@ struct WorkList {
 };
 
 // The next unit of this CTA into `unit` (every thread gets it); false when the stage is done.
-// Starts with a barrier, so the previous unit's shared state is free for the next one. No CTA
-// ever waits for another: a drained queue simply ends the loop.
+// Starts with a barrier, so the previous unit's shared state is free for the next one (slot: two ints
+// of shared memory, used in turn). No CTA ever waits for another: a drained queue simply ends the loop.
 __device__ __forceinline__ bool take_unit(const WorkList& w, int& unit, int& iter, int* slot) {
   const int total = w.prefix[w.nparts];
   if (!w.queue) {
@@ -38,10 +38,10 @@ __device__ __forceinline__ bool take_unit(const WorkList& w, int& unit, int& ite
     unit = blockIdx.x;
     return unit < total;
   }
+  int* s = slot + (iter++ & 1);
+  if (threadIdx.x == 0) *s = (int)atomicAdd(w.queue, 1u);
   __syncthreads();
-  if (threadIdx.x == 0) *slot = (int)atomicAdd(w.queue, 1u);
-  __syncthreads();
-  unit = *slot;
+  unit = *s;
   return unit < total;
 }
 
@@ -73,8 +73,10 @@ void launch_phases(const PlaneSet& s, cudaStream_t st);
 
 // Motion search of one pyramid level for every (job, reference, 8x8 cell), whole-pel (level 0's
 // field in quarter pels). Units: me_units(nrefs, fcols[level], frows[level], cells) per job (groups
-// of `cells` cells of one reference; cells 16 or 32).
+// of `cells` cells of one reference; cells 7, 15 or 30).
 int me_units(int nrefs, int cols, int rows, int cells);
+// The cells per CTA to run a level of `cells` cells (all jobs and references) with, `configured` or fewer.
+int me_level_cells(long long cells, int configured);
 void launch_me_level(const FrameJob* jobs, const WorkList& w, int level, int cells, cudaStream_t st);
 // Level 0's quarter-pel refinement, in place. Units: refine_units(nrefs, fcols[0], frows[0]) per job.
 int refine_units(int nrefs, int cols, int rows);

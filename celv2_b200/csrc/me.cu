@@ -5,25 +5,30 @@
 // (:122-133), me_refine (:141-154), me_cell (:162-193); driven level by level, coarsest first,
 // as src/gpu/cpu_engine.cpp:68-83 does.
 //
-// One CTA per 30 (or 15) consecutive 8x8 cells of one (job, reference):
+// One CTA per 30 (15, 7) consecutive 8x8 cells of one (job, reference):
 //  A. the cells' cur blocks are staged in shared memory; one thread per (cell, predictor centre)
 //     computes the six centre SADs;
 //  B. one thread per cell replays the reference's sequential choice of the two best distinct
-//     centres, and the searches (one or two per cell) get their 24 x 32-byte reference windows
-//     staged in shared memory with aligned 8-byte loads;
+//     centres (a best centre of SAD below kMePenalty is the result: nothing else can cost less), and
+//     the searches (one or two per cell) get their 24 x 32-byte reference windows staged in shared
+//     memory, a warp a search, by aligned 8-byte copies;
 //  C. one thread per (search, dx) column slides down the window's 24 rows: each row's 8 bytes at
 //     column dx are loaded once (two funnel shifts of three words) and feed, with vabsdiff4, every
 //     one of the 17 dy accumulators whose 8x8 block covers that row -- 24 row loads instead of
 //     17 x 8 per column. The column's best (cost << 9 | raster index) goes to a shared atomicMin,
 //     which yields the reference's first strict minimum in dy-major order;
-// Level 0's quarter-pel refinement is its own kernel (k_me_refine): a warp per position of a step,
-// a lane per cell.
-// Integer ALU bound: 289 x 16 byte-SIMD absolute-difference accumulates per searched centre.
+// Level 0's quarter-pel refinement is its own kernel (k_me_refine).
+// Integer ALU bound: 289 x 16 byte-SIMD absolute-difference accumulates per searched centre. Level 0 of
+// five 1080p frames of 7 references 1.49 -> 1.25 ms (natural-like) and 0.50 -> 0.43 ms (animation-like,
+// 1.50 before the cells that need no search had none) with the windows staged a warp a search instead of
+// finding search, cell and place again for every 8 bytes; CTAs of 128 threads and 15 cells 1.62, the
+// next unit asked for ahead 1.28, the cells' places found per thread instead of behind a barrier 1.28.
+#include <climits>
+
 #include "kernels.h"
 
 namespace celv2cu {
 
-constexpr int kMeThreads = 256;
 constexpr int kWinRows = 24, kWinWords = 8;    // a window row: 32 bytes from an 8-byte boundary
 constexpr int kWinStride = kWinRows * kWinWords + 8;  // +8 words: neighbouring windows use other banks
 // A merged search: the two centres of a cell at most 2 apart in x and y searched as one union
@@ -32,18 +37,22 @@ constexpr int kWinStride = kWinRows * kWinWords + 8;  // +8 words: neighbouring 
 constexpr int kMergeMax = 2, kUnion = 17 + kMergeMax, kMWinRows = kUnion + 7, kMWinWords = 10;
 static_assert(kMWinRows * kMWinWords <= 2 * kWinStride, "a merged window fits two windows' space");
 
-// Shared state of a CTA of CELLS cells (15 or 30: fewer cells per CTA give small pyramid levels
-// more CTAs; the autotuner picks per level). Nearly every cell searches two centres, so a CTA's
+// Shared state of a CTA of CELLS cells (15 or 30 as configured, the autotuner picking per level; 7 in
+// small launches, see me_level_cells). Nearly every cell searches two centres, so a CTA's
 // search phase has about 2 x 17 x CELLS (search, column) items: 30 and 15 cells make 1,020 and 510,
 // four and two nearly full rounds of 256 threads (32 and 16 cells left a last round 25% and 12%
 // full).
 template <int CELLS>
 struct MeSmem {
   static constexpr int kSearches = 2 * CELLS;  // at most two centres per cell
-  uint32_t cur[CELLS][16];
+  alignas(16) uint32_t cur[CELLS][16];
+  int bx[CELLS], by[CELLS];  // the cells' blocks (samples)
   int csad[CELLS][6];
   int ccx[CELLS][6], ccy[CELLS][6];
-  int scell[kSearches], sx[kSearches], sy[kSearches], soff[kSearches];
+  int scell[kSearches], sx[kSearches], sy[kSearches];
+  // the window: its first staged sample (column on an 8-byte boundary, row), the search's first column
+  // in it, whether it lies inside the margin
+  int wx[kSearches], wy[kSearches], soff[kSearches], wok[kSearches];
   unsigned skey[kSearches];
   // merged searches (entries from the back of the list): the second centre and its key
   int sx2[kSearches], sy2[kSearches];
@@ -98,6 +107,15 @@ __device__ __forceinline__ int sad8(const uint32_t* c, const DevPlane& ref, int 
   return (int)s;
 }
 
+// A cell's 16 words from shared memory.
+__device__ __forceinline__ void load_cur(const uint32_t* c, uint32_t* cw) {
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    const uint4 v = reinterpret_cast<const uint4*>(c)[k];
+    cw[4 * k] = v.x, cw[4 * k + 1] = v.y, cw[4 * k + 2] = v.z, cw[4 * k + 3] = v.w;
+  }
+}
+
 // The 4-byte windows at p and p + 1 (any alignment) from two aligned 32-bit loads.
 __device__ __forceinline__ void load_pair(const uint8_t* p, uint32_t& lo4, uint32_t& hi4) {
   const uintptr_t a = reinterpret_cast<uintptr_t>(p);
@@ -110,15 +128,16 @@ __device__ __forceinline__ void load_pair(const uint8_t* p, uint32_t& lo4, uint3
 // The refinement step's position n (raster 0..8 with the centre, 4, visited first).
 __device__ __forceinline__ int refine_pos(int t) { return t == 0 ? 4 : (t <= 4 ? t - 1 : t); }
 
-template <int CELLS>
-__global__ void __launch_bounds__(kMeThreads, 4) k_me_level(const FrameJob* __restrict__ jobs, WorkList w, int level) {
+template <int CELLS, int kMeThreads>
+__global__ void __launch_bounds__(kMeThreads, 1024 / kMeThreads) k_me_level(const FrameJob* __restrict__ jobs, WorkList w, int level) {
   constexpr int kMeCells = CELLS;
+  static_assert(CELLS * 6 <= kMeThreads, "a thread per cell and centre");
   extern __shared__ __align__(16) unsigned char smem_raw[];
   MeSmem<CELLS>& S = *reinterpret_cast<MeSmem<CELLS>*>(smem_raw);
-  __shared__ int unit_slot;
+  __shared__ int unit_slot[2];
   const int tid = threadIdx.x;
   int unit, iter = 0;
-  while (take_unit(w, unit, iter, &unit_slot)) {
+  while (take_unit(w, unit, iter, unit_slot)) {
   const int jb = part_of(w, unit);
   const FrameJob& job = jobs[w.part[jb].job];
   const int cols = job.fcols[level], rows = job.frows[level], ncell = cols * rows;
@@ -129,32 +148,38 @@ __global__ void __launch_bounds__(kMeThreads, 4) k_me_level(const FrameJob* __re
   const DevPlane cur = job.cur.lv[level], ref = job.ref[r].lv[level];
 
   // ---- A. cur blocks, predictor centres and their SADs (me_cell, inter_common.h:164-186) ----
-  for (int e = tid; e < kMeCells * 16; e += kMeThreads) {
-    const int c = e >> 4, k = e & 15;
-    const int cell = cell0 + (c < ncells ? c : 0), by = cell / cols, bx = cell - by * cols;
-    S.cur[c][k] = row4(cur, bx * 8 + 4 * (k & 1), by * 8 + (k >> 1));
-  }
   if (tid < kMeCells) {
-    const int cell = cell0 + tid, by = cell / cols, bx = cell - by * cols;
+    const int cell = cell0 + (tid < ncells ? tid : 0), by = cell / cols, bx = cell - by * cols;
+    S.bx[tid] = bx * 8, S.by[tid] = by * 8;
     S.need[tid] = tid < ncells && (level != 0 || cell_needed(job, r, bx, by));
   }
   if (tid == 0) S.nsearch = 0, S.nmerged = 0;
   __syncthreads();
   const bool top = level == kLevels - 1;
+  // (a block overhangs the plane by at most 7 samples: inside the margin; rows and margins are multiples
+  // of 8 bytes)
+  for (int e = tid; e < kMeCells * 8; e += kMeThreads) {
+    const int c = e >> 3, i = e & 7;
+    const uint2 v = *reinterpret_cast<const uint2*>(cur.p + (long long)(S.by[c] + i) * cur.stride + S.bx[c]);
+    S.cur[c][2 * i] = v.x, S.cur[c][2 * i + 1] = v.y;
+  }
+  int cx = 0, cy = 0;  // this thread's centre, of cell tid / 6 (centre 5: zero)
   if (!top && tid < kMeCells * 6) {
     const int c = tid / 6, k = tid - c * 6;
-    if (c < ncells && S.need[c]) {
-      const int cell = cell0 + c, by = cell / cols, bx = cell - by * cols;
-      int cx = 0, cy = 0;  // k == 5: zero
-      if (k < 5) {
-        const int* pf = job.field[r][level + 1];
-        const int pcols = job.fcols[level + 1], prows = job.frows[level + 1];
-        const int ox = k == 1 ? -1 : k == 2 ? 1 : 0, oy = k == 3 ? -1 : k == 4 ? 1 : 0;
-        const int m = pf[clampi(by / 2 + oy, 0, prows - 1) * pcols + clampi(bx / 2 + ox, 0, pcols - 1)];
-        cx = 2 * mv_x(m), cy = 2 * mv_y(m);
-      }
+    if (k < 5 && S.need[c]) {
+      const int* pf = job.field[r][level + 1];
+      const int pcols = job.fcols[level + 1], prows = job.frows[level + 1];
+      const int ox = k == 1 ? -1 : k == 2 ? 1 : 0, oy = k == 3 ? -1 : k == 4 ? 1 : 0;
+      const int m = pf[clampi((S.by[c] >> 4) + oy, 0, prows - 1) * pcols + clampi((S.bx[c] >> 4) + ox, 0, pcols - 1)];
+      cx = 2 * mv_x(m), cy = 2 * mv_y(m);
+    }
+  }
+  __syncthreads();
+  if (!top && tid < kMeCells * 6) {
+    const int c = tid / 6, k = tid - c * 6;
+    if (S.need[c]) {
       S.ccx[c][k] = cx, S.ccy[c][k] = cy;
-      S.csad[c][k] = sad8(S.cur[c], ref, bx * 8 + cx, by * 8 + cy);
+      S.csad[c][k] = sad8(S.cur[c], ref, S.bx[c] + cx, S.by[c] + cy);
     }
   }
   __syncthreads();
@@ -165,72 +190,83 @@ __global__ void __launch_bounds__(kMeThreads, 4) k_me_level(const FrameJob* __re
     const int c = tid;
     int px = 0, py = 0, px2 = 0, py2 = 0;
     bool two = false;
+    int best = 0x7fffffff;
     if (!top) {
-      int best = 0x7fffffff, second = 0x7fffffff;
+      int second = 0x7fffffff;
       for (int k = 0; k < 6; k++) {
-        const int cx = S.ccx[c][k], cy = S.ccy[c][k], s = S.csad[c][k];
-        if ((k > 0 && cx == px && cy == py) || (two && cx == px2 && cy == py2)) continue;
-        if (s < best) {
+        const int x = S.ccx[c][k], y = S.ccy[c][k], v = S.csad[c][k];
+        if ((k > 0 && x == px && y == py) || (two && x == px2 && y == py2)) continue;
+        if (v < best) {
           if (k > 0) second = best, px2 = px, py2 = py, two = true;
-          best = s, px = cx, py = cy;
-        } else if (s < second) {
-          second = s, px2 = cx, py2 = cy, two = true;
+          best = v, px = x, py = y;
+        } else if (v < second) {
+          second = v, px2 = x, py2 = y, two = true;
         }
       }
     }
-    const int cell = cell0 + c, by = cell / cols, bx = cell - by * cols;
-    if (two && abs(px - px2) <= kMergeMax && abs(py - py2) <= kMergeMax) {
+    // search s's window of `bytes` x `rows` around (x, y) - kMeRange
+    auto window = [&](int s, int x, int y, int bytes, int rows_) {
+      const int x0 = S.bx[c] + x - kMeRange, wx = x0 & ~7, wy = S.by[c] + y - kMeRange;
+      S.wx[s] = wx, S.wy[s] = wy, S.soff[s] = x0 - wx, S.wok[s] = inside(ref, wx, wy, bytes, rows_);
+    };
+    if (best < kMePenalty) {
+      // nothing to search: at the best centre the cost is its SAD alone, every other position of its
+      // window pays at least kMePenalty, and so does every one of the second centre's but that centre
+      // itself, whose SAD is no less -- the usual case on flat content, where a SAD is 0
+      S.first_search[c] = -1, S.two[c] = 0;
+      S.ccx[c][0] = px, S.ccy[c][0] = py;
+    } else if (two && abs(px - px2) <= kMergeMax && abs(py - py2) <= kMergeMax) {
       // one union window for both centres, its entry from the back of the list
       const int s = MeSmem<CELLS>::kSearches - 1 - atomicAdd(&S.nmerged, 1);
-      const int ux = min(px, px2) - kMeRange, wx0 = bx * 8 + ux;
       S.first_search[c] = s, S.two[c] = 2;
       S.scell[s] = c, S.sx[s] = px, S.sy[s] = py, S.sx2[s] = px2, S.sy2[s] = py2;
-      S.soff[s] = wx0 - (wx0 & ~7);
+      window(s, min(px, px2), min(py, py2), 4 * kMWinWords, kMWinRows);
       S.skey[s] = S.skey2[s] = 0xffffffffu;
     } else {
-    const int s0 = atomicAdd(&S.nsearch, two ? 2 : 1);
-    S.first_search[c] = s0, S.two[c] = two;
-    for (int k = 0; k < (two ? 2 : 1); k++) {
-      const int cxs = k ? px2 : px, cys = k ? py2 : py;
-      const int wx0 = bx * 8 + cxs - kMeRange;
-      S.scell[s0 + k] = c, S.sx[s0 + k] = cxs, S.sy[s0 + k] = cys;
-      S.soff[s0 + k] = wx0 - (wx0 & ~7);  // the window starts on the 8-byte boundary below wx0
-      S.skey[s0 + k] = 0xffffffffu;
-    }
+      const int s0 = atomicAdd(&S.nsearch, two ? 2 : 1);
+      S.first_search[c] = s0, S.two[c] = two;
+      for (int k = 0; k < (two ? 2 : 1); k++) {
+        const int x = k ? px2 : px, y = k ? py2 : py;
+        S.scell[s0 + k] = c, S.sx[s0 + k] = x, S.sy[s0 + k] = y;
+        window(s0 + k, x, y, 4 * kWinWords, kWinRows);
+        S.skey[s0 + k] = 0xffffffffu;
+      }
     }
   }
   __syncthreads();
   const int nsearch = S.nsearch, nmerged = S.nmerged;
-  // windows: rows y0 + cy - 8 .. + 23, 32 bytes from the 8-byte boundary at or below x0 + cx - 8;
-  // inside the margin as asynchronous 8-byte copies (all in flight at once: one memory latency for
-  // the whole staging), else word by word with clamping. Plane rows start 8-byte aligned (strides
-  // and margins are multiples of 8), and so do the window rows in shared memory.
-  for (int e = tid; e < nsearch * kWinRows * 4; e += kMeThreads) {
-    const int s = e / (kWinRows * 4), rem = e - s * (kWinRows * 4);
-    const int rr = rem >> 2, qd = rem & 3;
-    const int cell = cell0 + S.scell[s], by = cell / cols, bx = cell - by * cols;
-    const int wx = (bx * 8 + S.sx[s] - kMeRange) & ~7, wy = by * 8 + S.sy[s] - kMeRange;
+  // windows, a warp a search: 24 rows of 32 bytes, a lane an 8-byte column of every eighth row; inside
+  // the margin as asynchronous copies (all in flight at once: one memory latency for the whole staging),
+  // else word by word with clamping. Plane rows start 8-byte aligned, and so do the window rows in
+  // shared memory. (With the search, its cell and its place found again for every 8 bytes this loop was
+  // a fifth of the kernel's instructions.)
+  const int lane = tid & 31;
+  for (int s = tid >> 5; s < nsearch; s += kMeThreads / 32) {
+    const int rr = lane >> 2, qd = lane & 3, wx = S.wx[s] + 8 * qd, wy = S.wy[s] + rr;
     uint32_t* dst = S.win + s * kWinStride + rr * kWinWords + 2 * qd;
-    if (inside(ref, wx, wy, 4 * kWinWords, kWinRows)) {
-      cp_async8(dst, ref.p + (long long)(wy + rr) * ref.stride + wx + 8 * qd);
+    if (S.wok[s]) {
+      const uint8_t* g = ref.p + (long long)wy * ref.stride + wx;
+#pragma unroll
+      for (int i = 0; i < kWinRows / 8; i++) cp_async8(dst + 8 * i * kWinWords, g + (long long)(8 * i) * ref.stride);
     } else {
-      dst[0] = row4(ref, wx + 8 * qd, wy + rr), dst[1] = row4(ref, wx + 8 * qd + 4, wy + rr);
+      for (int i = 0; i < kWinRows; i += 8)
+        dst[i * kWinWords] = row4(ref, wx, wy + i), dst[i * kWinWords + 1] = row4(ref, wx + 4, wy + i);
     }
   }
-  // merged windows: rows from min(cy) - 8, 40 bytes from the 8-byte boundary at or below min(cx) - 8;
-  // merged search m (entry kSearches - 1 - m) in the window space of entries kSearches - 2 - 2m, +1
-  for (int e = tid; e < nmerged * kMWinRows * 5; e += kMeThreads) {
-    const int m = e / (kMWinRows * 5), rem = e - m * (kMWinRows * 5);
-    const int rr = rem / 5, qd = rem - rr * 5, s = MeSmem<CELLS>::kSearches - 1 - m;
-    const int cell = cell0 + S.scell[s], by = cell / cols, bx = cell - by * cols;
-    const int wx = (bx * 8 + min(S.sx[s], S.sx2[s]) - kMeRange) & ~7;
-    const int wy = by * 8 + min(S.sy[s], S.sy2[s]) - kMeRange;
-    uint32_t* dst = S.win + (MeSmem<CELLS>::kSearches - 2 - 2 * m) * kWinStride + rr * kMWinWords + 2 * qd;
-    if (inside(ref, wx, wy, 4 * kMWinWords, kMWinRows)) {
-      cp_async8(dst, ref.p + (long long)(wy + rr) * ref.stride + wx + 8 * qd);
-    } else {
-      dst[0] = row4(ref, wx + 8 * qd, wy + rr), dst[1] = row4(ref, wx + 8 * qd + 4, wy + rr);
-    }
+  // merged windows: 26 rows of 40 bytes, merged search m (entry kSearches - 1 - m) in the window space of
+  // entries kSearches - 2 - 2m, +1; five columns of every sixth row in 30 lanes
+  const int mr = lane / 5, mq = lane - mr * 5;
+  for (int m = tid >> 5; m < nmerged; m += kMeThreads / 32) {
+    const int s = MeSmem<CELLS>::kSearches - 1 - m, wx = S.wx[s] + 8 * mq, wy = S.wy[s];
+    uint32_t* dst = S.win + (MeSmem<CELLS>::kSearches - 2 - 2 * m) * kWinStride + 2 * mq;
+    const bool ok = S.wok[s];
+    if (mr < 6)
+      for (int rr = mr; rr < kMWinRows; rr += 6) {
+        if (ok)
+          cp_async8(dst + rr * kMWinWords, ref.p + (long long)(wy + rr) * ref.stride + wx);
+        else
+          dst[rr * kMWinWords] = row4(ref, wx, wy + rr), dst[rr * kMWinWords + 1] = row4(ref, wx + 4, wy + rr);
+      }
   }
   cp_async_wait_all();
   __syncthreads();
@@ -241,10 +277,8 @@ __global__ void __launch_bounds__(kMeThreads, 4) k_me_level(const FrameJob* __re
   for (int item = tid; item < nitems; item += kMeThreads) {
     if (item < nplain) {
     const int s = item / 17, dx = item - s * 17;
-    const uint32_t* c = S.cur[S.scell[s]];
     uint32_t cw[16];
-#pragma unroll
-    for (int k = 0; k < 16; k++) cw[k] = c[k];
+    load_cur(S.cur[S.scell[s]], cw);
     const int b = S.soff[s] + dx, wi = b >> 2;
     const unsigned sh = (unsigned)(b & 3) * 8;
     const uint32_t* wr = S.win + s * kWinStride + wi;
@@ -261,15 +295,12 @@ __global__ void __launch_bounds__(kMeThreads, 4) k_me_level(const FrameJob* __re
         if (dy >= 0 && dy <= 16) acc[dy] = sad4_acc(cw[2 * i + 1], w1, sad4_acc(cw[2 * i], w0, acc[dy]));
       }
     }
+    // the column's least (cost << 5 | dy): along a column raster order is dy's
     unsigned best = 0xffffffffu;
-    const unsigned pen_x = kMePenalty * abs(dx - kMeRange);
 #pragma unroll
-    for (int dy = 0; dy < 17; dy++) {
-      const unsigned cost = acc[dy] + pen_x + kMePenalty * abs(dy - kMeRange);
-      const unsigned key = (cost << 9) | (unsigned)(dy * 17 + dx);
-      best = key < best ? key : best;
-    }
-    atomicMin(&S.skey[s], best);
+    for (int dy = 0; dy < 17; dy++) best = min(best, (acc[dy] << 5) + (unsigned)(kMePenalty * (dy < kMeRange ? kMeRange - dy : dy - kMeRange) * 32 + dy));
+    const unsigned pen_x = kMePenalty * abs(dx - kMeRange);
+    atomicMin(&S.skey[s], ((best >> 5) + pen_x) << 9 | ((best & 31) * 17 + dx));
     } else {
     // merged searches: a thread per union column (at most 19); every union position's SAD is the
     // same for both centres, and each centre takes its own penalty and raster index -- the same
@@ -279,10 +310,8 @@ __global__ void __launch_bounds__(kMeThreads, 4) k_me_level(const FrameJob* __re
     const int cx1 = S.sx[s], cy1 = S.sy[s], cx2 = S.sx2[s], cy2 = S.sy2[s];
     const int ux = min(cx1, cx2), uy = min(cy1, cy2);  // union position 0 = centre offset -8
     if (du >= 17 + abs(cx1 - cx2)) continue;
-    const uint32_t* c = S.cur[S.scell[s]];
     uint32_t cw[16];
-#pragma unroll
-    for (int k = 0; k < 16; k++) cw[k] = c[k];
+    load_cur(S.cur[S.scell[s]], cw);
     const int b = S.soff[s] + du, wi = b >> 2;
     const unsigned sh = (unsigned)(b & 3) * 8;
     const uint32_t* wr = S.win + (MeSmem<CELLS>::kSearches - 2 - 2 * m) * kWinStride + wi;
@@ -322,19 +351,24 @@ __global__ void __launch_bounds__(kMeThreads, 4) k_me_level(const FrameJob* __re
   __syncthreads();
   if (tid < ncells && S.need[tid]) {
     const int s0 = S.first_search[tid];
+    int mx, my;
+    if (s0 < 0) {
+      mx = S.ccx[tid][0], my = S.ccy[tid][0];
+    } else {
     const unsigned k1 = S.skey[s0];
-    int mx = S.sx[s0] + (int)(k1 & 511) % 17 - kMeRange, my = S.sy[s0] + (int)(k1 & 511) / 17 - kMeRange;
+    mx = S.sx[s0] + (int)(k1 & 511) % 17 - kMeRange, my = S.sy[s0] + (int)(k1 & 511) / 17 - kMeRange;
     if (S.two[tid]) {  // the second centre's result only if strictly cheaper (me_cell, :189-192)
       const bool merged = S.two[tid] == 2;
       const unsigned k2 = merged ? S.skey2[s0] : S.skey[s0 + 1];
       const int sx2 = merged ? S.sx2[s0] : S.sx[s0 + 1], sy2 = merged ? S.sy2[s0] : S.sy[s0 + 1];
       if ((k2 >> 9) < (k1 >> 9)) mx = sx2 + (int)(k2 & 511) % 17 - kMeRange, my = sy2 + (int)(k2 & 511) / 17 - kMeRange;
     }
+    }
     // level 0 in quarter pels: k_me_refine refines it in place
     job.field[r][level][cell0 + tid] = level == 0 ? pack_mv(mx * 4, my * 4) : pack_mv(mx, my);
   }
   if (job.stats && tid < 32) {  // searched centres, one atomic per unit (the cells sit in warp 0)
-    const unsigned n = __reduce_add_sync(0xffffffffu, tid < ncells && S.need[tid] ? (S.two[tid] ? 2u : 1u) : 0u);
+    const unsigned n = __reduce_add_sync(0xffffffffu, tid < ncells && S.need[tid] && S.first_search[tid] >= 0 ? (S.two[tid] ? 2u : 1u) : 0u);
     if (tid == 0) atomicAdd(job.stats + level, (unsigned long long)n);
   }
   }  // units
@@ -350,17 +384,35 @@ __global__ void __launch_bounds__(kMeThreads, 4) k_me_level(const FrameJob* __re
 // per position re-read the cur coefficients from shared memory nine times a step). The four tiles'
 // SATDs meet in shared memory and every lane replays its cell's centre-first strict choice from
 // them (the same in all four warps, so one barrier per step). The second step's centre is the
-// first step's winner, whose SATD the first step has already computed.
+// first step's winner, whose SATD the first step has already computed. The centre comes first of all:
+// a move has to save more than kSubpelPenalty, so a unit none of whose centres costs more is done (five
+// 1080p animation-like frames of 7 references 0.53 -> 0.24 ms). The other positions go in pairs
+// (satd4_pair): 0.56 -> 0.53 ms on natural-like ones.
+// The four rows of the 4x4 tile at (ox, oy) displaced by quarter pels (qx, qy).
+__device__ __forceinline__ void rows_at(const DevPlane& ref, int ox, int oy, int qx, int qy, uint32_t* pr) {
+  DevPlane ph = ref;
+  ph.p = ref.p + (long long)((qy & 3) * 4 + (qx & 3)) * ref.phase;
+  const int x = ox + (qx >> 2), y = oy + (qy >> 2);
+  if (inside(ph, x, y, 4, 4)) {
+    const uint8_t* p = ph.p + (long long)y * ph.stride + x;
+#pragma unroll
+    for (int i = 0; i < 4; i++) pr[i] = load4(p + (long long)i * ph.stride);
+  } else {
+#pragma unroll
+    for (int i = 0; i < 4; i++) pr[i] = row4(ph, x, y + i);
+  }
+}
+
 constexpr int kRefineCells = 32, kRefineTiles = 4, kRefineThreads = 32 * kRefineTiles;
 
 __global__ void __launch_bounds__(kRefineThreads, 8) k_me_refine(const FrameJob* __restrict__ jobs, WorkList w) {
   // [step][pair][tile][cell]: the SATDs of positions 2 pair + 1 and 2 pair + 2 in halfwords (a cell's four
   // tiles sum to at most 65,280), and of the first step's centre
   __shared__ uint32_t sat[2][4][kRefineTiles][kRefineCells], sat0[kRefineTiles][kRefineCells];
-  __shared__ int unit_slot;
+  __shared__ int unit_slot[2];
   const int tid = threadIdx.x, c = tid & 31, t = tid >> 5;
   int unit, iter = 0;
-  while (take_unit(w, unit, iter, &unit_slot)) {
+  while (take_unit(w, unit, iter, unit_slot)) {
   const int jb = part_of(w, unit);
   const FrameJob& job = jobs[w.part[jb].job];
   const int cols = job.fcols[0], ncell = cols * job.frows[0];
@@ -385,7 +437,17 @@ __global__ void __launch_bounds__(kRefineThreads, 8) k_me_refine(const FrameJob*
   }
   const int m = field[cell];
   int cx = mv_x(m), cy = mv_y(m);  // quarter pels
-  int centre = 0;                  // the centre's SATD (the cell's four tiles), once known
+  int centre;                      // the centre's SATD (the cell's four tiles)
+  {
+    uint32_t pr[4];
+    rows_at(ref, ox, oy, cx, cy, pr);
+    sat0[t][c] = (uint32_t)satd4_rows(C, pr);
+    __syncthreads();
+    centre = (int)(sat0[0][c] + sat0[1][c] + sat0[2][c] + sat0[3][c]);
+    // a move must save more than kSubpelPenalty: cells whose centre costs no more stay (flat content: all
+    // of a unit's)
+    if (!__any_sync(0xffffffffu, need && centre > kSubpelPenalty)) continue;
+  }
 #pragma unroll
   for (int s = 0; s < 2; s++) {
     const int step = 2 - s;
@@ -397,9 +459,6 @@ __global__ void __launch_bounds__(kRefineThreads, 8) k_me_refine(const FrameJob*
       const long long rs = ref.stride;
       const uint8_t* p00 = ref.p + (long long)Y * rs + X;
       uint32_t pr[5], lf[5], rt[5];
-#pragma unroll
-      for (int i = 0; i < 4; i++) pr[i] = load4(p00 + i * rs);
-      sat0[t][c] = (uint32_t)satd4_rows(C, pr);  // the centre, phase (0, 0)
       const uint8_t* p20 = p00 + 8 * ref.phase;  // phase (2, 0): rows Y - 1 .. Y + 3
 #pragma unroll
       for (int i = 0; i < 5; i++) pr[i] = load4(p20 + (i - 1) * rs);
@@ -418,38 +477,18 @@ __global__ void __launch_bounds__(kRefineThreads, 8) k_me_refine(const FrameJob*
       sat[0][2][t][c] = __byte_perm(v45, v68, 0x5432);
       sat[0][3][t][c] = __byte_perm(v27, v68, 0x7632);
     } else {
-      // four rows at position k (the second step's centre, k = 0, is the first step's winner)
-      auto rows_at = [&](int k, uint32_t* pr) {
-        const int n = refine_pos(k);
-        const int qx = cx + (n % 3 - 1) * step, qy = cy + (n / 3 - 1) * step;
-        DevPlane ph = ref;
-        ph.p = ref.p + (long long)((qy & 3) * 4 + (qx & 3)) * ref.phase;
-        const int x = ox + (qx >> 2), y = oy + (qy >> 2);
-        if (inside(ph, x, y, 4, 4)) {
-          const uint8_t* p = ph.p + (long long)y * ph.stride + x;
-#pragma unroll
-          for (int i = 0; i < 4; i++) pr[i] = load4(p + (long long)i * ph.stride);
-        } else {
-#pragma unroll
-          for (int i = 0; i < 4; i++) pr[i] = row4(ph, x, y + i);
-        }
-      };
-      if (s == 0) {
-        uint32_t pr[4];
-        rows_at(0, pr);
-        sat0[t][c] = (uint32_t)satd4_rows(C, pr);
-      }
 #pragma unroll
       for (int k = 0; k < 4; k++) {
         uint32_t pa[4], pb[4];
-        rows_at(2 * k + 1, pa);
-        rows_at(2 * k + 2, pb);
+        const int na = refine_pos(2 * k + 1), nb = refine_pos(2 * k + 2);
+        rows_at(ref, ox, oy, cx + (na % 3 - 1) * step, cy + (na / 3 - 1) * step, pa);
+        rows_at(ref, ox, oy, cx + (nb % 3 - 1) * step, cy + (nb / 3 - 1) * step, pb);
         sat[s][k][t][c] = satd4_pair(C, pa, pb);
       }
     }
     __syncthreads();
     // the cell's choice (me_refine: the centre first, a move must save kSubpelPenalty)
-    int best = s == 0 ? (int)(sat0[0][c] + sat0[1][c] + sat0[2][c] + sat0[3][c]) : centre;
+    int best = centre;
     int raw = best, nx = cx, ny = cy;
 #pragma unroll
     for (int k = 0; k < 4; k++) {
@@ -477,33 +516,44 @@ void launch_me_refine(const FrameJob* jobs, const WorkList& w, cudaStream_t st) 
 
 int me_units(int nrefs, int cols, int rows, int cells) { return nrefs * ((cols * rows + cells - 1) / cells); }
 
-template <int CELLS>
+// Cells a CTA takes of a level: as configured (15 or 30) where the launch fills the GPU; seven, whose
+// searches are one round of 256 threads, while those CTAs are all resident at once: such a launch takes
+// one CTA's time, 19 us with 30 cells and 10 with seven.
+int me_level_cells(long long cells, int configured) {
+  const int full = persistent_grid((const void*)k_me_level<30, 256>, 256, sizeof(MeSmem<30>), INT_MAX);
+  return cells <= 7LL * full ? 7 : configured;
+}
+
+template <int CELLS, int T>
 static void launch_cells(const FrameJob* jobs, const WorkList& w, int level, cudaStream_t st) {
   const int units = w.prefix[w.nparts];
   const size_t smem = sizeof(MeSmem<CELLS>);
-  const int grid = w.queue ? persistent_grid((const void*)k_me_level<CELLS>, kMeThreads, smem, units) : units;
-  k_me_level<CELLS><<<grid, kMeThreads, smem, st>>>(jobs, w, level);
+  const int grid = w.queue ? persistent_grid((const void*)k_me_level<CELLS, T>, T, smem, units) : units;
+  k_me_level<CELLS, T><<<grid, T, smem, st>>>(jobs, w, level);
 }
 
 void launch_me_level(const FrameJob* jobs, const WorkList& w, int level, int cells, cudaStream_t st) {
   if (w.prefix[w.nparts] <= 0) return;
-  if (cells == 15)
-    launch_cells<15>(jobs, w, level, st);
+  if (cells == 7)
+    launch_cells<7, 256>(jobs, w, level, st);
+  else if (cells == 15)
+    launch_cells<15, 256>(jobs, w, level, st);
   else
-    launch_cells<30>(jobs, w, level, st);
+    launch_cells<30, 256>(jobs, w, level, st);
 }
 
-template <int CELLS>
+template <int CELLS, int T>
 static cudaError_t attributes_cells() {
   const size_t smem = sizeof(MeSmem<CELLS>);
-  const cudaError_t e = cudaFuncSetAttribute(k_me_level<CELLS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e == cudaSuccess) persistent_grid((const void*)k_me_level<CELLS>, kMeThreads, smem, 1);  // fills the grid cache
+  const cudaError_t e = cudaFuncSetAttribute(k_me_level<CELLS, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e == cudaSuccess) persistent_grid((const void*)k_me_level<CELLS, T>, T, smem, 1);  // fills the grid cache
   return e;
 }
 
 cudaError_t me_attributes() {
-  cudaError_t e = attributes_cells<15>();
-  if (e == cudaSuccess) e = attributes_cells<30>();
+  cudaError_t e = attributes_cells<7, 256>();
+  if (e == cudaSuccess) e = attributes_cells<15, 256>();
+  if (e == cudaSuccess) e = attributes_cells<30, 256>();
   if (e == cudaSuccess) persistent_grid((const void*)k_me_refine, kRefineThreads, 0, 1);  // fills the grid cache
   return e;
 }

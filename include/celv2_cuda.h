@@ -188,9 +188,10 @@ long long celv2_kernel_launches(const celv2_engine* e);
  *  CELV2_CFG_PERSISTENT_OFF: a bit mask of stages that run one CTA per unit even when
  *    CELV2_CFG_PERSISTENT is on (bit l: motion-search level l, 5 intra, 6 inter, 7 finalize,
  *    8 level 0's quarter-pel refinement).
- *  CELV2_CFG_INTER_CHUNK: distinct MVs per pass of the inter stage, 8..64 (default 64).
+ *  CELV2_CFG_INTER_CHUNK: distinct MVs per pass of the inter stage at most, 8..64 (default 64; the
+ *    whole-superblock kernel holds at most 30 where it runs four CTAs an SM).
  *  CELV2_CFG_ME_CELLS_L0 + l: 8x8 cells per motion-search CTA at pyramid level l, 15 or 30
- *    (default 30).
+ *    (default 30); levels too small to fill the GPU with CTAs of seven take seven.
  *  CELV2_CFG_FEATURES: 1 -- every inter frame's learned-pruner features are kept for
  *    celv2_features (include/celv2_pruner.h); 0 (default) -- only when the pruner runs.
  * The autotuner (celv2_b200/tune.py) times these per frame size and sets the fastest. */
