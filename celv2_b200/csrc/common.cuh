@@ -56,7 +56,7 @@ struct FrameJob {
   int sb_cols, sb_rows;
   int fcols[kLevels], frows[kLevels];
   int* field[kMaxRefs][kLevels];  // packed MVs: (mvy << 16) | (mvx & 0xffff)
-  const int* intra;        // [sb][kBlocks][kModes] SATDs (blocks < 5 unused)
+  const int* intra;        // [sb][kModes][kBlocks] SATDs (blocks < 5 unused)
   int2* inter;             // [sb][kMaxRefs][kBlocks]: (best SATD, packed MV)
   celv2_sb_out* out;       // [sb]
   long long lam;           // lambda_q8
@@ -140,56 +140,16 @@ __device__ __forceinline__ uint32_t load4(const uint8_t* p) {
   return __funnelshift_r(lo, __ldg(w + 1), sh);
 }
 
-// Sum of absolute 4x4 Hadamard coefficients (src/gpu/intra_common.h:131-146): rows, then columns,
-// the last column butterfly folded with the absolute values: |x + y| + |x - y| = 2 max(|x|, |y|).
-__device__ __forceinline__ int hadamard4x4(int d[16]) {
-#pragma unroll
-  for (int r = 0; r < 4; r++) {
-    const int s01 = d[4 * r] + d[4 * r + 1], d01 = d[4 * r] - d[4 * r + 1];
-    const int s23 = d[4 * r + 2] + d[4 * r + 3], d23 = d[4 * r + 2] - d[4 * r + 3];
-    d[4 * r] = s01 + s23, d[4 * r + 1] = d01 + d23, d[4 * r + 2] = s01 - s23, d[4 * r + 3] = d01 - d23;
-  }
-  int sum = 0;
-#pragma unroll
-  for (int c = 0; c < 4; c++) {
-    const int s01 = d[c] + d[4 + c], d01 = d[c] - d[4 + c];
-    const int s23 = d[8 + c] + d[12 + c], d23 = d[8 + c] - d[12 + c];
-    sum += max(abs(s01), abs(s23)) + max(abs(d01), abs(d23));
-  }
-  return 2 * sum;
+// The same, both words always loaded (planes have slack behind their last row).
+__device__ __forceinline__ uint32_t load4_pair(const uint8_t* p) {
+  const uintptr_t a = reinterpret_cast<uintptr_t>(p);
+  const uint32_t* w = reinterpret_cast<const uint32_t*>(a & ~uintptr_t(3));
+  return __funnelshift_r(__ldg(w), __ldg(w + 1), (uint32_t)(a & 3) * 8);
 }
 
 // Columns 0 and 2 (even) or 1 and 3 (odd) of a 4-byte row as two 16-bit lanes.
 __device__ __forceinline__ uint32_t bytes_even(uint32_t w) { return __byte_perm(w, 0, 0x4240); }
 __device__ __forceinline__ uint32_t bytes_odd(uint32_t w) { return __byte_perm(w, 0, 0x4341); }
-
-// hadamard4x4 of the byte residuals cur - pred of a 4x4 tile, rows as packed bytes: cur rows given
-// as their even / odd lanes (ce, co), prediction rows p. Each row's columns 0/2 and 1/3 ride as two
-// 16-bit lanes of one 32-bit integer, held as lo + hi * 65536 with |lo|, |hi| <= 2040 so plain
-// 32-bit adds are exact; three of the four butterfly stages run on both lanes at once, and the
-// last one with the absolute values folds into |x + y| + |x - y| = 2 max(|x|, |y|). The same sum
-// of 16 absolute Walsh-Hadamard coefficients as hadamard4x4.
-__device__ __forceinline__ int satd4_bytes(const uint32_t* ce, const uint32_t* co, const uint32_t* p) {
-  int A[4], B[4];
-#pragma unroll
-  for (int i = 0; i < 4; i++) {
-    const int e = (int)(ce[i] - bytes_even(p[i])), o = (int)(co[i] - bytes_odd(p[i]));
-    A[i] = e + o, B[i] = e - o;
-  }
-  int sum = 0;
-#pragma unroll
-  for (int h = 0; h < 2; h++) {
-    const int* X = h ? B : A;
-    const int s01 = X[0] + X[1], d01 = X[0] - X[1], s23 = X[2] + X[3], d23 = X[2] - X[3];
-    const int v[4] = {s01 + s23, d01 + d23, s01 - s23, d01 - d23};
-#pragma unroll
-    for (int k = 0; k < 4; k++) {
-      const int lo = (int)(short)(v[k] & 0xffff), hi = (v[k] - lo) >> 16;
-      sum += max(abs(lo), abs(hi));
-    }
-  }
-  return 2 * sum;
-}
 
 // dp4a with unsigned bytes a and signed bytes b: c + sum_k a_k * b_k.
 __device__ __forceinline__ int dp4a_us(uint32_t a, uint32_t b, int c) {
@@ -229,8 +189,8 @@ __device__ __forceinline__ void wh_rows_cur(const uint32_t* c, int* C) {
     for (int i = 0; i < 4; i++) C[4 * k + i] = dp4a_us(c[i], wh_row(k), 0);
 }
 
-// hadamard4x4 of the residual cur - pred of a 4x4 tile from the row-transformed cur tile C and the
-// prediction rows p (packed bytes): each residual row coefficient is one dp4a of the prediction
+// Sum of absolute 4x4 Hadamard coefficients (hadamard4x4, src/gpu/intra_common.h:131-146) of the residual
+// cur - pred of a 4x4 tile from the row-transformed cur tile C and the prediction rows p (packed bytes): each residual row coefficient is one dp4a of the prediction
 // row with the negated basis row, accumulated onto cur's; the column butterflies follow, the last
 // one folded with the absolute values into |x + y| + |x - y| = 2 max(|x|, |y|). The same sum of
 // 16 absolute coefficients.
@@ -284,14 +244,6 @@ __device__ __forceinline__ uint32_t satd4_two(const int* P, const uint32_t* p, c
     sum += max_u16x2(max_u16x2(s01, s23), 2 * B - min_u16x2(s01, s23)) + max_u16x2(max_u16x2(d01, d23), 2 * B - min_u16x2(d01, d23));
   }
   return 2 * (sum - 8 * B);
-}
-
-// Residual of one 4x4 row: four cur bytes minus four prediction bytes.
-__device__ __forceinline__ void residual_row(int* d, uint32_t c, uint32_t p) {
-  d[0] = (int)(c & 255) - (int)(p & 255);
-  d[1] = (int)((c >> 8) & 255) - (int)((p >> 8) & 255);
-  d[2] = (int)((c >> 16) & 255) - (int)((p >> 16) & 255);
-  d[3] = (int)(c >> 24) - (int)(p >> 24);
 }
 
 __device__ __forceinline__ int mv_x(int packed) { return (int)(short)(packed & 0xffff); }

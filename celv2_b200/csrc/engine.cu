@@ -1684,8 +1684,13 @@ int celv2_debug_intra(celv2_engine* e, int32_t* out) {
     if (!e || !out) invalid("null argument");
     CK(cudaSetDevice(e->device));
     e->wait_idle();
-    CK(cudaMemcpy(out, e->intra_prep[e->cur_src], (size_t)e->g.nsb * kBlocks * kModes * sizeof(int),
-                  cudaMemcpyDeviceToHost));
+    // mode by mode on the device, block by block for the caller
+    std::vector<int32_t> sat((size_t)e->g.nsb * kBlocks * kModes);
+    CK(cudaMemcpy(sat.data(), e->intra_prep[e->cur_src], sat.size() * sizeof(int32_t), cudaMemcpyDeviceToHost));
+    for (int s = 0; s < e->g.nsb; s++)
+      for (int b = 0; b < kBlocks; b++)
+        for (int m = 0; m < kModes; m++)
+          out[((size_t)s * kBlocks + b) * kModes + m] = sat[((size_t)s * kModes + m) * kBlocks + b];
   });
 }
 

@@ -282,10 +282,15 @@ __global__ void __launch_bounds__(kIntraThreads, 4) k_intra(const FrameJob* __re
       const int h = T - U0 + abs(s01 + s23) + abs(s01 - s23) + abs(d01 + d23) + abs(d01 - d23);
       sat[0] = (unsigned short)dc, sat[kIntraThreads] = (unsigned short)v, sat[2 * kIntraThreads] = (unsigned short)h;
     }
+    // the ten other modes two at a time (satd4_pair)
+    uint32_t pa[4] = {}, pb[4] = {};
+    auto both = [&](int m) {
+      const uint32_t v = satd4_pair(C, pa, pb);
+      sat[m * kIntraThreads] = (unsigned short)v, sat[(m + 1) * kIntraThreads] = (unsigned short)(v >> 16);
+    };
     // Smooth: bilinear blend of above, left, top-right and bottom-left, columns 0 / 2 and
     // 1 / 3 as two 16-bit lanes (a sum is at most 255 * 66 + 33)
     if (keep & CELV2_KEEP_MODE(3)) {
-      uint32_t pw[4];
       const int den = bw + bh + 2;
       // n / den as the top byte of n * ceil(2^24 / den): exact while n * (den * ceil(2^24 / den) -
       // 2^24) < 2^24 (division by invariant integers using multiplication, Granlund and Montgomery
@@ -303,13 +308,11 @@ __global__ void __launch_bounds__(kIntraThreads, 4) k_intra(const FrameJob* __re
         const uint32_t e = ae * wa + we * li + te + add, o = ao * wa + wo * li + to + add;
         const uint32_t q0 = (e & 0xffffu) * magic, q2 = (e >> 16) * magic;
         const uint32_t q1 = (o & 0xffffu) * magic, q3 = (o >> 16) * magic;
-        pw[i] = __byte_perm(__byte_perm(q0, q1, 0x0073), __byte_perm(q2, q3, 0x0073), 0x5410);
+        pa[i] = __byte_perm(__byte_perm(q0, q1, 0x0073), __byte_perm(q2, q3, 0x0073), 0x5410);
       }
-      sat[3 * kIntraThreads] = (unsigned short)satd4_rows(C, pw);
     }
     // SmoothV (h a power of two, the numerator non-negative): two 16-bit lanes at once
     if (keep & CELV2_KEEP_MODE(4)) {
-      uint32_t pw[4];
       const uint32_t ae = a4 & 0x00ff00ffu, ao = (a4 >> 8) & 0x00ff00ffu;
       const int bl = byte_at(S.tr, l + bh - 1);
 #pragma unroll
@@ -317,13 +320,12 @@ __global__ void __launch_bounds__(kIntraThreads, 4) k_intra(const FrameJob* __re
         const int ii = r0 + i;
         const uint32_t wa = (uint32_t)(bh - 1 - ii), add = (uint32_t)((ii + 1) * bl + bh / 2) * 0x00010001u;
         const uint32_t e = ((ae * wa + add) >> lgh) & 0x00ff00ffu, o = ((ao * wa + add) >> lgh) & 0x00ff00ffu;
-        pw[i] = e | o << 8;
+        pb[i] = e | o << 8;
       }
-      sat[4 * kIntraThreads] = (unsigned short)satd4_rows(C, pw);
     }
+    if (keep & (CELV2_KEEP_MODE(3) | CELV2_KEEP_MODE(4))) both(3);
     // SmoothH: per row the left sample, per column weights (bw - 1 - jj, jj + 1)
     if (keep & CELV2_KEEP_MODE(5)) {
-      uint32_t pw[4];
       const int tr = byte_at(S.px, a + bw - 1);
       const uint32_t we = (uint32_t)(bw - 1 - c0) | (uint32_t)(bw - 3 - c0) << 16;
       const uint32_t wo = (uint32_t)(bw - 2 - c0) | (uint32_t)(bw - 4 - c0) << 16;
@@ -333,16 +335,14 @@ __global__ void __launch_bounds__(kIntraThreads, 4) k_intra(const FrameJob* __re
       for (int i = 0; i < 4; i++) {
         const uint32_t li = (l4 >> (8 * i)) & 255u;
         const uint32_t e = ((li * we + te) >> lgw) & 0x00ff00ffu, o = ((li * wo + to) >> lgw) & 0x00ff00ffu;
-        pw[i] = e | o << 8;
+        pa[i] = e | o << 8;
       }
-      sat[5 * kIntraThreads] = (unsigned short)satd4_rows(C, pw);
     }
     // Paeth, four samples at a time. With u = A - tl and v = L - tl the three distances are pl = |u|,
     // pa = |v| and ptl = |u + v|: where u and v differ in sign that is ||u| - |v||, else it is at
     // least both others (255 in its place). A byte compare x <= y is bit 15 of 0x8000 + y - x in
     // 16-bit lanes, spread over the byte by prmt's sign mode
     if (keep & CELV2_KEEP_MODE(6)) {
-      uint32_t pw[4];
       const uint32_t tl4 = (uint32_t)byte_at(S.px, a - 1) * 0x01010101u;
       // bytes 0 / 2 and 1 / 3 of w as lanes; le4: the bytes' mask of x <= y, y's lanes carrying 0x8000
       auto ev = [](uint32_t w) { return w & 0x00ff00ffu; };
@@ -358,38 +358,34 @@ __global__ void __launch_bounds__(kIntraThreads, 4) k_intra(const FrameJob* __re
         const uint32_t pae = ev(pa), de = ev(d) | h, dd = od(d) | h;
         const uint32_t ml = spread(((pae | h) - ple) & (de - ple), ((pae | h) - plo) & (dd - plo));
         const uint32_t ma = spread(de - pae, dd - pae);
-        pw[i] = (li & ml) | (~ml & ((a4 & ma) | (tl4 & ~ma)));
+        pb[i] = (li & ml) | (~ml & ((a4 & ma) | (tl4 & ~ma)));
       }
-      sat[6 * kIntraThreads] = (unsigned short)satd4_rows(C, pw);
     }
+    if (keep & (CELV2_KEEP_MODE(5) | CELV2_KEEP_MODE(6))) both(5);
     // D45: derivative 64, no blend: row i is A[r0 + i + 1 + c0 ..] (never past A[w + h - 1])
     if (keep & CELV2_KEEP_MODE(7)) {
-      uint32_t pw[4];
       const uint32_t* q = S.px + ((a + r0 + c0) >> 2);
       const uint32_t w0 = q[0], w1 = q[1];
 #pragma unroll
-      for (int i = 0; i < 3; i++) pw[i] = __funnelshift_r(w0, w1, 8 * (i + 1));
-      pw[3] = w1;
-      sat[7 * kIntraThreads] = (unsigned short)satd4_rows(C, pw);
+      for (int i = 0; i < 3; i++) pa[i] = __funnelshift_r(w0, w1, 8 * (i + 1));
+      pa[3] = w1;
     }
     // D67: derivative 27, one weight per row
     if (keep & CELV2_KEEP_MODE(8)) {
-      uint32_t pw[4];
 #pragma unroll
       for (int i = 0; i < 4; i++) {
         const int pos = (r0 + i + 1) * 27;
         uint32_t w0, w1;
         lds_pair(S.px, a + (pos >> 6) + c0, w0, w1);
-        pw[i] = blend4(w0, w1, (pos & 63) >> 1);
+        pb[i] = blend4(w0, w1, (pos & 63) >> 1);
       }
-      sat[8 * kIntraThreads] = (unsigned short)satd4_rows(C, pw);
     }
+    if (keep & (CELV2_KEEP_MODE(7) | CELV2_KEEP_MODE(8))) both(7);
     // D113, by rows: row ii is taken from the left below column ((ii + 1) * 27 - 1) >> 6
     if (keep & CELV2_KEEP_MODE(9)) {
-      uint32_t pw[4];
       if (((r0 + 1) * 27 - 1) >> 6 < c0 + 4) {
 #pragma unroll
-        for (int i = 0; i < 4; i++) pw[i] = z2_above(S.px, a, c0, r0 + i, 27);
+        for (int i = 0; i < 4; i++) pa[i] = z2_above(S.px, a, c0, r0 + i, 27);
       }
       if (((r0 + 4) * 27 - 1) >> 6 > c0) {
         uint32_t q[4];
@@ -399,15 +395,13 @@ __global__ void __launch_bounds__(kIntraThreads, 4) k_intra(const FrameJob* __re
 #pragma unroll
         for (int i = 0; i < 4; i++) {
           const uint32_t k = low_bytes((((r0 + i + 1) * 27 - 1) >> 6) - c0);
-          pw[i] = (q[i] & k) | (pw[i] & ~k);
+          pa[i] = (q[i] & k) | (pa[i] & ~k);
         }
       }
-      sat[9 * kIntraThreads] = (unsigned short)satd4_rows(C, pw);
     }
     // D135: derivatives 64 / 64, no blend: row i is the run of L reversed, A[-1], A from
     // A[c0 - r0 - 1 - i] on, so the tile's rows are windows of two words of it
     if (keep & CELV2_KEEP_MODE(10)) {
-      uint32_t pw[4];
       const int d = c0 - r0;  // a multiple of 4
       uint32_t q[2];
 #pragma unroll
@@ -421,9 +415,9 @@ __global__ void __launch_bounds__(kIntraThreads, 4) k_intra(const FrameJob* __re
         }
       }
 #pragma unroll
-      for (int i = 0; i < 4; i++) pw[i] = __funnelshift_r(q[0], q[1], 24 - 8 * i);
-      sat[10 * kIntraThreads] = (unsigned short)satd4_rows(C, pw);
+      for (int i = 0; i < 4; i++) pb[i] = __funnelshift_r(q[0], q[1], 24 - 8 * i);
     }
+    if (keep & (CELV2_KEEP_MODE(9) | CELV2_KEEP_MODE(10))) both(9);
     if (keep & (CELV2_KEEP_MODE(11) | CELV2_KEEP_MODE(12))) {
       // D157 and D203 predict columns: from here on C is the transform of the cur tile's columns
       uint32_t col[4];
@@ -433,10 +427,9 @@ __global__ void __launch_bounds__(kIntraThreads, 4) k_intra(const FrameJob* __re
     }
     // D157, by columns: column jj is taken from above in rows below 64 (jj + 1) / 151
     if (keep & CELV2_KEEP_MODE(11)) {
-      uint32_t pw[4];
       if (64 * (c0 + 1) / 151 < r0 + 4) {
 #pragma unroll
-        for (int j = 0; j < 4; j++) pw[j] = z2_left(S.tr, l, r0, c0 + j, 27);
+        for (int j = 0; j < 4; j++) pa[j] = z2_left(S.tr, l, r0, c0 + j, 27);
       }
       if (64 * (c0 + 4) / 151 > r0) {
         uint32_t q[4];
@@ -446,23 +439,21 @@ __global__ void __launch_bounds__(kIntraThreads, 4) k_intra(const FrameJob* __re
 #pragma unroll
         for (int j = 0; j < 4; j++) {
           const uint32_t k = low_bytes(64 * (c0 + j + 1) / 151 - r0);
-          pw[j] = (q[j] & k) | (pw[j] & ~k);
+          pa[j] = (q[j] & k) | (pa[j] & ~k);
         }
       }
-      sat[11 * kIntraThreads] = (unsigned short)satd4_rows(C, pw);
     }
     // z3: D203 (derivative 27), by columns from the column left
     if (keep & CELV2_KEEP_MODE(12)) {
-      uint32_t pw[4];
 #pragma unroll
       for (int j = 0; j < 4; j++) {
         const int pos = (c0 + j + 1) * 27;
         uint32_t w0, w1;
         lds_pair(S.tr, l + (pos >> 6) + r0, w0, w1);
-        pw[j] = blend4(w0, w1, (pos & 63) >> 1);
+        pb[j] = blend4(w0, w1, (pos & 63) >> 1);
       }
-      sat[12 * kIntraThreads] = (unsigned short)satd4_rows(C, pw);
     }
+    if (keep & (CELV2_KEEP_MODE(11) | CELV2_KEEP_MODE(12))) both(11);
     __syncthreads();  // the step's SATDs; the other buffer's readers are past the step before
     // a block's sums: thread (mode, 8 items) adds their halfwords, blocks of more meet in acc
     for (int e = tid; e < kModes * (kIntraThreads / 8); e += kIntraThreads) {
@@ -491,8 +482,12 @@ __global__ void __launch_bounds__(kIntraThreads, 4) k_intra(const FrameJob* __re
   }
   __syncthreads();
   int* out = const_cast<int*>(job.intra) + (long long)sb * kBlocks * kModes;
-  for (int e = b0 * kModes + tid; e < b1 * kModes; e += kIntraThreads)
-    if (parts < 9 || mine(e / kModes)) out[e] = S.acc[e];
+  // mode by mode, as the finalize stage's blocks read them
+  for (int bl = b0 + tid; bl < b1; bl += kIntraThreads)
+    if (parts < 9 || mine(bl)) {
+#pragma unroll
+      for (int m = 0; m < kModes; m++) out[m * kBlocks + bl] = S.acc[bl * kModes + m];
+    }
   }  // units
 }
 

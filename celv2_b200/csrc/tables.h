@@ -17,34 +17,20 @@ constexpr int kItems = 3072;       // every block's tiles
 constexpr int kIntraFirst = 768;   // first item of a block below 64x64
 constexpr int kIntraItems = kItems - kIntraFirst;
 
-// Tiles per block of the class item i belongs to (the reduction segment width).
-__device__ __forceinline__ int item_width(int i) {
-  return i < 256 ? 256 : i < 768 ? 128 : i < 1024 ? 64 : i < 1536 ? 32 : i < 1792 ? 16 : i < 2304 ? 8 : i < 2560 ? 4 : 2;
-}
-
-// Item i's block and tile position in the superblock (tile units of 4 samples), from the class
-// structure: class c covers squares of level c / 2, whole (even c) or as halves (odd c).
-__device__ __forceinline__ void item_decode(int i, int& b, int& tx, int& ty) {
-  const int c = i < 256 ? 0 : i < 768 ? 1 : i < 1024 ? 2 : i < 1536 ? 3 : i < 1792 ? 4 : i < 2304 ? 5 : i < 2560 ? 6 : 7;
-  const int start = c == 0 ? 0 : c == 1 ? 256 : c == 2 ? 768 : c == 3 ? 1024 : c == 4 ? 1536 : c == 5 ? 1792 : c == 6 ? 2304 : 2560;
-  const int level = c >> 1;
-  const int lwt = (c & 1) ? (2 * (4 - level) - 1) : (2 * (4 - level));  // log2(tiles per block)
-  const int k = i - start, blk = k >> lwt, t = k & ((1 << lwt) - 1);
-  const int sq = sb_level_offset(level) + ((c & 1) ? (blk >> 2) : blk);
-  const int kind = (c & 1) ? 1 + (blk & 3) : 0;
-  b = sq * 5 + kind;
-  int x, y, w, h;
-  sb_block_geom(b, x, y, w, h);
-  const int tw = w >> 2;
-  tx = (x >> 2) + (t % tw), ty = (y >> 2) + (t / tw);
-}
-
-// Sum of v over the lanes of this lane's segment of `width` lanes (power of two); every lane of
-// the segment ends with the sum. For width >= 32 the whole warp is one segment.
-__device__ __forceinline__ int segment_sum(int v, int width) {
-  const int span = width < 32 ? width : 32;
-  for (int off = span >> 1; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
-  return v;
+// Item i's block b, the block's place (x, y) in the superblock and the tile's (c0, r0) in the block, in
+// samples, and log2 of the block's tiles: class c covers the squares of level c / 2, whole (even c) or
+// as halves (odd c); a class's items all lie in one step of 256 (or several whole ones).
+__device__ __forceinline__ void item_place(int i, int& b, int& x, int& y, int& c0, int& r0, int& lwt) {
+  const int st = i >> 8;  // steps per class: 1, 2, 1, 2, 1, 2, 1, 2
+  const int level = st / 3, sub = st - level * 3, lgs = 6 - level;
+  lwt = 2 * (4 - level) - (sub != 0);
+  const int k = (sub == 2 ? 256 : 0) + (i & 255), blk = k >> lwt, t = k & ((1 << lwt) - 1);
+  const int idx = sub ? blk >> 2 : blk, kind = sub ? 1 + (blk & 3) : 0;
+  b = (sb_level_offset(level) + idx) * 5 + kind;
+  const int lgw = lgs - (kind >= 3), lgh = lgs - (kind == 1 || kind == 2);
+  x = ((idx & ((1 << level) - 1)) << lgs) + (kind == 4 ? 1 << lgw : 0);
+  y = ((idx >> level) << lgs) + (kind == 2 ? 1 << lgh : 0);
+  c0 = (t & ((1 << (lgw - 2)) - 1)) * 4, r0 = (t >> (lgw - 2)) * 4;
 }
 
 }  // namespace celv2cu
