@@ -823,23 +823,24 @@ struct celv2_engine {
     return 1;
   }
 
-  // The pruner's features per job, then per job one kernel running the network on each
-  // superblock and writing its mask; returns the kernels launched.
+  // The pruner's features of every job that has them, then the network and the keep words of every
+  // superblock that has it; returns the kernels launched.
   int enqueue_pruner(const std::vector<FrameJob>& jobs, const std::vector<NetJob>& nets, cudaStream_t stream) {
-    const int n = std::min((int)jobs.size(), (int)nets.size());
-    int launched = 0;
-    for (int j = 0; j < n; j++) {
+    NetList feats{}, run{};
+    auto add = [&](NetList& l, int j) {
       const NetJob& nj = nets[j];
-      if (!nj.feats) continue;
-      const int nsb = jobs[j].sb_cols * jobs[j].sb_rows;
-      launch_features(djobs + j, nsb, nj.feats, stream);
-      launched++;
-      if (nj.net) {
-        launch_infer(nj.params, nj.wb, nj.feats, nsb, jobs[j].nrefs, nj.th, nj.keep, stream);
-        launched++;
-      }
+      l.e[l.n] = NetList::Entry{j, jobs[j].nrefs, nj.feats, nj.params, nj.wb, nj.keep, nj.th};
+      l.prefix[l.n + 1] = l.prefix[l.n] + jobs[j].sb_cols * jobs[j].sb_rows;
+      l.n++;
+    };
+    for (int j = 0; j < std::min((int)jobs.size(), (int)nets.size()); j++) {
+      if (!nets[j].feats) continue;
+      add(feats, j);
+      if (nets[j].net) add(run, j);
     }
-    return launched;
+    launch_features(djobs, feats, stream);
+    launch_infer(run, stream);
+    return (feats.n > 0) + (run.n > 0);
   }
 
   // Everything of a batch up to its slices: motion search, refinement, and intra (unless it runs on

@@ -99,24 +99,30 @@ void inter_window(unsigned& bytes, unsigned& rows);
 // Per-block choice, compound, partition choice and the decision records. Units: the parts' superblocks.
 void launch_finalize(const FrameJob* jobs, const WorkList& w, cudaStream_t st);
 
-// The learned pruner (pruner.cu): one job's features (nsb x CELV2_PRUNER_FEATURES), the network's
-// forward pass into a cache of batch x CELV2_PRUNER_ACTS floats (logits last), and the masks.
-void launch_features(const FrameJob* djob, int nsb, float* out, cudaStream_t st);
-void pruner_forward(const float* params, const float* x, int batch, float* acts, cudaStream_t st);
-// The pruner's decision rule: per output group the probability a kept option needs (references,
-// intra, block levels, intra modes), and the band around them inside which a superblock falls back
-// to the full search.
+// The learned pruner's decision rule (pruner.cu): per output group the probability a kept option needs
+// (references, intra, block levels, intra modes), and the band around them inside which a superblock
+// falls back to the full search.
 struct PrunerThresholds {
   float ref, intra, level, mode, band;
 };
-void launch_masks(const float* logits, int nsb, int nrefs, const PrunerThresholds& th, uint32_t* keep,
-                  cudaStream_t st);
-// The engine's inference: the network and the mask of every superblock of one job in one kernel,
-// from bf16 weight copies (infer_weights: infer_weight_elems() bf16 elements).
+// The jobs of a batch with features or a network: entry i owns superblocks [prefix[i], prefix[i + 1]).
+struct NetList {
+  int n;
+  int prefix[kMaxJobs + 1];
+  struct Entry {
+    int job, nrefs;
+    float* feats;         // superblocks x CELV2_PRUNER_FEATURES
+    const float* params;  // the network's parameters
+    const void* wb;       // and their bf16 copies (infer_weights: infer_weight_elems() elements)
+    uint32_t* keep;       // the keep words it writes
+    PrunerThresholds th;
+  } e[kMaxJobs];
+};
+// Every entry's features; the network and the keep words of every superblock of the list.
+void launch_features(const FrameJob* jobs, const NetList& l, cudaStream_t st);
+void launch_infer(const NetList& l, cudaStream_t st);
 size_t infer_weight_elems();
 void infer_weights(const float* params, void* wb, cudaStream_t st);
-void launch_infer(const float* params, const void* wb, const float* feats, int nsb, int nrefs,
-                  const PrunerThresholds& th, uint32_t* keep, cudaStream_t st);
 
 // Set-up of the constant tables (once per device).
 cudaError_t init_tables();

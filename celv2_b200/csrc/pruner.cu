@@ -653,24 +653,29 @@ void backward(const float* P, int batch, const float* acts, const float* dlogits
 
 // ---- features and masks (the engine side) ----
 
-// One CTA (128 threads) per superblock of one job: the luma at level 2, the level-1 cost map per
-// reference, presence flags and lambda (include/celv2_pruner.h).
-__global__ void __launch_bounds__(128) k_features(const FrameJob* __restrict__ jobp, float* __restrict__ out) {
-  const FrameJob& job = *jobp;
-  const int sb = blockIdx.x, tid = threadIdx.x;
+__device__ __forceinline__ int entry_of(const NetList& l, int sb) {
+  int i = 0;
+  while (i + 1 < l.n && sb >= l.prefix[i + 1]) i++;
+  return i;
+}
+
+// One CTA (128 threads) per superblock of the batch: the luma at level 2, the level-1 cost map per
+// reference (a thread per cell and reference, rows as words where they lie inside the margins), presence
+// flags and lambda (include/celv2_pruner.h).
+__global__ void __launch_bounds__(128) k_features(const FrameJob* __restrict__ jobs, NetList l) {
+  const int en = entry_of(l, blockIdx.x);
+  const FrameJob& job = jobs[l.e[en].job];
+  const int sb = blockIdx.x - l.prefix[en], tid = threadIdx.x;
   const int sby = sb / job.sb_cols, sbx = sb - sby * job.sb_cols;
-  float* f = out + (long long)sb * nn::kF;
-  __shared__ float red[128];
-  const DevPlane l2 = job.cur.lv[2];
-  int v0 = at(l2, sby * 16 + (tid >> 4), sbx * 16 + (tid & 15));
-  int v1 = at(l2, sby * 16 + 8 + (tid >> 4), sbx * 16 + (tid & 15));
-  red[tid] = (float)(v0 + v1);
+  float* f = l.e[en].feats + (long long)sb * nn::kF;
+  __shared__ int red[4];
+  const DevPlane& l2 = job.cur.lv[2];
+  const int v0 = at(l2, sby * 16 + (tid >> 4), sbx * 16 + (tid & 15));
+  const int v1 = at(l2, sby * 16 + 8 + (tid >> 4), sbx * 16 + (tid & 15));
+  const int sum = __reduce_add_sync(0xffffffffu, v0 + v1);  // whole numbers: exact in any order
+  if ((tid & 31) == 0) red[tid >> 5] = sum;
   __syncthreads();
-  for (int s = 64; s > 0; s >>= 1) {
-    if (tid < s) red[tid] += red[tid + s];
-    __syncthreads();
-  }
-  const float mean = red[0] / 256.f;
+  const float mean = (float)(red[0] + red[1] + red[2] + red[3]) / 256.f;
   f[tid] = ((float)v0 - mean) / 64.f;
   f[128 + tid] = ((float)v1 - mean) / 64.f;
   if (tid < kMaxRefs * 16) {
@@ -679,11 +684,20 @@ __global__ void __launch_bounds__(128) k_features(const FrameJob* __restrict__ j
     if (r < job.nrefs) {
       const int cols = job.fcols[1], rows = job.frows[1];
       const int cx = min(sbx * 4 + (cell & 3), cols - 1), cy = min(sby * 4 + (cell >> 2), rows - 1);
-      const int m = job.field[r][1][cy * cols + cx], mx = mv_x(m), my = mv_y(m);
-      const DevPlane cur = job.cur.lv[1], ref = job.ref[r].lv[1];
-      int sad = 0;
-      for (int i = 0; i < 8; i++)
-        for (int j = 0; j < 8; j++) sad += abs(at(cur, cy * 8 + i, cx * 8 + j) - at(ref, cy * 8 + my + i, cx * 8 + mx + j));
+      const int m = job.field[r][1][cy * cols + cx], x = cx * 8 + mv_x(m), y = cy * 8 + mv_y(m);
+      const DevPlane &cur = job.cur.lv[1], &ref = job.ref[r].lv[1];
+      unsigned sad = 0;
+      if (inside(cur, cx * 8, cy * 8, 8, 8) && inside(ref, x, y, 8, 8)) {
+        const uint8_t *pc = cur.p + (long long)cy * 8 * cur.stride + cx * 8, *pr = ref.p + (long long)y * ref.stride + x;
+#pragma unroll
+        for (int i = 0; i < 8; i++)
+#pragma unroll
+          for (int h = 0; h < 2; h++)
+            sad += __vsadu4(load4_pair(pc + (long long)i * cur.stride + 4 * h), load4_pair(pr + (long long)i * ref.stride + 4 * h));
+      } else {
+        for (int i = 0; i < 8; i++)
+          for (int j = 0; j < 8; j++) sad += abs(at(cur, cy * 8 + i, cx * 8 + j) - at(ref, y + i, x + j));
+      }
       v = log2f(1.f + (float)sad) / 14.f;
     }
     f[256 + tid] = v;
@@ -692,8 +706,8 @@ __global__ void __launch_bounds__(128) k_features(const FrameJob* __restrict__ j
   if (tid == 0) f[375] = log2f((float)(job.lam > 1 ? job.lam : 1)) / 20.f;
 }
 
-void launch_features(const FrameJob* djob, int nsb, float* out, cudaStream_t st) {
-  k_features<<<nsb, 128, 0, st>>>(djob, out);
+void launch_features(const FrameJob* jobs, const NetList& l, cudaStream_t st) {
+  if (l.prefix[l.n] > 0) k_features<<<l.prefix[l.n], 128, 0, st>>>(jobs, l);
 }
 
 // The keep word (include/celv2_decision.h) of one superblock from its logits: reference r kept
@@ -732,28 +746,15 @@ __device__ __forceinline__ uint32_t mask_word(const float* z, int nrefs, const P
   return unsure ? 0xFFFFFFFFu : k;
 }
 
-__global__ void k_masks(const float* __restrict__ logits, int nsb, int nrefs, PrunerThresholds th,
-                        uint32_t* __restrict__ keep) {
-  const int sb = blockIdx.x * blockDim.x + threadIdx.x;
-  if (sb >= nsb) return;
-  keep[sb] = mask_word(logits + (long long)sb * nn::kOut, nrefs, th);
-}
-
-void launch_masks(const float* logits, int nsb, int nrefs, const PrunerThresholds& th, uint32_t* keep,
-                  cudaStream_t st) {
-  k_masks<<<(nsb + 127) / 128, 128, 0, st>>>(logits, nsb, nrefs, th, keep);
-}
-
-void pruner_forward(const float* params, const float* x, int batch, float* acts, cudaStream_t st) {
-  nn::forward(params, x, batch, acts, st);
-}
-
 // ---- the engine's inference: the whole network for one superblock per CTA, then its mask ----
 // The same arithmetic as nn::forward (BF16 operands, FP32 sums; only the order of the sums
 // differs): the 3x3 convolution 1 -> 16 and the dense layers on the CUDA cores (bf16-rounded
 // operands), the two strided convolutions (85% of the FLOPs) as mma.sync m16n8k16 tiles whose A
 // operand is read straight from the previous activation in shared memory (an implicit im2col).
-// Weights: bf16 copies made once (infer_weights), W4 transposed so a CTA's 64 threads read rows.
+// Weights: bf16 copies made once (infer_weights), W4 transposed so a CTA's 64 threads read rows. All the
+// superblocks of a batch go in one launch, as their features do: five 1080p jobs 218 -> 123 us (a pair of
+// launches a job, 510 CTAs each, left the GPU with little in flight). The sums' order is fixed: a keep word
+// follows from comparisons of what they give.
 namespace nn {
 constexpr int kIW2 = 0, kIW3 = kIW2 + 32 * 144, kIW4 = kIW3 + 32 * 288, kIWs = kIW4 + 632 * 64;  // bf16 elements
 
@@ -770,30 +771,44 @@ __global__ void k_infer_weights(const float* __restrict__ P, __nv_bfloat16* __re
   }
 }
 
-__global__ void __launch_bounds__(128) k_infer(const float* __restrict__ P, const __nv_bfloat16* __restrict__ Wb,
-                                               const float* __restrict__ feats, int nrefs, PrunerThresholds th,
-                                               uint32_t* __restrict__ keep) {
+__global__ void __launch_bounds__(128) k_infer(NetList l) {
   __shared__ float xr[kF];                            // the features, bf16-rounded
-  __shared__ __align__(16) __nv_bfloat16 a1[256][16];  // conv1 output, (y, x) rows, channels
-  __shared__ __align__(16) __nv_bfloat16 a2[64][32];
+  __shared__ float img[18][18], w1[9][16];            // the image with a border of zeros; conv1's weights, rounded
+  __shared__ __align__(16) bf16 a1[256][16];           // conv1 output, (y, x) rows, channels
+  __shared__ __align__(16) bf16 a2[64][32];
   __shared__ float h0[632], a4[64], part[128];
   __shared__ float logits[kOut];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
-  const float* x = feats + (long long)blockIdx.x * kF;
-  for (int i = tid; i < kF; i += 128) xr[i] = rbf(x[i]);
+  const int en = entry_of(l, blockIdx.x), sb = blockIdx.x - l.prefix[en];
+  const float* __restrict__ P = l.e[en].params;
+  const bf16* __restrict__ Wb = static_cast<const bf16*>(l.e[en].wb);
+  const float* x = l.e[en].feats + (long long)sb * kF;
+  for (int i = tid; i < 18 * 18; i += 128) (&img[0][0])[i] = 0.f;
+  for (int i = tid; i < 144; i += 128) w1[i % 9][i / 9] = rbf(P[kW1 + i]);
   __syncthreads();
-  // conv 3x3 1 -> 16, stride 1
-  for (int e = tid; e < 256 * 16; e += 128) {
-    const int p = e >> 4, c = e & 15, y = p >> 4, xx = p & 15;
-    float s = 0.f;
+  for (int i = tid; i < kF; i += 128) {
+    const float v = rbf(x[i]);
+    xr[i] = v;
+    if (i < 256) img[1 + (i >> 4)][1 + (i & 15)] = v;
+  }
+  __syncthreads();
+  // conv 3x3 1 -> 16, stride 1: a thread a channel, every eighth position (taps outside add nothing, whatever
+  // the weights)
+  {
+    const int c = tid & 15;
+    const float b = P[kB1 + c];
+    float w[9];
 #pragma unroll
-    for (int ky = 0; ky < 3; ky++)
+    for (int k = 0; k < 9; k++) w[k] = w1[k][c];
+    for (int p = tid >> 4; p < 256; p += 8) {
+      const int y = p >> 4, xx = p & 15;
+      float s = 0.f;
 #pragma unroll
-      for (int kx = 0; kx < 3; kx++) {
-        const int iy = y + ky - 1, ix = xx + kx - 1;
-        if (iy >= 0 && iy < 16 && ix >= 0 && ix < 16) s += xr[iy * 16 + ix] * rbf(P[kW1 + c * 9 + ky * 3 + kx]);
-      }
-    a1[p][c] = __float2bfloat16_rn(fmaxf(s + P[kB1 + c], 0.f));
+      for (int k = 0; k < 9; k++)
+        if (!((k < 3 && y == 0) || (k >= 6 && y == 15) || (k % 3 == 0 && xx == 0) || (k % 3 == 2 && xx == 15)))
+          s += img[y + k / 3][xx + k % 3] * w[k];
+      a1[p][c] = __float2bfloat16_rn(fmaxf(s + b, 0.f));
+    }
   }
   __syncthreads();
   // conv 3x3 16 -> 32, stride 2: rows = 64 output positions (warp w: 16w..16w+15), K = tap x 16
@@ -852,6 +867,7 @@ __global__ void __launch_bounds__(128) k_infer(const float* __restrict__ P, cons
   {
     const int o = tid & 63, half = tid >> 6;
     float s = 0.f;
+#pragma unroll 16
     for (int k = half * 316; k < half * 316 + 316; k++) s += h0[k] * __bfloat162float(Wb[kIW4 + k * 64 + o]);
     part[tid] = s;
   }
@@ -865,7 +881,7 @@ __global__ void __launch_bounds__(128) k_infer(const float* __restrict__ P, cons
     if (lane == 0) logits[o] = s + P[kB5 + o];
   }
   __syncthreads();
-  if (tid == 0) keep[blockIdx.x] = mask_word(logits, nrefs, th);  // k_masks' rule
+  if (tid == 0) l.e[en].keep[sb] = mask_word(logits, l.e[en].nrefs, l.e[en].th);
 }
 }  // namespace nn
 
@@ -874,9 +890,8 @@ size_t infer_weight_elems() { return nn::kIWs; }
 void infer_weights(const float* params, void* wb, cudaStream_t st) {
   nn::k_infer_weights<<<nn::grid_for(nn::kIWs), 256, 0, st>>>(params, static_cast<__nv_bfloat16*>(wb));
 }
-void launch_infer(const float* params, const void* wb, const float* feats, int nsb, int nrefs,
-                  const PrunerThresholds& th, uint32_t* keep, cudaStream_t st) {
-  nn::k_infer<<<nsb, 128, 0, st>>>(params, static_cast<const __nv_bfloat16*>(wb), feats, nrefs, th, keep);
+void launch_infer(const NetList& l, cudaStream_t st) {
+  if (l.prefix[l.n] > 0) nn::k_infer<<<l.prefix[l.n], 128, 0, st>>>(l);
 }
 
 }  // namespace celv2cu
