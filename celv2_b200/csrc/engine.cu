@@ -294,9 +294,10 @@ struct celv2_engine {
   // batch's records to cross PCIe); copied[p] marks buffer set p's copies done.
   cudaStream_t copy_st = nullptr;
   cudaStream_t up_st = nullptr;  // celv2_upload's stream (frame-store uploads)
+  static constexpr int kMaxSlices = 16, kMaxWaves = 2;
   cudaStream_t fin_st = nullptr;  // the finalize of a batch in slices (high priority; st waits for it)
   cudaStream_t side_st = nullptr;  // every other slice's inter stage
-  cudaEvent_t front_done = nullptr, slice_ready[8] = {}, slice_done[8] = {};  // per slice (kMaxSlices)
+  cudaEvent_t front_done = nullptr, slice_ready[kMaxSlices] = {}, slice_done[kMaxSlices] = {};
   static constexpr int kRecordSets = 3;
   cudaEvent_t copied[kRecordSets] = {};
   bool copy_pending[kRecordSets] = {};
@@ -313,10 +314,10 @@ struct celv2_engine {
   double stage_ms[kStages] = {};
   long long stage_n[kStages] = {};
   unsigned long long* stats = nullptr;  // device work counters (kStats), while timing
-  // stage work queues (device counters): prepare's intra (its own stream); the motion-search levels
-  // and the refinement; per slice its intra, inter, inter by regions and finalize
-  static constexpr int kQueuePrep = 0, kQueueMe = 1, kQueueRefine = kQueueMe + kLevels, kQueueSlice = kQueueRefine + 1;
-  static constexpr int kMaxSlices = 8, kQueues = kQueueSlice + 4 * kMaxSlices;
+  // stage work queues (device counters): prepare's intra (its own stream); per wave the motion-search
+  // levels and the refinement; per slice its intra, inter, inter by regions and finalize
+  static constexpr int kQueuePrep = 0, kQueueMe = 1, kQueueSlice = kQueueMe + kMaxWaves * (kLevels + 1);
+  static constexpr int kQueues = kQueueSlice + 4 * kMaxSlices;
   unsigned* queues = nullptr;
   int* fault = nullptr;  // behind the ring, page-locked: set by a kernel whose wait for its copies ran out
   bool persistent = true;      // the queue-draining persistent stage kernels (else one CTA per unit)
@@ -713,18 +714,28 @@ struct celv2_engine {
     int sbs = 0;
   };
 
-  // Rows of superblocks in decision order, cut into slices for the records' way to the host. A
-  // batch's records leave at PCIe speed only once its last stage has run, so a launch of many
+  // Jobs j0 .. j1 - 1 searched together, decided in slices s0 .. s1 - 1.
+  struct Wave {
+    int j0, j1, s0, s1;
+  };
+  struct Plan {
+    std::vector<Slice> slices;
+    std::vector<Wave> waves;
+  };
+
+  // Rows of superblocks in decision order, cut into at most `most` slices for the records' way to the
+  // host. A batch's records leave at PCIe speed only once its last stage has run, so a launch of many
   // superblocks has its inter stage and finalize run slice by slice, the copies of one behind the
   // stages of the next. A slice is worth it from kSliceSbs superblocks on: 5 MB, ~90 us of copy,
   // against the ~30 us that the drained ends of its launches cost. Five 1080p leaves of 7 references
-  // in 2 / 4 / 8 slices: 7.29 / 6.47 / 6.08 ms; ten 720p leaves of 2 3.90 / 3.64 / 3.54; one masked 4K
-  // frame 3.24 / 3.17 / 3.17; a 1080p frame of the encoder's loop (3 at most) 2.01 / 1.94 / 2.0.
+  // in 2 / 4 / 8 / 16 slices: 7.29 / 6.47 / 5.63 / 5.45 ms; ten 720p leaves of 2 3.90 / 3.64 / 3.38 /
+  // 3.37; frames of six sizes 7.25 in 8, 6.86 in 16; one masked 4K frame 3.24 / 3.17 / 2.27 / 2.26; a
+  // 1080p frame of the encoder's loop (3 at most) 2.01 / 1.94 / 2.0.
   static constexpr int kSliceSbs = 128;
-  static std::vector<Slice> cut(const std::vector<SbRange>& rows, bool to_host) {
+  static std::vector<Slice> cut(const std::vector<SbRange>& rows, int most) {
     int total = 0;
     for (const SbRange& r : rows) total += r.sbs;
-    const int n = to_host ? std::max(1, std::min(kMaxSlices, total / kSliceSbs)) : 1;
+    const int n = std::max(1, std::min(most, total / kSliceSbs));
     std::vector<Slice> out(1);
     int done = 0;
     for (const SbRange& r : rows) {
@@ -744,45 +755,71 @@ struct celv2_engine {
     return out;
   }
 
-  // The rows of every job, job after job.
-  static std::vector<SbRange> rows_of(const std::vector<FrameJob>& jobs) {
-    std::vector<SbRange> rows;
-    for (int j = 0; j < (int)jobs.size(); j++)
-      for (int r = 0; r < jobs[j].sb_rows; r++) rows.push_back(SbRange{j, r * jobs[j].sb_cols, jobs[j].sb_cols});
-    return rows;
+  // A batch's way through the stages. Where the motion search of every job comes first, the records
+  // leave during the inter stage and finalize alone, and those are the shorter the fewer references there
+  // are (~0.1 us a superblock and reference, ~0.1 a superblock; its record's copy 0.73). So two waves of
+  // jobs are searched and decided one after the other where there are at most kWaveRefs references a
+  // superblock: ten 720p frames of 1 / 3 / 5 / 7 references 3.21 -> 2.65, 3.88 -> 3.45, 4.51 -> 4.29, 5.33
+  // -> 5.19 ms (in part by waiting for half the uploads only), but frames already on the GPU, five of
+  // 1080p, 2.90 -> 2.47, 3.69 -> 3.63, 4.36 -> 4.41, 5.12 -> 5.34: half a batch fills the GPU less well,
+  // its small search levels least. Three waves: 2.42, 3.41, 4.45, 5.38, and 720p 2.51, 3.46, 4.43, 5.52.
+  // Eight 640x360 frames (480 superblocks) 0.90 -> 0.83, 1.17 -> 1.08, 1.35 -> 1.28 ms.
+  static constexpr int kWaveSbs = 240, kWaveRefs = 5;
+  static Plan plan(const std::vector<FrameJob>& jobs, bool to_host) {
+    const int n = (int)jobs.size();
+    auto sbs = [&](int j) { return jobs[j].sb_cols * jobs[j].sb_rows; };
+    long long total = 0, units = 0;
+    for (int j = 0; j < n; j++) total += sbs(j), units += (long long)sbs(j) * jobs[j].nrefs;
+    int split = n;  // the second wave's first job
+    if (to_host && n > 1 && units > 0 && total >= 2 * kWaveSbs && units <= kWaveRefs * total) {
+      long long first = sbs(0);
+      for (split = 1; split < n - 1 && 2 * (first + sbs(split)) <= total; split++) first += sbs(split);
+    }
+    Plan p;
+    for (int j0 = 0; j0 < n; j0 = split, split = n) {
+      std::vector<SbRange> rows;
+      for (int j = j0; j < split; j++)
+        for (int r = 0; r < jobs[j].sb_rows; r++) rows.push_back(SbRange{j, r * jobs[j].sb_cols, jobs[j].sb_cols});
+      const int s0 = (int)p.slices.size();
+      for (Slice& s : cut(rows, !to_host ? 1 : j0 == 0 && split == n ? kMaxSlices : kMaxSlices / kMaxWaves))
+        p.slices.push_back(std::move(s));
+      p.waves.push_back(Wave{j0, split, s0, (int)p.slices.size()});
+    }
+    return p;
   }
 
   unsigned* queue(int stage_bit, int index) const {
     return persistent && !(persistent_off >> stage_bit & 1) ? queues + index : nullptr;
   }
 
-  // Queues the stages that come before the superblock stages, for the jobs whose descriptors are in
-  // djobs: motion search, the pruner between its levels 1 and 0, refinement; returns the kernels
-  // launched. Zeroes the work queues of the whole batch.
-  int enqueue_search(const std::vector<FrameJob>& jobs, cudaStream_t stream, const std::vector<NetJob>& nets) {
-    const int n = (int)jobs.size();
+  // Queues the stages that come before the superblock stages, for wave i's jobs (their descriptors in
+  // djobs): motion search, the pruner between its levels 1 and 0, refinement; returns the kernels
+  // launched.
+  int enqueue_search(const std::vector<FrameJob>& jobs, const Wave& v, int i, cudaStream_t stream,
+                     const std::vector<NetJob>& nets) {
+    const int n = v.j1 - v.j0, q = kQueueMe + i * (kLevels + 1);
+    const FrameJob* job = jobs.data() + v.j0;
     int launched = 0;
-    if (persistent) CK(cudaMemsetAsync(queues + kQueueMe, 0, (kQueues - kQueueMe) * sizeof(unsigned), stream));
     WorkList w{};
     w.nparts = n;
-    for (int j = 0; j < n; j++) w.part[j] = SbRange{j, 0, jobs[j].sb_cols * jobs[j].sb_rows};
+    for (int j = 0; j < n; j++) w.part[j] = SbRange{v.j0 + j, 0, job[j].sb_cols * job[j].sb_rows};
     for (int l = kLevels - 1; l >= 0; l--) {
       long long total = 0;
-      for (const FrameJob& jb : jobs) total += (long long)jb.nrefs * jb.fcols[l] * jb.frows[l];
+      for (int j = 0; j < n; j++) total += (long long)job[j].nrefs * job[j].fcols[l] * job[j].frows[l];
       const int cells = me_level_cells(total, me_cells[l]);
       for (int j = 0; j < n; j++)
-        w.prefix[j + 1] = w.prefix[j] + me_units(jobs[j].nrefs, jobs[j].fcols[l], jobs[j].frows[l], cells);
+        w.prefix[j + 1] = w.prefix[j] + me_units(job[j].nrefs, job[j].fcols[l], job[j].frows[l], cells);
       if (l == 0 && !nets.empty())  // the learned pruner, from the level-1 motion search
-        stage(kStPruner, stream, [&] { launched += enqueue_pruner(jobs, nets, stream); });
-      w.queue = queue(l, kQueueMe + l);
+        stage(kStPruner, stream, [&] { launched += enqueue_pruner(jobs, v, nets, stream); });
+      w.queue = queue(l, q + l);
       if (w.prefix[n] > 0) {
         stage(kStMe0 - l, stream, [&] { launch_me_level(djobs, w, l, cells, stream); });
         launched++;
       }
     }
     for (int j = 0; j < n; j++)
-      w.prefix[j + 1] = w.prefix[j] + refine_units(jobs[j].nrefs, jobs[j].fcols[0], jobs[j].frows[0]);
-    w.queue = queue(8, kQueueRefine);
+      w.prefix[j + 1] = w.prefix[j] + refine_units(job[j].nrefs, job[j].fcols[0], job[j].frows[0]);
+    w.queue = queue(8, q + kLevels);
     if (w.prefix[n] > 0) {
       stage(kStRefine, stream, [&] { launch_me_refine(djobs, w, stream); });
       launched++;
@@ -804,8 +841,8 @@ struct celv2_engine {
   }
 
   // Slice i's intra, inter and finalize; each returns the kernels launched.
-  int enqueue_intra(const std::vector<FrameJob>& jobs, const Slice& s, int i, cudaStream_t stream) {
-    const WorkList w = slice_list(jobs, s, false, queue(5, kQueueSlice + 4 * i));
+  int enqueue_intra(const std::vector<FrameJob>& jobs, const Slice& s, int q, cudaStream_t stream) {
+    const WorkList w = slice_list(jobs, s, false, queue(5, q));
     stage(kStIntra, stream, [&] { launch_intra(djobs, w, stream); });
     return 1;
   }
@@ -826,9 +863,9 @@ struct celv2_engine {
     return 1;
   }
 
-  // The pruner's features of every job that has them, then the network and the keep words of every
+  // The pruner's features of every job of a wave that has them, then the network and the keep words of every
   // superblock that has it; returns the kernels launched.
-  int enqueue_pruner(const std::vector<FrameJob>& jobs, const std::vector<NetJob>& nets, cudaStream_t stream) {
+  int enqueue_pruner(const std::vector<FrameJob>& jobs, const Wave& v, const std::vector<NetJob>& nets, cudaStream_t stream) {
     NetList feats{}, run{};
     auto add = [&](NetList& l, int j) {
       const NetJob& nj = nets[j];
@@ -836,7 +873,7 @@ struct celv2_engine {
       l.prefix[l.n + 1] = l.prefix[l.n] + jobs[j].sb_cols * jobs[j].sb_rows;
       l.n++;
     };
-    for (int j = 0; j < std::min((int)jobs.size(), (int)nets.size()); j++) {
+    for (int j = v.j0; j < std::min(v.j1, (int)nets.size()); j++) {
       if (!nets[j].feats) continue;
       add(feats, j);
       if (nets[j].net) add(run, j);
@@ -846,23 +883,24 @@ struct celv2_engine {
     return (feats.n > 0) + (run.n > 0);
   }
 
-  // Everything of a batch up to its slices: motion search, refinement, and intra (unless it runs on
+  // Everything of wave i up to its slices: motion search, refinement, and intra (unless it runs on
   // another stream, which records intra_done) where the slices do not run it; of a batch in one slice
   // also its inter stage and finalize. A batch without references has its intra in the slices: it is
   // all the work there is before the records.
   int enqueue_front(const std::vector<FrameJob>& jobs, cudaEvent_t intra_done, const std::vector<NetJob>& nets,
-                    const std::vector<Slice>& slices) {
-    int launched = enqueue_search(jobs, st, nets);
-    const bool whole = slices.size() == 1;
+                    const Plan& p, int i) {
+    const Wave& v = p.waves[i];
+    int launched = enqueue_search(jobs, v, i, st, nets);
+    const bool whole = p.slices.size() == 1;
     if (!intra_done && (whole || any_refs(jobs))) {
       Slice all;
-      for (int j = 0; j < (int)jobs.size(); j++) all.parts.push_back(SbRange{j, 0, jobs[j].sb_cols * jobs[j].sb_rows});
-      launched += enqueue_intra(jobs, all, 0, st);
+      for (int j = v.j0; j < v.j1; j++) all.parts.push_back(SbRange{j, 0, jobs[j].sb_cols * jobs[j].sb_rows});
+      launched += enqueue_intra(jobs, all, kQueueSlice + 4 * v.s0, st);
     }
     if (whole) {
-      launched += enqueue_inter(jobs, slices[0], 0, st);
+      launched += enqueue_inter(jobs, p.slices[0], 0, st);
       if (intra_done) CK(cudaStreamWaitEvent(st, intra_done, 0));
-      launched += enqueue_finalize(jobs, slices[0], 0, st);
+      launched += enqueue_finalize(jobs, p.slices[0], 0, st);
     }
     return launched;
   }
@@ -886,40 +924,44 @@ struct celv2_engine {
     CK(cudaStreamCreateWithPriority(&fin_st, cudaStreamNonBlocking, greatest));
   }
 
-  // The stages of a batch on st, its descriptors sent through the pinned ring (graph: the part up to
-  // the slices replayed as a CUDA graph). done(i, stream) is called once slice i's records are queued
-  // on `stream` -- to queue their copies. Several slices: their inter stages go to two streams in turn, so
+  // The stages of a batch on st, its descriptors sent through the pinned ring (graph: each wave's part up
+  // to its slices replayed as a CUDA graph). before(v) queues on st what wave v's jobs wait for; done(i,
+  // stream) is called once slice i's records are queued on `stream` -- to queue their copies. Several slices: their inter stages go to two streams in turn, so
   // one's CTAs take the SMs that the drained launch before it leaves (in one stream eight slices of five
   // 1080p leaves spent 2.07 ms in the stage that takes 1.60 in one launch), and their finalize to a third
   // of higher priority; st waits for the last finalize.
-  template <typename F>
+  template <typename B, typename F>
   void run(const std::vector<FrameJob>& jobs, cudaEvent_t intra_done, const std::vector<NetJob>& nets,
-           const std::vector<Slice>& slices, bool graph, F&& done) {
-    if (graph) {  // (never with intra on another stream)
-      launch_graph(jobs, nets, slices);
-    } else {
-      put_jobs(jobs.data(), (int)jobs.size(), djobs, st);
-      kernel_launches += enqueue_front(jobs, intra_done, nets, slices);
+           const Plan& p, bool graph, B&& before, F&& done) {
+    put_jobs(jobs.data(), (int)jobs.size(), djobs, st);
+    if (persistent) CK(cudaMemsetAsync(queues + kQueueMe, 0, (kQueues - kQueueMe) * sizeof(unsigned), st));
+    const int n = (int)p.slices.size();
+    if (n > 1) {
+      make_fin_stream();
+      if (intra_done) CK(cudaStreamWaitEvent(fin_st, intra_done, 0));
     }
-    const int n = (int)slices.size();
-    if (n == 1) {
-      done(0, st);
-      return;
-    }
-    make_fin_stream();
     const bool intra_here = !intra_done && !any_refs(jobs);
-    if (intra_done) CK(cudaStreamWaitEvent(fin_st, intra_done, 0));
-    CK(cudaEventRecord(front_done, st));
-    CK(cudaStreamWaitEvent(side_st, front_done, 0));
-    for (int i = 0; i < n; i++) {
-      cudaStream_t s = i & 1 ? side_st : st;
-      if (intra_here) kernel_launches += enqueue_intra(jobs, slices[i], i, s);
-      kernel_launches += enqueue_inter(jobs, slices[i], i, s);
-      CK(cudaEventRecord(slice_ready[i], s));
-      CK(cudaStreamWaitEvent(fin_st, slice_ready[i], 0));
-      kernel_launches += enqueue_finalize(jobs, slices[i], i, fin_st);
-      CK(cudaEventRecord(slice_done[i], fin_st));
-      done(i, fin_st);
+    for (int w = 0; w < (int)p.waves.size(); w++) {
+      const Wave& v = p.waves[w];
+      before(v);
+      kernel_launches += graph ? launch_graph(jobs, nets, p, w)  // (never with intra on another stream)
+                               : enqueue_front(jobs, intra_done, nets, p, w);
+      if (n == 1) {
+        done(0, st);
+        return;
+      }
+      CK(cudaEventRecord(front_done, st));
+      CK(cudaStreamWaitEvent(side_st, front_done, 0));
+      for (int i = v.s0; i < v.s1; i++) {
+        cudaStream_t s = i & 1 ? side_st : st;
+        if (intra_here) kernel_launches += enqueue_intra(jobs, p.slices[i], kQueueSlice + 4 * i, s);
+        kernel_launches += enqueue_inter(jobs, p.slices[i], i, s);
+        CK(cudaEventRecord(slice_ready[i], s));
+        CK(cudaStreamWaitEvent(fin_st, slice_ready[i], 0));
+        kernel_launches += enqueue_finalize(jobs, p.slices[i], i, fin_st);
+        CK(cudaEventRecord(slice_done[i], fin_st));
+        done(i, fin_st);
+      }
     }
     CK(cudaStreamWaitEvent(st, slice_done[n - 1], 0));
   }
@@ -1001,11 +1043,14 @@ struct celv2_engine {
           if (s * per + i < g.sb_rows) order.push_back(s * per + i);
       std::vector<SbRange> rows;
       for (int r : order) rows.push_back(SbRange{0, r * g.sb_cols, g.sb_cols});
-      std::vector<Slice> slices = cut(rows, true);
+      Plan p;
+      p.slices = cut(rows, kMaxSlices);
+      std::vector<Slice>& slices = p.slices;
       if ((int)slices.size() > kMaxSlices) slices.assign(1, Slice{});
       if (slices.size() == 1) slices[0].parts.assign(1, SbRange{0, 0, g.nsb}), slices[0].sbs = g.nsb;
+      p.waves.assign(1, Wave{0, 1, 0, (int)slices.size()});
       size_t next = 0;  // the next row of `order` to copy
-      run(jobs, prepared ? prep_done : nullptr, nets, slices, false, [&](int i, cudaStream_t ready) {
+      run(jobs, prepared ? prep_done : nullptr, nets, p, false, [](const Wave&) {}, [&](int i, cudaStream_t ready) {
         // one slice: the copies follow on st; several: on copy_st, beside the next slices' stages
         cudaStream_t cs = st;
         if (ready != st) {
@@ -1196,7 +1241,8 @@ struct celv2_engine {
         if (dests[j]) invalid("group: set_output names host memory, but to_host 0 leaves the records on the device");
     if (njobs > group_cap) reserve_group(std::max(njobs, 8));
     std::vector<FrameJob> jobs(njobs);
-    std::vector<Slot*> reads;
+    std::vector<Slot*> reads;  // per job its source and its references, from first[job]
+    std::vector<int> first(njobs);
     for (int j = 0; j < njobs; j++) {
       Slot* cur = find(src_keys[j]);
       if (!cur) invalid("group: no stored frame with the source key");
@@ -1208,13 +1254,9 @@ struct celv2_engine {
         refs[r] = find(ref_keys[j][r]);
         if (!refs[r]) invalid("group: no stored frame with a reference key");
       }
-      wait_ready(*cur, st);
+      first[j] = (int)reads.size();
       reads.push_back(cur);
-      for (int r = 0; r < nrefs[j]; r++) {
-        wait_ready(*refs[r], st);
-        reads.push_back(refs[r]);
-      }
-      make_phases(refs, nrefs[j], st);
+      for (int r = 0; r < nrefs[j]; r++) reads.push_back(refs[r]);
       fill_job(jobs[j], cur->pyr, refs, nrefs[j], group[j], group[j].intra, lams[j]);
     }
     std::vector<NetJob> nets(njobs);
@@ -1227,10 +1269,18 @@ struct celv2_engine {
     for (int j = 0; j < njobs; j++) jobs[j].out = group[j].records(par);
     for (int j = 0; j < njobs; j++)
       group_out[j] = !to_host ? nullptr : dests[j] ? dests[j] : group_host + (size_t)j * g.nsb;
-    const std::vector<Slice> slices = cut(rows_of(jobs), to_host);
-    run(jobs, nullptr, nets, slices, use_graphs && !timing, [&](int i, cudaStream_t ready) {
+    const Plan p = plan(jobs, to_host);
+    // a wave waits for the uploads of its own frames only
+    auto before = [&](const Wave& v) {
+      for (int j = v.j0; j < v.j1; j++) {
+        Slot* const* f = reads.data() + first[j];
+        for (int r = 0; r <= nrefs[j]; r++) wait_ready(*f[r], st);
+        make_phases(f + 1, nrefs[j], st);
+      }
+    };
+    run(jobs, nullptr, nets, p, use_graphs && !timing, before, [&](int i, cudaStream_t ready) {
       if (!to_host) return;  // records left on the device
-      copy_slice(slices[i], i, ready, [&](int j) { return std::make_pair(jobs[j].out, group_out[j]); });
+      copy_slice(p.slices[i], i, ready, [&](int j) { return std::make_pair(jobs[j].out, group_out[j]); });
     });
     mark_used(reads.data(), (int)reads.size(), st);
     if (to_host) {
@@ -1274,19 +1324,18 @@ struct celv2_engine {
     graphs.clear();
   }
 
-  // The batch up to its slices (enqueue_front), replayed.
-  void launch_graph(const std::vector<FrameJob>& jobs, const std::vector<NetJob>& nets,
-                    const std::vector<Slice>& slices) {
-    // the shape: whether its superblock stages are in the graph or follow in slices; per job its
-    // reference count, whether it has keep words (which decides whether the region pass of the inter
+  // Wave i of a batch up to its slices (enqueue_front), replayed; returns its kernels.
+  int launch_graph(const std::vector<FrameJob>& jobs, const std::vector<NetJob>& nets, const Plan& p, int i) {
+    // the shape: whether its superblock stages are in the graph or follow in slices; the wave, its
+    // first job and its first slice (its queues); per job of it its reference count, whether it has keep words (which decides whether the region pass of the inter
     // stage is launched at all), features and the network
-    std::vector<int> key{slices.size() == 1};
-    for (size_t j = 0; j < jobs.size(); j++)
+    const Wave& v = p.waves[i];
+    std::vector<int> key{p.slices.size() == 1, i, v.j0, v.s0};
+    for (int j = v.j0; j < v.j1; j++)
       key.push_back(jobs[j].nrefs * 8 + (jobs[j].keep ? 4 : 0) + (nets[j].feats ? 2 : 0) + (nets[j].net ? 1 : 0));
     Graph* gr = nullptr;
     for (Graph& x : graphs)
       if (x.key == key) gr = &x;
-    const int n = (int)jobs.size();
     if (!gr) {
       graphs.emplace_back();
       gr = &graphs.back();
@@ -1294,7 +1343,7 @@ struct celv2_engine {
       cudaGraph_t graph = nullptr;
       CK(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
       try {
-        gr->kernels = enqueue_front(jobs, nullptr, nets, slices);
+        gr->kernels = enqueue_front(jobs, nullptr, nets, p, i);
       } catch (...) {
         cudaStreamEndCapture(st, &graph);
         if (graph) cudaGraphDestroy(graph);
@@ -1306,9 +1355,8 @@ struct celv2_engine {
       cudaGraphDestroy(graph);
       CK(e);
     }
-    put_jobs(jobs.data(), n, djobs, st);
     CK(cudaGraphLaunch(gr->exec, st));
-    kernel_launches += gr->kernels;
+    return gr->kernels;
   }
 };
 
@@ -1411,10 +1459,10 @@ void launch_multi(int njobs, celv2_engine* const* engines, const long long* src_
     en.e->group_out[en.slot] = en.dest;
   }
   // the records on the lead's copy stream, overlapping later work
-  const std::vector<celv2_engine::Slice> slices = celv2_engine::cut(celv2_engine::rows_of(jobs), to_host);
-  lead->run(jobs, nullptr, nets, slices, false, [&](int i, cudaStream_t ready) {
+  const celv2_engine::Plan p = celv2_engine::plan(jobs, to_host);
+  lead->run(jobs, nullptr, nets, p, false, [](const celv2_engine::Wave&) {}, [&](int i, cudaStream_t ready) {
     if (!to_host) return;
-    lead->copy_slice(slices[i], i, ready, [&](int j) { return std::make_pair(jobs[j].out, entries[j].dest); });
+    lead->copy_slice(p.slices[i], i, ready, [&](int j) { return std::make_pair(jobs[j].out, entries[j].dest); });
   });
   for (size_t i = 0; i < uniq.size(); i++) uniq[i]->mark_used(reads[i].data(), (int)reads[i].size(), lead->st);
   if (to_host)
