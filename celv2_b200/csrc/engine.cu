@@ -597,6 +597,12 @@ struct celv2_engine {
     return Incoming{&s, &sg, PlaneIn{sg.dev, wide ? f->bit_depth - 8 : -1, s.pyr}};
   }
 
+  // Whether a plane goes to the GPU in one piece. A batch's descriptors and zeroed queues then go ahead of the
+  // planes' kernels: behind them, before the first stage, they were 18 us of a 416x240 frame's 360 and 11 of a
+  // 202x122 one's 107 (now 349, 97). For planes in pieces they stay behind: a 1080p KEY frame took 930 us
+  // with them ahead against 912, two of its encoder loop's frames 3.53 ms against 3.45 (measured; why is open).
+  bool one_piece(const celv2_frame* f) const { return (size_t)g.pw * g.ph * (f->y ? 1 : 2) <= kCopyPiece; }
+
   // Queues level 0 and the pyramid of every frame brought in on `stream`, one launch for all of them.
   void make_planes(const std::vector<Incoming>& in, cudaStream_t stream) {
     for (size_t i = 0; i < in.size();) {
@@ -705,6 +711,12 @@ struct celv2_engine {
     CK(cudaMemcpyAsync(dst, h, n * sizeof(FrameJob), cudaMemcpyHostToDevice, stream));
     CK(cudaEventRecord(ring_done[i], stream));
     ring_pending[i] = true;
+  }
+
+  // Queues a batch's descriptors, and its work queues' zeros, on st.
+  void put_batch(const std::vector<FrameJob>& jobs) {
+    put_jobs(jobs.data(), (int)jobs.size(), djobs, st);
+    if (persistent) CK(cudaMemsetAsync(queues + kQueueMe, 0, (kQueues - kQueueMe) * sizeof(unsigned), st));
   }
 
   // ---- the stages of a batch ----
@@ -924,8 +936,8 @@ struct celv2_engine {
     CK(cudaStreamCreateWithPriority(&fin_st, cudaStreamNonBlocking, greatest));
   }
 
-  // The stages of a batch on st, its descriptors sent through the pinned ring (graph: each wave's part up
-  // to its slices replayed as a CUDA graph). before(v) queues on st what wave v's jobs wait for; done(i,
+  // The stages of a batch on st, its descriptors and zeroed queues already queued there (put_batch; graph:
+  // each wave's part up to its slices replayed as a CUDA graph). before(v) queues on st what wave v's jobs wait for; done(i,
   // stream) is called once slice i's records are queued on `stream` -- to queue their copies. Several slices: their inter stages go to two streams in turn, so
   // one's CTAs take the SMs that the drained launch before it leaves (in one stream eight slices of five
   // 1080p leaves spent 2.07 ms in the stage that takes 1.60 in one launch), and their finalize to a third
@@ -933,8 +945,6 @@ struct celv2_engine {
   template <typename B, typename F>
   void run(const std::vector<FrameJob>& jobs, cudaEvent_t intra_done, const std::vector<NetJob>& nets,
            const Plan& p, bool graph, B&& before, F&& done) {
-    put_jobs(jobs.data(), (int)jobs.size(), djobs, st);
-    if (persistent) CK(cudaMemsetAsync(queues + kQueueMe, 0, (kQueues - kQueueMe) * sizeof(unsigned), st));
     const int n = (int)p.slices.size();
     if (n > 1) {
       make_fin_stream();
@@ -992,6 +1002,7 @@ struct celv2_engine {
     if (nrefs > 0 && (g.pw < 16 || g.ph < 16)) invalid("CudaEngine: inter frames need at least 9x9 pixels");
     if (pending) wait_idle();
     recover_stages();
+    std::vector<std::pair<Slot*, int>> fresh_refs;  // references not in the cache yet, until they are on their way
     try {
       // the prepared source, else an upload into the other slot: with the intra stage beside the
       // references' uploads and the motion search, on prepare's stream, where nothing decides it anew
@@ -1006,34 +1017,42 @@ struct celv2_engine {
         if (nrefs > 0 && keep0.empty() && !pruner_params) {
           start_source(src, use);
           prepared = true;
-        } else {
-          make_planes({bring(src, srcs[use], st, false)}, st);
         }
       }
-      if (prepared) CK(cudaStreamWaitEvent(st, src_up, 0));
       srcs[use].key = -1;  // used: a later prepare() may overwrite it
       cur_src = use;
       const long long now = ++launches;
       Slot* used[kMaxRefs];
-      std::vector<Incoming> fresh_refs;
       for (int r = 0; r < nrefs; r++) {
         bool fresh;
         Slot* s = ref_slot(keys ? keys[r] : -1, keys, keys ? nrefs : 0, now, fresh);
-        wait_ready(*s, st);  // a frame of the store; a dropped one's upload may still run
         if (fresh) {
-          fresh_refs.push_back(bring(&refs[r], *s, st, true));
+          alloc_slot(*s, true);
+          fresh_refs.emplace_back(s, r);
           s->key = keys ? keys[r] : -1;
         }
         s->used = now;
         used[r] = s;
       }
-      make_planes(fresh_refs, st);
-      make_phases(used, nrefs, st);
       std::vector<FrameJob> jobs(1);
       fill_job(jobs[0], srcs[use].pyr, used, nrefs, single, intra_prep[use], lam);
       jobs[0].keep = put_keep(keep0, single, st);
       const std::vector<NetJob> nets{net_for(jobs[0], single, !keep0.empty())};
       if (nets[0].net) jobs[0].keep = single.keep;
+      std::vector<Incoming> in;
+      if (!prepared) in.push_back(bring(src, srcs[use], st, false));
+      for (const auto& [s, r] : fresh_refs) {
+        wait_ready(*s, st);  // a dropped store frame's memory: its upload may still run
+        in.push_back(bring(&refs[r], *s, st, true));
+      }
+      const bool small = one_piece(src);
+      if (small) put_batch(jobs);
+      make_planes(in, st);
+      fresh_refs.clear();
+      for (int r = 0; r < nrefs; r++) wait_ready(*used[r], st);  // frames of the store
+      make_phases(used, nrefs, st);
+      if (!small) put_batch(jobs);
+      if (prepared) CK(cudaStreamWaitEvent(st, src_up, 0));
       // rows back to the host in row-stream order
       const int streams = std::max(1, std::min(row_streams, g.sb_rows));
       const int per = (g.sb_rows + streams - 1) / streams;
@@ -1076,6 +1095,7 @@ struct celv2_engine {
       last_out = dest;
       pending = true;
     } catch (...) {
+      for (const auto& f : fresh_refs) f.first->key = -1;  // their planes were not made
       cudaStreamSynchronize(st);  // a failure leaves no work running
       if (side_st) cudaStreamSynchronize(side_st);
       if (fin_st) cudaStreamSynchronize(fin_st);
@@ -1100,8 +1120,9 @@ struct celv2_engine {
   // every superblock (prep_done) of source slot i.
   void start_source(const celv2_frame* f, int i) {
     Slot& s = srcs[i];
-    make_planes({bring(f, s, prep_st, false)}, prep_st);
-    CK(cudaEventRecord(src_up, prep_st));
+    const std::vector<Incoming> in{bring(f, s, prep_st, false)};
+    const bool small = one_piece(f);
+    if (!small) make_planes(in, prep_st), CK(cudaEventRecord(src_up, prep_st));
     std::vector<FrameJob> jobs(1);
     JobBuffers none{};
     fill_job(jobs[0], s.pyr, nullptr, 0, none, intra_prep[i], 0);
@@ -1116,6 +1137,7 @@ struct celv2_engine {
       CK(cudaMemsetAsync(queues + kQueuePrep, 0, sizeof(unsigned), prep_st));
       w.queue = queues + kQueuePrep;
     }
+    if (small) make_planes(in, prep_st), CK(cudaEventRecord(src_up, prep_st));
     stage(kStIntra, prep_st, [&] { launch_intra(dprep, w, prep_st); });
     kernel_launches++;
     CK(cudaGetLastError());
@@ -1278,6 +1300,7 @@ struct celv2_engine {
         make_phases(f + 1, nrefs[j], st);
       }
     };
+    put_batch(jobs);
     run(jobs, nullptr, nets, p, use_graphs && !timing, before, [&](int i, cudaStream_t ready) {
       if (!to_host) return;  // records left on the device
       copy_slice(p.slices[i], i, ready, [&](int j) { return std::make_pair(jobs[j].out, group_out[j]); });
@@ -1460,6 +1483,7 @@ void launch_multi(int njobs, celv2_engine* const* engines, const long long* src_
   }
   // the records on the lead's copy stream, overlapping later work
   const celv2_engine::Plan p = celv2_engine::plan(jobs, to_host);
+  lead->put_batch(jobs);
   lead->run(jobs, nullptr, nets, p, false, [](const celv2_engine::Wave&) {}, [&](int i, cudaStream_t ready) {
     if (!to_host) return;
     lead->copy_slice(p.slices[i], i, ready, [&](int j) { return std::make_pair(jobs[j].out, entries[j].dest); });
