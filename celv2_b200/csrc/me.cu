@@ -116,15 +116,6 @@ __device__ __forceinline__ void load_cur(const uint32_t* c, uint32_t* cw) {
   }
 }
 
-// The 4-byte windows at p and p + 1 (any alignment) from two aligned 32-bit loads.
-__device__ __forceinline__ void load_pair(const uint8_t* p, uint32_t& lo4, uint32_t& hi4) {
-  const uintptr_t a = reinterpret_cast<uintptr_t>(p);
-  const uint32_t* w = reinterpret_cast<const uint32_t*>(a & ~uintptr_t(3));
-  const uint32_t sh = (uint32_t)(a & 3) * 8, w0 = __ldg(w), w1 = __ldg(w + 1);
-  lo4 = __funnelshift_r(w0, w1, sh);
-  hi4 = __funnelshift_rc(w0, w1, sh + 8);  // a shift of 32 gives w1
-}
-
 // The refinement step's position n (raster 0..8 with the centre, 4, visited first).
 __device__ __forceinline__ int refine_pos(int t) { return t == 0 ? 4 : (t <= 4 ? t - 1 : t); }
 
@@ -375,42 +366,53 @@ __global__ void __launch_bounds__(kMeThreads, 1024 / kMeThreads) k_me_level(cons
 }
 
 // ---- quarter-pel refinement of level 0 (me_refine, inter_common.h:141-154) ----
-// One CTA per 32 consecutive level-0 cells of one (job, reference), 4 warps: warp t holds tile t
-// of the cells' four 4x4 tiles, a lane per cell, the cur tile row-transformed once into registers.
-// In each step a lane scores its tile at the step's nine positions; the lanes of a load read the
-// same row of the same tile for 32 neighbouring cells, which where their MVs agree -- most of a
-// frame -- is one contiguous run of a phase plane's row (a lane per (cell, position, tile)
-// scattered each warp's loads over nine phase planes and was bound by the L1's wavefronts; a warp
-// per position re-read the cur coefficients from shared memory nine times a step). The four tiles'
-// SATDs meet in shared memory and every lane replays its cell's centre-first strict choice from
-// them (the same in all four warps, so one barrier per step). The second step's centre is the
-// first step's winner, whose SATD the first step has already computed. The centre comes first of all:
-// a move has to save more than kSubpelPenalty, so a unit none of whose centres costs more is done (five
-// 1080p animation-like frames of 7 references 0.53 -> 0.24 ms). The other positions go in pairs
-// (satd4_pair): 0.56 -> 0.53 ms on natural-like ones.
-// The four rows of the 4x4 tile at (ox, oy) displaced by quarter pels (qx, qy).
-__device__ __forceinline__ void rows_at(const DevPlane& ref, int ox, int oy, int qx, int qy, uint32_t* pr) {
+// One CTA of two warps per 32 consecutive level-0 cells of one (job, reference): a warp holds the halves
+// of 16 cells, a lane the upper or the lower two of a cell's four 4x4 tiles side by side, their cur rows
+// row-transformed once into registers. In each step a lane scores its tiles at the step's nine positions,
+// three words a row and one satd4_two each; the lanes of a load read the same row of 16 neighbouring
+// cells, which where their MVs agree -- most of a frame -- is one contiguous run of a phase plane's row
+// (a lane per (cell, position, tile) scattered each warp's loads over nine phase planes and was bound by
+// the L1's wavefronts). One shuffle adds a cell's halves, two positions at a time, and both its lanes
+// replay the centre-first strict choice: no shared memory, no barrier within a unit. The second step's
+// centre is the first step's winner, whose SATD the first step has already computed. The centre comes
+// first of all: a move has to save more than kSubpelPenalty, so a warp none of whose centres costs more is
+// done (five 1080p animation-like frames of 7 references 0.53 -> 0.24 ms).
+// Five 1080p frames of 7 references: natural-like 532 -> 438 us, one masked 4K animation-like 114 -> 85,
+// against a lane per tile in four warps with the sums through shared memory and a barrier each step. 72
+// registers: with 64 it spills (502), with 80 the animation-like one takes 90 (natural-like 434).
+
+// The rows of a half cell's two tiles at (ox, oy) displaced by quarter pels (qx, qy).
+__device__ __forceinline__ void rows_at(const DevPlane& ref, int ox, int oy, int qx, int qy, uint32_t* a, uint32_t* b) {
   DevPlane ph = ref;
   ph.p = ref.p + (long long)((qy & 3) * 4 + (qx & 3)) * ref.phase;
   const int x = ox + (qx >> 2), y = oy + (qy >> 2);
-  if (inside(ph, x, y, 4, 4)) {
-    const uint8_t* p = ph.p + (long long)y * ph.stride + x;
+  if (inside(ph, x, y, 8, 4)) {
+    const uintptr_t p = reinterpret_cast<uintptr_t>(ph.p + (long long)y * ph.stride + x);
+    const uint32_t* w = reinterpret_cast<const uint32_t*>(p & ~uintptr_t(3));
+    const uint32_t sh = (uint32_t)(p & 3) * 8;
+    const int ws = ph.stride >> 2;  // strides are multiples of 64
 #pragma unroll
-    for (int i = 0; i < 4; i++) pr[i] = load4(p + (long long)i * ph.stride);
+    for (int i = 0; i < 4; i++) {
+      const uint32_t w0 = __ldg(w + i * ws), w1 = __ldg(w + i * ws + 1), w2 = __ldg(w + i * ws + 2);
+      a[i] = __funnelshift_r(w0, w1, sh), b[i] = __funnelshift_r(w1, w2, sh);
+    }
   } else {
 #pragma unroll
-    for (int i = 0; i < 4; i++) pr[i] = row4(ph, x, y + i);
+    for (int i = 0; i < 4; i++) a[i] = row4(ph, x, y + i), b[i] = row4(ph, x + 4, y + i);
   }
 }
 
-constexpr int kRefineCells = 32, kRefineTiles = 4, kRefineThreads = 32 * kRefineTiles;
+// The SATD of both tiles.
+__device__ __forceinline__ uint32_t satd_half(const int* P, const uint32_t* a, const uint32_t* b) {
+  const uint32_t v = satd4_two(P, a, b);
+  return (v & 0xffffu) + (v >> 16);  // at most 32,640
+}
 
-__global__ void __launch_bounds__(kRefineThreads, 8) k_me_refine(const FrameJob* __restrict__ jobs, WorkList w) {
-  // [step][pair][tile][cell]: the SATDs of positions 2 pair + 1 and 2 pair + 2 in halfwords (a cell's four
-  // tiles sum to at most 65,280), and of the first step's centre
-  __shared__ uint32_t sat[2][4][kRefineTiles][kRefineCells], sat0[kRefineTiles][kRefineCells];
+constexpr int kRefineCells = 32, kRefineThreads = 2 * kRefineCells;
+
+__global__ void __launch_bounds__(kRefineThreads, 14) k_me_refine(const FrameJob* __restrict__ jobs, WorkList w) {
   __shared__ int unit_slot[2];
-  const int tid = threadIdx.x, c = tid & 31, t = tid >> 5;
+  const int tid = threadIdx.x, c = (tid >> 5) * 16 + (tid & 15), half = tid >> 4 & 1;
   int unit, iter = 0;
   while (take_unit(w, unit, iter, unit_slot)) {
   const int jb = part_of(w, unit);
@@ -422,86 +424,101 @@ __global__ void __launch_bounds__(kRefineThreads, 8) k_me_refine(const FrameJob*
   const int ncells = min(kRefineCells, ncell - cell0);
   const int cell = cell0 + min(c, ncells - 1), by = cell / cols, bx = cell - by * cols;
   const bool need = c < ncells && cell_needed(job, r, bx, by);
-  // a unit none of whose cells a kept reference reads (pruned search): nothing to refine
-  if (!__syncthreads_or(need)) continue;
+  // a warp none of whose cells a kept reference reads (pruned search): nothing to refine
+  if (!__any_sync(0xffffffffu, need)) continue;
   const DevPlane cur = job.cur.lv[0], ref = job.ref[r].lv[0];
   int* field = job.field[r][0];
-  // this lane's tile of its cell: origin, cur rows row-transformed
-  const int ox = bx * 8 + 4 * (t & 1), oy = by * 8 + 4 * (t >> 1);
-  int C[16];
+  // this lane's half of its cell: origin, both tiles' cur rows row-transformed
+  const int ox = bx * 8, oy = by * 8 + 4 * half;
+  int P[16];
   {
     uint32_t cw[4];
+    int C[16];
+#pragma unroll
+    for (int i = 0; i < 4; i++) cw[i] = row4(cur, ox + 4, oy + i);
+    wh_rows_cur(cw, C);
 #pragma unroll
     for (int i = 0; i < 4; i++) cw[i] = row4(cur, ox, oy + i);
-    wh_rows_cur(cw, C);
+    wh_rows_cur(cw, P);
+#pragma unroll
+    for (int i = 0; i < 16; i++) P[i] += C[i] * 65536;
   }
   const int m = field[cell];
-  int cx = mv_x(m), cy = mv_y(m);  // quarter pels
-  int centre;                      // the centre's SATD (the cell's four tiles)
+  int cx = mv_x(m), cy = mv_y(m);  // quarter pels, whole pels so far
+  int centre;                      // the centre's SATD (the whole cell)
   {
-    uint32_t pr[4];
-    rows_at(ref, ox, oy, cx, cy, pr);
-    sat0[t][c] = (uint32_t)satd4_rows(C, pr);
-    __syncthreads();
-    centre = (int)(sat0[0][c] + sat0[1][c] + sat0[2][c] + sat0[3][c]);
+    uint32_t a[4], b[4];
+    rows_at(ref, ox, oy, cx, cy, a, b);
+    centre = (int)satd_half(P, a, b);
+    centre += __shfl_xor_sync(0xffffffffu, centre, 16);
     // a move must save more than kSubpelPenalty: cells whose centre costs no more stay (flat content: all
-    // of a unit's)
+    // of a warp's)
     if (!__any_sync(0xffffffffu, need && centre > kSubpelPenalty)) continue;
   }
-#pragma unroll
-  for (int s = 0; s < 2; s++) {
-    const int step = 2 - s;
-    // the half-pel step around a whole-pel MV reads four phase planes only (phase 2 one pel left
-    // or up of phase 0 at -1/2 pel, at the same pel at +1/2): the rows of the 5 x 5 footprint are
-    // loaded once per plane and the positions that share a plane take 4-byte windows of them
+  // takes a position (dx, dy) of the step around (px, py) if it beats the best so far
+  int best, raw, px, py, nx, ny;
+  auto choose = [&](int v, int dx, int dy) {
+    if (v + kSubpelPenalty < best) best = v + kSubpelPenalty, raw = v, nx = px + dx, ny = py + dy;
+  };
+#pragma unroll 1
+  for (int step = 2; step >= 1; step--) {
+    best = raw = centre, px = nx = cx, py = ny = cy;
+    // the half-pel step around the whole-pel MV reads four phase planes only (phase 2 one pel left
+    // or up of phase 0 at -1/2 pel, at the same pel at +1/2): the rows of the 9 x 5 footprint are
+    // loaded once per plane and the positions that share a plane take 8-byte windows of them
     const int X = ox + (cx >> 2), Y = oy + (cy >> 2);
-    if (s == 0 && !((cx | cy) & 3) && inside(ref, X - 1, Y - 1, 5, 5)) {
-      const long long rs = ref.stride;
-      const uint8_t* p00 = ref.p + (long long)Y * rs + X;
-      uint32_t pr[5], lf[5], rt[5];
-      const uint8_t* p20 = p00 + 8 * ref.phase;  // phase (2, 0): rows Y - 1 .. Y + 3
+    if (step == 2 && __all_sync(0xffffffffu, inside(ref, X - 1, Y - 1, 9, 5))) {
+      const int ws = ref.stride >> 2;
+      // n rows from Y + y0 of phase `ph` at column X + x: the windows at it and (x < 0) a column on
+      uint32_t a[5], b[5], e[5], f[5];
+      auto rows = [&](int ph, int x, int y0, int n) {
+        const uintptr_t p = reinterpret_cast<uintptr_t>(ref.p + ph * ref.phase + (long long)(Y + y0) * ref.stride + X + x);
+        const uint32_t* q = reinterpret_cast<const uint32_t*>(p & ~uintptr_t(3));
+        const uint32_t sh = (uint32_t)(p & 3) * 8;
 #pragma unroll
-      for (int i = 0; i < 5; i++) pr[i] = load4(p20 + (i - 1) * rs);
-      const uint32_t v27 = satd4_pair(C, pr, pr + 1);  // positions 2 and 7: (0, -1/2), (0, +1/2)
-      const uint8_t* p02 = p00 + 2 * ref.phase - 1;  // phase (0, 2): columns X - 1 .. X + 3
-#pragma unroll
-      for (int i = 0; i < 4; i++) load_pair(p02 + i * rs, lf[i], rt[i]);
-      const uint32_t v45 = satd4_pair(C, lf, rt);  // 4 and 5: (-1/2, 0), (+1/2, 0)
-      const uint8_t* p22 = p00 + 10 * ref.phase - 1;  // phase (2, 2): both
-#pragma unroll
-      for (int i = 0; i < 5; i++) load_pair(p22 + (i - 1) * rs, lf[i], rt[i]);
-      const uint32_t v13 = satd4_pair(C, lf, rt);          // 1 and 3: (-1/2, -1/2), (+1/2, -1/2)
-      const uint32_t v68 = satd4_pair(C, lf + 1, rt + 1);  // 6 and 8: (-1/2, +1/2), (+1/2, +1/2)
-      sat[0][0][t][c] = __byte_perm(v13, v27, 0x5410);
-      sat[0][1][t][c] = __byte_perm(v13, v45, 0x5432);
-      sat[0][2][t][c] = __byte_perm(v45, v68, 0x5432);
-      sat[0][3][t][c] = __byte_perm(v27, v68, 0x7632);
+        for (int i = 0; i < 5; i++)
+          if (i < n) {
+            const uint32_t w0 = __ldg(q + i * ws), w1 = __ldg(q + i * ws + 1), w2 = __ldg(q + i * ws + 2);
+            a[i] = __funnelshift_r(w0, w1, sh), b[i] = __funnelshift_r(w1, w2, sh);
+            if (x < 0) e[i] = __funnelshift_rc(w0, w1, sh + 8), f[i] = __funnelshift_rc(w1, w2, sh + 8);  // 32: the next word
+          }
+      };
+      // per word two positions' SATDs of the half, then of the cell (at most 65,280 each)
+      rows(8, 0, -1, 5);  // phase (2, 0): (0, -1/2) and (0, +1/2)
+      uint32_t up = satd_half(P, a, b) << 16, down = satd_half(P, a + 1, b + 1) << 16;
+      rows(2, -1, 0, 4);  // phase (0, 2): (-1/2, 0) and (+1/2, 0)
+      uint32_t mid = satd_half(P, a, b) | satd_half(P, e, f) << 16;
+      rows(10, -1, -1, 5);  // phase (2, 2): the corners
+      up |= satd_half(P, a, b), down |= satd_half(P, a + 1, b + 1);
+      uint32_t right = satd_half(P, e, f) | satd_half(P, e + 1, f + 1) << 16;
+      up += __shfl_xor_sync(0xffffffffu, up, 16), mid += __shfl_xor_sync(0xffffffffu, mid, 16);
+      down += __shfl_xor_sync(0xffffffffu, down, 16), right += __shfl_xor_sync(0xffffffffu, right, 16);
+      choose(up & 0xffffu, -2, -2), choose(up >> 16, 0, -2), choose(right & 0xffffu, 2, -2);
+      choose(mid & 0xffffu, -2, 0), choose(mid >> 16, 2, 0);
+      choose(down & 0xffffu, -2, 2), choose(down >> 16, 0, 2), choose(right >> 16, 2, 2);
     } else {
+      // the eight positions in order, two at a time
+#pragma unroll 1
+      for (int k = 1; k < 9; k += 2) {
+        uint32_t two = 0;
+        int d[2][2];
 #pragma unroll
-      for (int k = 0; k < 4; k++) {
-        uint32_t pa[4], pb[4];
-        const int na = refine_pos(2 * k + 1), nb = refine_pos(2 * k + 2);
-        rows_at(ref, ox, oy, cx + (na % 3 - 1) * step, cy + (na / 3 - 1) * step, pa);
-        rows_at(ref, ox, oy, cx + (nb % 3 - 1) * step, cy + (nb / 3 - 1) * step, pb);
-        sat[s][k][t][c] = satd4_pair(C, pa, pb);
+        for (int h = 0; h < 2; h++) {
+          uint32_t a[4], b[4];
+          const int n = refine_pos(k + h), row = n >= 6 ? 1 : n >= 3 ? 0 : -1;
+          d[h][0] = (n - 4 - 3 * row) * step, d[h][1] = row * step;
+          rows_at(ref, ox, oy, cx + d[h][0], cy + d[h][1], a, b);
+          two |= satd_half(P, a, b) << (16 * h);
+        }
+        two += __shfl_xor_sync(0xffffffffu, two, 16);
+        choose(two & 0xffffu, d[0][0], d[0][1]);
+        choose(two >> 16, d[1][0], d[1][1]);
       }
     }
-    __syncthreads();
-    // the cell's choice (me_refine: the centre first, a move must save kSubpelPenalty)
-    int best = centre;
-    int raw = best, nx = cx, ny = cy;
-#pragma unroll
-    for (int k = 0; k < 4; k++) {
-      const uint32_t two = sat[s][k][0][c] + sat[s][k][1][c] + sat[s][k][2][c] + sat[s][k][3][c];
-#pragma unroll
-      for (int h = 0; h < 2; h++) {
-        const int v = (int)(h ? two >> 16 : two & 0xffffu), n = refine_pos(2 * k + 1 + h);
-        if (v + kSubpelPenalty < best) best = v + kSubpelPenalty, raw = v, nx = cx + (n % 3 - 1) * step, ny = cy + (n / 3 - 1) * step;
-      }
-    }
+    // the next step's centre: its SATD is known
     centre = raw, cx = nx, cy = ny;
   }
-  if (t == 0 && need) field[cell] = pack_mv(cx, cy);
+  if (!half && need) field[cell] = pack_mv(cx, cy);
   }  // units
 }
 
