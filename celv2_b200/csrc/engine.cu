@@ -8,10 +8,10 @@
 //  - two source slots: while one frame is decided, prepare() builds the next one's pyramid and
 //    intra SATDs on a second stream (vk_engine.cpp:80-87,188-205);
 //  - per launch: the stage kernels on the main stream -- motion search level by level for every
-//    reference, intra (unless prepared), inter candidates, finalize -- then one device-to-host
-//    copy per superblock row with an event, so rows are collected as they arrive
-//    (vk_engine.cpp:288-328);
-//  - uploads go through a ring of pinned staging buffers: launch() copies the caller's planes into
+//    reference, intra (unless prepared), inter candidates, finalize, the last two in slices --
+//    then device-to-host copies of superblock rows with an event each, so rows are collected as
+//    they arrive (vk_engine.cpp:288-328);
+//  - uploads go through a pool of pinned staging buffers: launch() copies the caller's planes into
 //    pinned memory before it returns (the reference requires that the inputs may change at once,
 //    decision_engine.h:12-16).
 // No CPU fallback: every decision is made by the kernels; a missing GPU is an error.

@@ -24,7 +24,7 @@
 // DC, V and H predictions change only 1, 4 and 4 of the 16 coefficients (a constant tile only the
 // DC; equal rows only the first coefficient of each column transform; constant rows only the
 // first row transform), so those three modes cost a few operations on the cur transform; the ten
-// others pack their prediction rows into bytes and run the dp4a row transform (satd4_rows).
+// others pack their prediction rows into bytes and run the dp4a row transform two at a time (satd4_pair).
 // Word-wide predictions: D45's and D135's rows are windows of two words, D67 / D203 blends of two
 // 4-byte runs with one weight per row / column, in two 16-bit lanes. D113 and D157 project onto the
 // row above or the left column, sample by sample; along a row every sample that lands above shares

@@ -111,7 +111,8 @@ __device__ __forceinline__ int tap_row(int oy, int ox, int ky, int kx) {
 // ---- forward: the convolutions, two samples at a time ----
 struct FwdSmem {
   bf16 w2[32 * kSw2], w3[32 * kSw3];
-  float w1[9][16], b1[16], b2[32], b3[32];
+  bf16 w1[16][kS1];          // nine taps, then zeros
+  float b1[16], b2[32], b3[32];
   float x[2][18][18];        // the images, BF16-rounded, with a border of zeros
   bf16 a1[2][257][kS1], a2[2][65][kS2];
 };
@@ -122,7 +123,7 @@ __global__ void __launch_bounds__(kNnThreads, 3) k_conv_forward(const float* __r
   FwdSmem& S = *reinterpret_cast<FwdSmem*>(smem_raw);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
   stage_conv_weights(P, S.w2, S.w3);
-  if (tid < 144) S.w1[tid % 9][tid / 9] = rbf(P[kW1 + tid]);
+  S.w1[tid >> 4][tid & 15] = __float2bfloat16_rn((tid & 15) < 9 ? P[kW1 + (tid >> 4) * 9 + (tid & 15)] : 0.f);
   if (tid < 16) S.b1[tid] = P[kB1 + tid];
   if (tid < 32) S.b2[tid] = P[kB2 + tid], S.b3[tid] = P[kB3 + tid];
   for (int i = tid; i < 2 * 18 * 18; i += kNnThreads) (&S.x[0][0][0])[i] = 0.f;
@@ -142,37 +143,37 @@ __global__ void __launch_bounds__(kNnThreads, 3) k_conv_forward(const float* __r
       }
     }
     __syncthreads();
-    {  // 3x3, 1 -> 16: a thread a position, its nine samples against all sixteen channels
-      const int y = tid >> 4, x = tid & 15;
-#pragma unroll 1
-      for (int s = 0; s < 2; s++) {
-        float acc[16];
+    const int s = warp >> 2, q = warp & 3;  // the warp's sample, and its quarter of the work
+    {  // 3x3, 1 -> 16: four rows of 16 positions a warp, a row one product of its nine taps
+      uint32_t w[4];
 #pragma unroll
-        for (int c = 0; c < 16; c++) acc[c] = 0.f;
-#pragma unroll 1
-        for (int ky = 0; ky < 3; ky++)
+      for (int j = 0; j < 4; j++) w[j] = *reinterpret_cast<const uint32_t*>(&S.w1[(j >> 1) * 8 + g][2 * t + (j & 1) * 8]);
+      const int k0 = 2 * t, k1 = 2 * t + 1;
 #pragma unroll
-          for (int kx = 0; kx < 3; kx++) {
-            const float v = S.x[s][y + ky][x + kx];
+      for (int i = 0; i < 4; i++) {
+        const int y = q * 4 + i;
+        uint32_t a[4];
 #pragma unroll
-            for (int c = 0; c < 16; c++) acc[c] += v * S.w1[3 * ky + kx][c];
-          }
-        uint32_t h[8];
-#pragma unroll
-        for (int c = 0; c < 16; c++) acc[c] = fmaxf(acc[c] + S.b1[c], 0.f);
-#pragma unroll
-        for (int c = 0; c < 8; c++) h[c] = pack2(acc[2 * c], acc[2 * c + 1]);
-        uint4* row = reinterpret_cast<uint4*>(S.a1[s][tid]);
-        row[0] = make_uint4(h[0], h[1], h[2], h[3]), row[1] = make_uint4(h[4], h[5], h[6], h[7]);
-        if (s < nb) {
-          float4* o = reinterpret_cast<float4*>(a1g + (long long)(b0 + s) * kA1 + tid * 16);
-#pragma unroll
-          for (int c = 0; c < 4; c++) o[c] = make_float4(acc[4 * c], acc[4 * c + 1], acc[4 * c + 2], acc[4 * c + 3]);
+        for (int h = 0; h < 2; h++) {
+          const int x = g + 8 * h;
+          a[h] = pack2(S.x[s][y + k0 / 3][x + k0 % 3], S.x[s][y + k1 / 3][x + k1 % 3]);
+          a[2 + h] = t == 0 ? pack2(S.x[s][y + 2][x + 2], 0.f) : 0u;
         }
+        float acc[2][4] = {};
+        mma16816(acc[0], a, w[0], w[1]);
+        mma16816(acc[1], a, w[2], w[3]);
+#pragma unroll
+        for (int j = 0; j < 2; j++)
+#pragma unroll
+          for (int h = 0; h < 2; h++) {
+            const int r = y * 16 + g + 8 * h, n = j * 8 + 2 * t;
+            const float v0 = fmaxf(acc[j][2 * h] + S.b1[n], 0.f), v1 = fmaxf(acc[j][2 * h + 1] + S.b1[n + 1], 0.f);
+            *reinterpret_cast<uint32_t*>(&S.a1[s][r][n]) = pack2(v0, v1);
+            if (s < nb) *reinterpret_cast<float2*>(a1g + (long long)(b0 + s) * kA1 + r * 16 + n) = make_float2(v0, v1);
+          }
       }
     }
     __syncthreads();
-    const int s = warp >> 2, q = warp & 3;  // the warp's sample, and its quarter of the work
     {  // 3x3 stride 2, 16 -> 32: 16 output positions a warp
       float acc[4][4] = {};
       const int pos = q * 16 + (lane & 15), kc = (lane >> 4) * 8;
@@ -242,7 +243,9 @@ __global__ void __launch_bounds__(kNnThreads) k_dense_forward(const float* __res
     *reinterpret_cast<uint2*>(&S.h0[r][k]) = make_uint2(pack2(v.x, v.y), pack2(v.z, v.w));
   }
   for (int i = tid; i < 24 * 64; i += kNnThreads) S.w5[i >> 6][i & 63] = __float2bfloat16_rn(P[kW5 + i]);
-  float acc[2][4] = {};
+  // sums of 80 inputs, added up in FP32 (the tensor cores' accumulators round towards zero), the first and
+  // the bias last
+  float acc[2][4] = {}, first[2][4], sum[2][4] = {};
   for (int k0 = 0; k0 < 640; k0 += kKc) {
     __syncthreads();
 #pragma unroll 16
@@ -258,6 +261,16 @@ __global__ void __launch_bounds__(kNnThreads) k_dense_forward(const float* __res
       ldsm4<false>(w, &S.w4[np * 16 + (lane & 7) + (lane >> 4) * 8][k + ((lane >> 3) & 1) * 8]);
       mma16816(acc[0], a, w[0], w[1]);
       mma16816(acc[1], a, w[2], w[3]);
+      if ((k0 + k + 16) % 80 == 0) {
+#pragma unroll
+        for (int j = 0; j < 2; j++)
+#pragma unroll
+          for (int q = 0; q < 4; q++) {
+            if (k0 + k < 80) first[j][q] = acc[j][q] + P[kB4 + np * 16 + j * 8 + 2 * t + (q & 1)];
+            else sum[j][q] += acc[j][q];
+            acc[j][q] = 0.f;
+          }
+      }
     }
   }
 #pragma unroll
@@ -265,7 +278,7 @@ __global__ void __launch_bounds__(kNnThreads) k_dense_forward(const float* __res
 #pragma unroll
     for (int h = 0; h < 2; h++) {
       const int r = mt * 16 + g + 8 * h, n = np * 16 + j * 8 + 2 * t;
-      const float v0 = fmaxf(acc[j][2 * h] + P[kB4 + n], 0.f), v1 = fmaxf(acc[j][2 * h + 1] + P[kB4 + n + 1], 0.f);
+      const float v0 = fmaxf(sum[j][2 * h] + first[j][2 * h], 0.f), v1 = fmaxf(sum[j][2 * h + 1] + first[j][2 * h + 1], 0.f);
       *reinterpret_cast<uint32_t*>(&S.a4[r][n]) = pack2(v0, v1);
       if (b0 + r < batch) *reinterpret_cast<float2*>(a4g + (long long)(b0 + r) * kA4 + n) = make_float2(v0, v1);
     }
@@ -483,12 +496,15 @@ __global__ void __launch_bounds__(kNnThreads, 2) k_conv_backward(const float* __
             const bf16* row = S.dz3[oy < 4 && ox < 4 ? oy * 4 + ox : 16];
             const bf16* wp = S.w3 + (lane & 15) * kSw3 + (ky * 3 + kx) * 32 + nt * 8;
             uint32_t a[4], w[2];
+            float tap[4] = {};
             ldsm4<false>(a, row + (lane >> 4) * 8);
             ldsm2<true>(w, wp);
-            mma16816(acc, a, w[0], w[1]);
+            mma16816(tap, a, w[0], w[1]);
             ldsm4<false>(a, row + 16 + (lane >> 4) * 8);
             ldsm2<true>(w, wp + 16 * kSw3);
-            mma16816(acc, a, w[0], w[1]);
+            mma16816(tap, a, w[0], w[1]);
+#pragma unroll
+            for (int e = 0; e < 4; e++) acc[e] += tap[e];  // (the taps' sum in FP32)
           }
 #pragma unroll
         for (int h = 0; h < 2; h++) {
@@ -528,13 +544,16 @@ __global__ void __launch_bounds__(kNnThreads, 2) k_conv_backward(const float* __
             const bf16* row = S.dz2[oy < 8 && ox < 8 ? oy * 8 + ox : 64];
             const bf16* wp = S.w2 + (lane & 15) * kSw2 + (ky * 3 + kx) * 16 + (lane >> 4) * 8;
             uint32_t a[4], w[4];
+            float tap[2][4] = {};
 #pragma unroll
             for (int k = 0; k < 32; k += 16) {
               ldsm4<false>(a, row + k + (lane >> 4) * 8);
               ldsm4<true>(w, wp + k * kSw2);
-              mma16816(acc[0], a, w[0], w[1]);
-              mma16816(acc[1], a, w[2], w[3]);
+              mma16816(tap[0], a, w[0], w[1]);
+              mma16816(tap[1], a, w[2], w[3]);
             }
+#pragma unroll
+            for (int e = 0; e < 8; e++) acc[e >> 2][e & 3] += tap[e >> 2][e & 3];  // (the taps' sum in FP32)
           }
 #pragma unroll
         for (int j = 0; j < 2; j++)

@@ -14,8 +14,6 @@
 namespace celv2cu {
 
 constexpr int kItems = 3072;       // every block's tiles
-constexpr int kIntraFirst = 768;   // first item of a block below 64x64
-constexpr int kIntraItems = kItems - kIntraFirst;
 
 // Item i's block b, the block's place (x, y) in the superblock and the tile's (c0, r0) in the block, in
 // samples, and log2 of the block's tiles: class c covers the squares of level c / 2, whole (even c) or
