@@ -733,6 +733,9 @@ struct celv2_engine {
   struct Plan {
     std::vector<Slice> slices;
     std::vector<Wave> waves;
+    // several slices and no references in the whole batch: intra is all the work there is before the
+    // records, and runs slice by slice too. Else it comes before the slices (enqueue_front).
+    bool intra_in_slices = false;
   };
 
   // Rows of superblocks in decision order, cut into at most `most` slices for the records' way to the
@@ -797,6 +800,7 @@ struct celv2_engine {
         p.slices.push_back(std::move(s));
       p.waves.push_back(Wave{j0, split, s0, (int)p.slices.size()});
     }
+    p.intra_in_slices = p.slices.size() > 1 && units == 0;
     return p;
   }
 
@@ -897,14 +901,13 @@ struct celv2_engine {
 
   // Everything of wave i up to its slices: motion search, refinement, and intra (unless it runs on
   // another stream, which records intra_done) where the slices do not run it; of a batch in one slice
-  // also its inter stage and finalize. A batch without references has its intra in the slices: it is
-  // all the work there is before the records.
+  // also its inter stage and finalize.
   int enqueue_front(const std::vector<FrameJob>& jobs, cudaEvent_t intra_done, const std::vector<NetJob>& nets,
                     const Plan& p, int i) {
     const Wave& v = p.waves[i];
     int launched = enqueue_search(jobs, v, i, st, nets);
     const bool whole = p.slices.size() == 1;
-    if (!intra_done && (whole || any_refs(jobs))) {
+    if (!intra_done && !p.intra_in_slices) {
       Slice all;
       for (int j = v.j0; j < v.j1; j++) all.parts.push_back(SbRange{j, 0, jobs[j].sb_cols * jobs[j].sb_rows});
       launched += enqueue_intra(jobs, all, kQueueSlice + 4 * v.s0, st);
@@ -915,11 +918,6 @@ struct celv2_engine {
       launched += enqueue_finalize(jobs, p.slices[0], 0, st);
     }
     return launched;
-  }
-  static bool any_refs(const std::vector<FrameJob>& jobs) {
-    for (const FrameJob& j : jobs)
-      if (j.nrefs > 0) return true;
-    return false;
   }
 
   // What batches in several slices need, made with the first of them.
@@ -950,7 +948,7 @@ struct celv2_engine {
       make_fin_stream();
       if (intra_done) CK(cudaStreamWaitEvent(fin_st, intra_done, 0));
     }
-    const bool intra_here = !intra_done && !any_refs(jobs);
+    const bool intra_here = !intra_done && p.intra_in_slices;
     for (int w = 0; w < (int)p.waves.size(); w++) {
       const Wave& v = p.waves[w];
       before(v);
@@ -1068,6 +1066,7 @@ struct celv2_engine {
       if ((int)slices.size() > kMaxSlices) slices.assign(1, Slice{});
       if (slices.size() == 1) slices[0].parts.assign(1, SbRange{0, 0, g.nsb}), slices[0].sbs = g.nsb;
       p.waves.assign(1, Wave{0, 1, 0, (int)slices.size()});
+      p.intra_in_slices = slices.size() > 1 && nrefs == 0;
       size_t next = 0;  // the next row of `order` to copy
       run(jobs, prepared ? prep_done : nullptr, nets, p, false, [](const Wave&) {}, [&](int i, cudaStream_t ready) {
         // one slice: the copies follow on st; several: on copy_st, beside the next slices' stages
@@ -1334,7 +1333,7 @@ struct celv2_engine {
   // through the pinned ring (stream order puts it after the previous batch's kernels), so a replay
   // never waits on the host for an earlier replay of the same graph.
   struct Graph {
-    std::vector<int> key;  // each job's reference count
+    std::vector<int> key;  // the shape (launch_graph)
     cudaGraphExec_t exec = nullptr;
     int kernels = 0;
   };
@@ -1349,11 +1348,13 @@ struct celv2_engine {
 
   // Wave i of a batch up to its slices (enqueue_front), replayed; returns its kernels.
   int launch_graph(const std::vector<FrameJob>& jobs, const std::vector<NetJob>& nets, const Plan& p, int i) {
-    // the shape: whether its superblock stages are in the graph or follow in slices; the wave, its
-    // first job and its first slice (its queues); per job of it its reference count, whether it has keep words (which decides whether the region pass of the inter
-    // stage is launched at all), features and the network
+    // the shape, which says all that enqueue_front goes by: whether the superblock stages are in the graph
+    // or follow in slices, and whether intra does (that hangs on every job of the batch, not the wave's
+    // alone); the wave, its first job and its first slice (its queues); per job of it its reference count,
+    // whether it has keep words (which decides whether the region pass of the inter stage is launched at
+    // all), features and the network
     const Wave& v = p.waves[i];
-    std::vector<int> key{p.slices.size() == 1, i, v.j0, v.s0};
+    std::vector<int> key{p.slices.size() == 1, p.intra_in_slices, i, v.j0, v.s0};
     for (int j = v.j0; j < v.j1; j++)
       key.push_back(jobs[j].nrefs * 8 + (jobs[j].keep ? 4 : 0) + (nets[j].feats ? 2 : 0) + (nets[j].net ? 1 : 0));
     Graph* gr = nullptr;
