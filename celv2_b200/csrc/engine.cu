@@ -1089,6 +1089,8 @@ struct celv2_engine {
           next += n;
         }
       });
+      // st stands behind the launch as a whole, its records' copies among it (one slice's are on it anyway)
+      if (slices.size() > 1) CK(cudaStreamWaitEvent(st, row_done[order.back()], 0));
       mark_used(used, nrefs, st);
       last_nrefs = nrefs;
       last_out = dest;

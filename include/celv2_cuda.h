@@ -208,7 +208,8 @@ int celv2_get_config(const celv2_engine* e, int key, int* value);
 
 /* ---- Measurement ---- */
 
-/* The engine's main stream (a cudaStream_t), for timing events around its work. */
+/* The engine's main stream (a cudaStream_t), for timing events around its work: all of a celv2_launch,
+ * its records' copies to the host among it; of a batch the stages (its copies run beside it). */
 int celv2_stream(const celv2_engine* e, void** stream);
 /* Stage timing: when enabled, every stage launch is bracketed by CUDA events on its stream.
  * celv2_stage_times returns (and resets) the summed milliseconds and launch counts per stage, in
