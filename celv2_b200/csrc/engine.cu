@@ -271,6 +271,7 @@ struct celv2_engine {
   int row_streams = 1;
   bool pending = false;
   int last_nrefs = 0;
+  int fail_slice = -1;  // celv2_debug_fail: run() fails before it queues this slice
   FrameJob* djobs = nullptr;     // 2 * kMaxJobs + 1 device descriptors (the last: prepare's)
   // Descriptors go to the device from a ring of pinned buffers: an asynchronous copy from pageable
   // memory may wait for the stream, which would serialise back-to-back launches.
@@ -949,8 +950,14 @@ struct celv2_engine {
       if (intra_done) CK(cudaStreamWaitEvent(fin_st, intra_done, 0));
     }
     const bool intra_here = !intra_done && p.intra_in_slices;
+    auto injected = [&](int i) {
+      if (i != fail_slice) return;
+      fail_slice = -1;
+      throw Error(CELV2_ESTATE, "a failure asked for by celv2_debug_fail");
+    };
     for (int w = 0; w < (int)p.waves.size(); w++) {
       const Wave& v = p.waves[w];
+      if (n == 1) injected(0);
       before(v);
       kernel_launches += graph ? launch_graph(jobs, nets, p, w)  // (never with intra on another stream)
                                : enqueue_front(jobs, intra_done, nets, p, w);
@@ -962,6 +969,7 @@ struct celv2_engine {
       CK(cudaStreamWaitEvent(side_st, front_done, 0));
       for (int i = v.s0; i < v.s1; i++) {
         cudaStream_t s = i & 1 ? side_st : st;
+        injected(i);
         if (intra_here) kernel_launches += enqueue_intra(jobs, p.slices[i], kQueueSlice + 4 * i, s);
         kernel_launches += enqueue_inter(jobs, p.slices[i], i, s);
         CK(cudaEventRecord(slice_ready[i], s));
@@ -972,6 +980,17 @@ struct celv2_engine {
       }
     }
     CK(cudaStreamWaitEvent(st, slice_done[n - 1], 0));
+  }
+
+  // After a batch that failed on its way to the GPU: what it had queued ends on every stream (a part of it on
+  // one would not be behind the rest in `st`, and the next batch takes its descriptors, queues and buffers),
+  // and nothing that it was to make counts as made.
+  void settle() {
+    for (cudaStream_t s : {up_st, prep_st, st, side_st, fin_st, copy_st})
+      if (s) cudaStreamSynchronize(s);
+    for (Stage& x : stages) x.taken = false;
+    for (Slot* s : store) s->phases = false;
+    pending = false;
   }
 
   void wait_idle() {
@@ -1097,12 +1116,7 @@ struct celv2_engine {
       pending = true;
     } catch (...) {
       for (const auto& f : fresh_refs) f.first->key = -1;  // their planes were not made
-      cudaStreamSynchronize(st);  // a failure leaves no work running
-      if (side_st) cudaStreamSynchronize(side_st);
-      if (fin_st) cudaStreamSynchronize(fin_st);
-      cudaStreamSynchronize(copy_st);
-      cudaStreamSynchronize(prep_st);
-      pending = false;
+      settle();  // a failure leaves no work running
       throw;
     }
   }
@@ -1282,35 +1296,42 @@ struct celv2_engine {
       for (int r = 0; r < nrefs[j]; r++) reads.push_back(refs[r]);
       fill_job(jobs[j], cur->pyr, refs, nrefs[j], group[j], group[j].intra, lams[j]);
     }
-    std::vector<NetJob> nets(njobs);
-    for (int j = 0; j < njobs; j++) {
-      jobs[j].keep = put_keep(keeps[j], group[j], st);
-      nets[j] = net_for(jobs[j], group[j], !keeps[j].empty());
-      if (nets[j].net) jobs[j].keep = group[j].keep;
-    }
-    const int par = take_parity(st);
-    for (int j = 0; j < njobs; j++) jobs[j].out = group[j].records(par);
-    for (int j = 0; j < njobs; j++)
-      group_out[j] = !to_host ? nullptr : dests[j] ? dests[j] : group_host + (size_t)j * g.nsb;
-    const Plan p = plan(jobs, to_host);
-    // a wave waits for the uploads of its own frames only
-    auto before = [&](const Wave& v) {
-      for (int j = v.j0; j < v.j1; j++) {
-        Slot* const* f = reads.data() + first[j];
-        for (int r = 0; r <= nrefs[j]; r++) wait_ready(*f[r], st);
-        make_phases(f + 1, nrefs[j], st);
+    celv2_sb_out* out[kMaxJobs] = {};  // where each job's records go
+    try {
+      std::vector<NetJob> nets(njobs);
+      for (int j = 0; j < njobs; j++) {
+        jobs[j].keep = put_keep(keeps[j], group[j], st);
+        nets[j] = net_for(jobs[j], group[j], !keeps[j].empty());
+        if (nets[j].net) jobs[j].keep = group[j].keep;
       }
-    };
-    put_batch(jobs);
-    run(jobs, nullptr, nets, p, use_graphs && !timing, before, [&](int i, cudaStream_t ready) {
-      if (!to_host) return;  // records left on the device
-      copy_slice(p.slices[i], i, ready, [&](int j) { return std::make_pair(jobs[j].out, group_out[j]); });
-    });
-    mark_used(reads.data(), (int)reads.size(), st);
-    if (to_host) {
-      CK(cudaEventRecord(copied[par], copy_st));
-      copy_pending[par] = true;
+      const int par = take_parity(st);
+      for (int j = 0; j < njobs; j++) jobs[j].out = group[j].records(par);
+      for (int j = 0; j < njobs; j++)
+        out[j] = !to_host ? nullptr : dests[j] ? dests[j] : group_host + (size_t)j * g.nsb;
+      const Plan p = plan(jobs, to_host);
+      // a wave waits for the uploads of its own frames only
+      auto before = [&](const Wave& v) {
+        for (int j = v.j0; j < v.j1; j++) {
+          Slot* const* f = reads.data() + first[j];
+          for (int r = 0; r <= nrefs[j]; r++) wait_ready(*f[r], st);
+          make_phases(f + 1, nrefs[j], st);
+        }
+      };
+      put_batch(jobs);
+      run(jobs, nullptr, nets, p, use_graphs && !timing, before, [&](int i, cudaStream_t ready) {
+        if (!to_host) return;  // records left on the device
+        copy_slice(p.slices[i], i, ready, [&](int j) { return std::make_pair(jobs[j].out, out[j]); });
+      });
+      mark_used(reads.data(), (int)reads.size(), st);
+      if (to_host) {
+        CK(cudaEventRecord(copied[par], copy_st));
+        copy_pending[par] = true;
+      }
+    } catch (...) {
+      settle();  // the records of the group before stay readable
+      throw;
     }
+    std::copy(out, out + njobs, group_out);
     group_jobs = njobs;
     ++launches;
     launches_group = launches;
@@ -1430,6 +1451,8 @@ void launch_multi(int njobs, celv2_engine* const* engines, const long long* src_
     for (int j = 0; j < njobs; j++) count += engines[j] == e;
     if (count > e->group_cap) e->reserve_group(std::max(count, 8));
   }
+  std::vector<int> next(uniq.size(), 0);  // each engine's jobs
+  try {
   // the other engines' queued work first: the lead stream waits for each of their streams
   for (celv2_engine* e : uniq)
     if (e != lead) {
@@ -1450,7 +1473,6 @@ void launch_multi(int njobs, celv2_engine* const* engines, const long long* src_
   std::vector<int> par;  // each engine's device record buffer set for this batch
   for (celv2_engine* e : uniq) par.push_back(e->take_parity(lead->st));
   std::vector<Entry> entries;
-  std::vector<int> next(uniq.size(), 0);
   std::vector<std::vector<Slot*>> reads(uniq.size());  // each engine's store slots this batch reads
   for (int j = 0; j < njobs; j++) {
     celv2_engine* e = engines[j];
@@ -1482,7 +1504,6 @@ void launch_multi(int njobs, celv2_engine* const* engines, const long long* src_
   for (Entry& en : entries) {
     if (!to_host) en.dest = nullptr;  // records left on the device
     else if (!en.dest) en.dest = en.e->group_host + (size_t)en.slot * en.e->g.nsb;
-    en.e->group_out[en.slot] = en.dest;
   }
   // the records on the lead's copy stream, overlapping later work
   const celv2_engine::Plan p = celv2_engine::plan(jobs, to_host);
@@ -1503,15 +1524,21 @@ void launch_multi(int njobs, celv2_engine* const* engines, const long long* src_
   cudaEvent_t done;
   CK(cudaEventCreateWithFlags(&done, cudaEventDisableTiming));
   CK(cudaEventRecord(done, lead->st));
+  for (celv2_engine* e : uniq)
+    if (e != lead) CK(cudaStreamWaitEvent(e->st, done, 0));
+  cudaEventDestroy(done);
+  for (const Entry& en : entries) en.e->group_out[en.slot] = en.dest;
+  } catch (...) {
+    for (celv2_engine* e : uniq) e->settle();  // (the lead first: the others' streams may wait for its)
+    throw;
+  }
   for (size_t i = 0; i < uniq.size(); i++) {
     celv2_engine* e = uniq[i];
-    if (e != lead) CK(cudaStreamWaitEvent(e->st, done, 0));
     e->group_jobs = next[i];
     ++e->launches;
     e->launches_group = e->launches;
     e->pending = true;
   }
-  cudaEventDestroy(done);
 }
 
 }  // namespace
@@ -1785,6 +1812,13 @@ int celv2_debug_inter(celv2_engine* e, int32_t* out) {
     CK(cudaSetDevice(e->device));
     e->wait_idle();
     CK(cudaMemcpy(out, e->single.inter, (size_t)e->g.nsb * kMaxRefs * kBlocks * sizeof(int2), cudaMemcpyDeviceToHost));
+  });
+}
+
+int celv2_debug_fail(celv2_engine* e, int slice) {
+  return guarded([&] {
+    if (!e || slice < 0) invalid("debug_fail: an engine and a slice");
+    e->fail_slice = slice;
   });
 }
 

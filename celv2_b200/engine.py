@@ -61,6 +61,7 @@ SIGNATURES = {
                                     C.POINTER(C.c_int)]),
     "celv2_debug_intra": (C.c_int, [C.c_void_p, C.POINTER(C.c_int32)]),
     "celv2_debug_inter": (C.c_int, [C.c_void_p, C.POINTER(C.c_int32)]),
+    "celv2_debug_fail": (C.c_int, [C.c_void_p, C.c_int]),
     "celv2_kernel_launches": (C.c_longlong, [C.c_void_p]),
     "celv2_stream": (C.c_int, [C.c_void_p, C.POINTER(C.c_void_p)]),
     "celv2_stage_timing": (C.c_int, [C.c_void_p, C.c_int]),
@@ -551,6 +552,10 @@ class CudaEngine:
         return {STAGE_NAMES[i]: (ms[i], cnt[i]) for i in range(n)}
 
     # ---- inspection ----
+    def debug_fail(self, slice_: int) -> None:
+        """celv2_debug_fail: the next launch fails before it queues this slice."""
+        _check(library().celv2_debug_fail(self._h, slice_))
+
     def debug_field(self, r: int, level: int) -> np.ndarray:
         pw, ph = (self.width + 7) & ~7, (self.height + 7) & ~7
         w, h = pw, ph

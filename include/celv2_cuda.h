@@ -174,6 +174,9 @@ int celv2_debug_field(celv2_engine* e, int r, int level, int32_t* out, int* cols
 int celv2_debug_intra(celv2_engine* e, int32_t* out);
 /* The last launch's per-reference bests: sb_cols * sb_rows * 7 * 425 (SATD, packed MV) pairs. */
 int celv2_debug_inter(celv2_engine* e, int32_t* out);
+/* A failure on the host, once: the next launch that comes so far (celv2_launch_multi: led by this engine) fails
+ * with CELV2_ESTATE before it queues that slice of its superblocks. */
+int celv2_debug_fail(celv2_engine* e, int slice);
 /* Kernel launches the engine has issued so far (all stages). */
 long long celv2_kernel_launches(const celv2_engine* e);
 
