@@ -21,6 +21,7 @@
 
 #include <algorithm>
 #include <array>
+#include <atomic>
 #include <cstdio>
 #include <cstring>
 #include <mutex>
@@ -320,7 +321,10 @@ struct celv2_engine {
   static constexpr int kQueuePrep = 0, kQueueMe = 1, kQueueSlice = kQueueMe + kMaxWaves * (kLevels + 1);
   static constexpr int kQueues = kQueueSlice + 4 * kMaxSlices;
   unsigned* queues = nullptr;
-  int* fault = nullptr;  // behind the ring, page-locked: set by a kernel whose wait for its copies ran out
+  // behind the ring, page-locked: set by a kernel whose wait for its copies ran out. Every call that hands
+  // records out fails from then on, up to the next batch (fault_told: one of them has, maybe on another thread)
+  int* fault = nullptr;
+  std::atomic<bool> fault_told{false};
   bool persistent = true;      // the queue-draining persistent stage kernels (else one CTA per unit)
   unsigned persistent_off = 0; // stages (bit i: queue i) that run one CTA per unit anyway
   int me_cells[kLevels] = {30, 30, 30, 30, 30};
@@ -993,7 +997,7 @@ struct celv2_engine {
     pending = false;
   }
 
-  void wait_idle() {
+  void drain() {
     CK(cudaStreamSynchronize(up_st));
     CK(cudaStreamSynchronize(st));
     CK(cudaStreamSynchronize(copy_st));
@@ -1002,10 +1006,25 @@ struct celv2_engine {
       CK(cudaStreamSynchronize(prep_st));
       harvest();
     }
-    if (*static_cast<volatile int*>(fault)) {
-      *fault = 0;
-      throw Error(CELV2_ECUDA, "a kernel's wait for its copies ran out: the last batch is not decided");
-    }
+  }
+
+  void check_fault() {
+    if (!*static_cast<volatile int*>(fault)) return;
+    fault_told = true;
+    throw Error(CELV2_ECUDA, "a kernel's wait for its copies ran out: the last batch is not decided");
+  }
+  // A new batch: a fault that the caller has been told of is over with the batches that it may belong to.
+  void clear_fault() {
+    if (!fault_told) return;
+    drain();
+    *fault = 0;
+    fault_told = false;
+  }
+
+  // Before records, or what else a batch left, are read.
+  void wait_idle() {
+    drain();
+    check_fault();
   }
 
   void launch(const celv2_frame* src, const celv2_frame* refs, int nrefs, long long lam, const long long* keys,
@@ -1017,6 +1036,7 @@ struct celv2_engine {
     if (nrefs < 0 || nrefs > kMaxRefs) invalid("CudaEngine: too many references");
     for (int r = 0; r < nrefs; r++) check_frame(&refs[r], "reference");
     if (nrefs > 0 && (g.pw < 16 || g.ph < 16)) invalid("CudaEngine: inter frames need at least 9x9 pixels");
+    clear_fault();
     if (pending) wait_idle();
     recover_stages();
     std::vector<std::pair<Slot*, int>> fresh_refs;  // references not in the cache yet, until they are on their way
@@ -1163,6 +1183,7 @@ struct celv2_engine {
     if (row < 0 || row >= g.sb_rows) invalid("row out of range");
     if (!pending && launches == 0) throw Error(CELV2_ESTATE, "no launch to collect");
     CK(cudaEventSynchronize(row_done[row]));
+    check_fault();
     return last_out + (size_t)row * g.sb_cols;
   }
 
@@ -1188,7 +1209,7 @@ struct celv2_engine {
   // ---- group path ----
   void reserve_group(int frames) {
     if (frames <= group_cap) return;
-    wait_idle();
+    drain();
     free_graphs();  // they hold the old buffers' addresses
     group_jobs = 0;  // the last group's records go with the old host buffer
     for (JobBuffers& b : group) free_buffers(b);
@@ -1276,6 +1297,7 @@ struct celv2_engine {
     if (!to_host)
       for (int j = 0; j < njobs; j++)
         if (dests[j]) invalid("group: set_output names host memory, but to_host 0 leaves the records on the device");
+    clear_fault();
     if (njobs > group_cap) reserve_group(std::max(njobs, 8));
     std::vector<FrameJob> jobs(njobs);
     std::vector<Slot*> reads;  // per job its source and its references, from first[job]
@@ -1447,6 +1469,7 @@ void launch_multi(int njobs, celv2_engine* const* engines, const long long* src_
     }
   }
   for (celv2_engine* e : uniq) {
+    e->clear_fault();
     int count = 0;
     for (int j = 0; j < njobs; j++) count += engines[j] == e;
     if (count > e->group_cap) e->reserve_group(std::max(count, 8));
@@ -1763,7 +1786,7 @@ int celv2_clear_store(celv2_engine* e) {
   return guarded([&] {
     if (!e) invalid("null engine");
     CK(cudaSetDevice(e->device));
-    e->wait_idle();
+    e->drain();
     for (Slot* s : e->store) celv2_engine::free_slot(s);
     e->store.clear();
   });
@@ -1817,8 +1840,9 @@ int celv2_debug_inter(celv2_engine* e, int32_t* out) {
 
 int celv2_debug_fail(celv2_engine* e, int slice) {
   return guarded([&] {
-    if (!e || slice < 0) invalid("debug_fail: an engine and a slice");
-    e->fail_slice = slice;
+    if (!e || slice < -1) invalid("debug_fail: an engine and a slice, or -1");
+    if (slice < 0) *static_cast<volatile int*>(e->fault) = 1;
+    else e->fail_slice = slice;
   });
 }
 
@@ -1833,7 +1857,7 @@ int celv2_set_pruner(celv2_engine* e, const float* params, float ref_threshold, 
                     band >= 0.f))
       invalid("set_pruner: thresholds must lie in [0, 1] and the band be >= 0");
     CK(cudaSetDevice(e->device));
-    e->wait_idle();
+    e->drain();
     e->free_graphs();  // captured batches hold the old settings
     if (!params) {
       cudaFree(e->pruner_params), cudaFree(e->nn_wb);
@@ -1886,7 +1910,7 @@ int celv2_set_config(celv2_engine* e, int key, int value) {
   return guarded([&] {
     if (!e) invalid("null engine");
     CK(cudaSetDevice(e->device));
-    e->wait_idle();
+    e->drain();
     switch (key) {
       case CELV2_CFG_PERSISTENT: e->persistent = value != 0, e->free_graphs(); break;
       case CELV2_CFG_GRAPHS: e->use_graphs = value != 0; break;
@@ -1939,7 +1963,7 @@ int celv2_stage_timing(celv2_engine* e, int enable) {
   return guarded([&] {
     if (!e) invalid("null engine");
     CK(cudaSetDevice(e->device));
-    e->wait_idle();
+    e->drain();
     e->timing = enable != 0;
     if (e->timing && !e->stats) {
       CK(cudaMalloc(&e->stats, kStats * sizeof(unsigned long long)));
@@ -1952,7 +1976,7 @@ int celv2_work_counters(celv2_engine* e, unsigned long long* out, int n) {
   return guarded([&] {
     if (!e || !out) invalid("null argument");
     CK(cudaSetDevice(e->device));
-    e->wait_idle();
+    e->drain();
     CK(cudaStreamSynchronize(e->prep_st));
     unsigned long long v[kStats] = {};
     if (e->stats) {
@@ -1967,7 +1991,7 @@ int celv2_stage_times(celv2_engine* e, double* ms, long long* launches, int n) {
   return guarded([&] {
     if (!e || !ms || !launches) invalid("null argument");
     CK(cudaSetDevice(e->device));
-    e->wait_idle();
+    e->drain();
     CK(cudaStreamSynchronize(e->prep_st));
     e->harvest();
     for (int i = 0; i < n && i < kStages; i++) ms[i] = e->stage_ms[i], launches[i] = e->stage_n[i];

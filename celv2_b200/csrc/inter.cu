@@ -269,6 +269,12 @@ __device__ __forceinline__ void tma_box(unsigned dst, const void* map, int x, in
       : "memory");
 }
 
+// A wait that ran out: none of the launch's jobs counts as decided (with its CTAs gone, units of any of them may
+// be left that no CTA takes).
+__device__ __forceinline__ void mark_fault(const FrameJob* jobs, const WorkList& w) {
+  for (int p = 0; p < w.nparts; p++) *jobs[w.part[p].job].fault = 1;
+}
+
 // G groups of 256 threads, 2G halves: half h takes MV h of a step's 2G. pass: MVs whose sums shared
 // memory holds, a multiple of 2G.
 template <int G>
@@ -363,7 +369,7 @@ __global__ void __launch_bounds__(kInterThreads* G, 4 / G) k_inter(const FrameJo
     if (s >= steps) return;
     const unsigned bar = full_s + 8 * to;
     if (!mbar_wait(empty_s + 8 * to, round ^ 1)) {
-      *job.fault = 1;
+      mark_fault(jobs, w);
       return;
     }
     int2 e[M];
@@ -507,7 +513,7 @@ __global__ void __launch_bounds__(kInterThreads* G, 4 / G) k_inter(const FrameJo
     __syncthreads();  // the next pass overwrites the sums
   }
   if (!ok) {  // a wait ran out: the batch is marked, this CTA's steps still in flight are given their time
-    if (tid == 0) *job.fault = 1;
+    if (tid == 0) mark_fault(jobs, w);
     for (int k = s + 1; k < min(s + 3, steps); k++) mbar_wait(full_s + 8 * (k % kRing), parity >> (k % kRing) & 1);
     return;
   }

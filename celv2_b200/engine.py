@@ -553,7 +553,8 @@ class CudaEngine:
 
     # ---- inspection ----
     def debug_fail(self, slice_: int) -> None:
-        """celv2_debug_fail: the next launch fails before it queues this slice."""
+        """celv2_debug_fail: the next launch fails before it queues this slice (-1: the batch in flight reads
+        as undecided)."""
         _check(library().celv2_debug_fail(self._h, slice_))
 
     def debug_field(self, r: int, level: int) -> np.ndarray:

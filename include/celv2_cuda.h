@@ -80,7 +80,9 @@ int celv2_row_order(const celv2_engine* e, int* rows);
  * next launch). */
 int celv2_wait_row(celv2_engine* e, int row, const celv2_sb_out** records);
 
-/* Returns with no work of the last launch pending (collect's end). */
+/* Returns with no work of the last launch pending (collect's end). The inter stage's waits for its copies are
+ * bounded; when one runs out, the batches in flight are not decided, and this, celv2_wait_row and every other call
+ * that hands out what a batch left return CELV2_ECUDA until the next launch. */
 int celv2_finish(celv2_engine* e);
 
 /* The calling thread's last error message ("" if none). */
@@ -175,7 +177,8 @@ int celv2_debug_intra(celv2_engine* e, int32_t* out);
 /* The last launch's per-reference bests: sb_cols * sb_rows * 7 * 425 (SATD, packed MV) pairs. */
 int celv2_debug_inter(celv2_engine* e, int32_t* out);
 /* A failure on the host, once: the next launch that comes so far (celv2_launch_multi: led by this engine) fails
- * with CELV2_ESTATE before it queues that slice of its superblocks. */
+ * with CELV2_ESTATE before it queues that slice of its superblocks. Slice -1: the batch in flight reads as one
+ * of whose kernels a wait ran out (celv2_finish). */
 int celv2_debug_fail(celv2_engine* e, int slice);
 /* Kernel launches the engine has issued so far (all stages). */
 long long celv2_kernel_launches(const celv2_engine* e);
