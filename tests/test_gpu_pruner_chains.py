@@ -52,3 +52,19 @@ def test_weight_gradient_chains_are_bounded():
             err = ((g - w).norm() / w.norm()).item()
             print(name, err)
             assert err < 1e-5, (name, err)
+
+
+def test_bias_gradients_meet_in_few_additions():
+    """The last layer's biases: FP32 sums of 131,072 positive numbers, in FP64 the sum of them. At most 64 CTAs' four
+    row groups are added in a row to the same number: a random walk of 256 round-to-nearest errors (0.29 of an ulp, the
+    ulp at most 2^-23 of the sum so far), 0.29 * 2^-23 * sqrt(256 / 3) = 3.2e-7 of a bias; the threads' own sums before it
+    (512 in a row, 256 of them side by side) add a tenth of that. 6e-7 leaves the walk its spread. (2,048 CTAs' lost
+    1.0e-6.)"""
+    torch.manual_seed(6)
+    params = torch.rand(E.PRUNER_PARAMS, device="cuda") * 0.04 + 0.01
+    x = torch.rand(BATCH, E.PRUNER_FEATURES, device="cuda") + 0.5
+    dl = torch.rand(BATCH, E.PRUNER_OUTPUTS, device="cuda") + 0.5
+    got = gradients(params, x, dl)[-E.PRUNER_OUTPUTS:]
+    want = dl.double().sum(0)
+    torch.cuda.empty_cache()
+    assert ((got - want).norm() / want.norm()).item() < 6e-7
