@@ -471,7 +471,14 @@ struct celv2_engine {
     CK(cudaStreamCreateWithFlags(&copy_st, cudaStreamNonBlocking));
     CK(cudaStreamCreateWithFlags(&up_st, cudaStreamNonBlocking));
     for (cudaEvent_t& e : copied) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-    CK(cudaEventCreateWithFlags(&slice_done[0], cudaEventDisableTiming));
+    // (made here, not with the first batch in slices: a stream is 0.1 to 3 ms)
+    int least = 0, greatest = 0;
+    CK(cudaDeviceGetStreamPriorityRange(&least, &greatest));
+    CK(cudaStreamCreateWithFlags(&side_st, cudaStreamNonBlocking));
+    CK(cudaStreamCreateWithPriority(&fin_st, cudaStreamNonBlocking, greatest));
+    CK(cudaEventCreateWithFlags(&front_done, cudaEventDisableTiming));
+    for (cudaEvent_t& e : slice_ready) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    for (cudaEvent_t& e : slice_done) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     CK(cudaMalloc(&djobs, kRingJobs * sizeof(FrameJob)));
     CK(cudaMalloc(&queues, kQueues * sizeof(unsigned)));
     CK(cudaMallocHost(&ring, (size_t)kRing * kRingJobs * sizeof(FrameJob) + sizeof(int)));
@@ -925,20 +932,6 @@ struct celv2_engine {
     return launched;
   }
 
-  // What batches in several slices need, made with the first of them.
-  void make_fin_stream() {
-    if (fin_st) return;
-    int least = 0, greatest = 0;
-    CK(cudaDeviceGetStreamPriorityRange(&least, &greatest));
-    for (int i = 0; i < kMaxSlices; i++)
-      if (!slice_ready[i]) CK(cudaEventCreateWithFlags(&slice_ready[i], cudaEventDisableTiming));
-    for (int i = 1; i < kMaxSlices; i++)
-      if (!slice_done[i]) CK(cudaEventCreateWithFlags(&slice_done[i], cudaEventDisableTiming));
-    if (!front_done) CK(cudaEventCreateWithFlags(&front_done, cudaEventDisableTiming));
-    if (!side_st) CK(cudaStreamCreateWithFlags(&side_st, cudaStreamNonBlocking));
-    CK(cudaStreamCreateWithPriority(&fin_st, cudaStreamNonBlocking, greatest));
-  }
-
   // The stages of a batch on st, its descriptors and zeroed queues already queued there (put_batch; graph:
   // each wave's part up to its slices replayed as a CUDA graph). before(v) queues on st what wave v's jobs wait for; done(i,
   // stream) is called once slice i's records are queued on `stream` -- to queue their copies. Several slices: their inter stages go to two streams in turn, so
@@ -949,10 +942,7 @@ struct celv2_engine {
   void run(const std::vector<FrameJob>& jobs, cudaEvent_t intra_done, const std::vector<NetJob>& nets,
            const Plan& p, bool graph, B&& before, F&& done) {
     const int n = (int)p.slices.size();
-    if (n > 1) {
-      make_fin_stream();
-      if (intra_done) CK(cudaStreamWaitEvent(fin_st, intra_done, 0));
-    }
+    if (n > 1 && intra_done) CK(cudaStreamWaitEvent(fin_st, intra_done, 0));
     const bool intra_here = !intra_done && p.intra_in_slices;
     auto injected = [&](int i) {
       if (i != fail_slice) return;
