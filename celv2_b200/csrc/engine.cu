@@ -273,10 +273,12 @@ struct celv2_engine {
   bool pending = false;
   int last_nrefs = 0;
   int fail_slice = -1;  // celv2_debug_fail: run() fails before it queues this slice
-  FrameJob* djobs = nullptr;     // 2 * kMaxJobs + 1 device descriptors (the last: prepare's)
+  FrameJob* djobs = nullptr;     // kMaxJobs + 1 device descriptors (the last: prepare's)
   // Descriptors go to the device from a ring of pinned buffers: an asynchronous copy from pageable
   // memory may wait for the stream, which would serialise back-to-back launches.
-  static constexpr int kRing = 8, kRingJobs = 2 * kMaxJobs + 1;
+  // (With room for twice a batch's jobs the ring was 1.5 MB, and the records, planes and so on of a small engine
+  // no longer fitted into the same 2 MB of page-locked memory: its first 202x122 frame took 2.9 ms, now 0.2.)
+  static constexpr int kRing = 8, kRingJobs = kMaxJobs + 1;
   // Store slots an upload may add rather than wait for a dropped slot's readers (a caller that
   // issues far ahead of the GPU would otherwise grow the store without bound).
   static constexpr int kStoreSlotsIdle = 48;
