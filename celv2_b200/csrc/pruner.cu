@@ -5,13 +5,15 @@
 // moves between its layers. The forward pass runs all three convolutions of two samples in one CTA,
 // the backward pass all three of one: the activations' BF16 copies sit in shared memory and a
 // convolution's column matrix exists only as the row addresses ldmatrix is given (a zero row for the
-// padding); weight gradients stay in the CTA's accumulators over all its samples. Operands are rounded
-// to BF16, mma.sync m16n8k16 with FP32 accumulators, bias, ReLU and masks on the FP32 values, which is
-// what the cache between the passes holds. A step on 4,096 samples 2.33 -> 0.28 ms against column
+// padding); weight gradients stay in the CTA's accumulators over up to 32 of its samples. Operands are rounded
+// to BF16, mma.sync m16n8k16 with FP32 accumulators, bias and ReLU on the FP32 values, which is what the
+// cache between the passes holds (the convolutions' backward masks ask its BF16 copies, zero where it is
+// zero or below 2^-134). A step on 4,096 samples 2.33 -> 0.28 ms against column
 // matrices written out and read back for every layer (390 MB) and weight gradients of a few CTAs.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <climits>
 #include <string>
 
 #include "celv2_pruner.h"
@@ -426,12 +428,13 @@ int dense_samples(int batch, int least) {
   return per < least ? least : per > 2048 ? 2048 : per;
 }
 
-// ---- backward: the convolutions, a sample at a time, their weight gradients over up to 32 of a CTA's samples ----
+// ---- backward: the convolutions, a sample at a time, their weight gradients over a CTA's samples ----
 // The tensor cores' accumulators round towards zero, a loss that grows with every product added, so a chain of
-// theirs is at most kChain samples (for W2, with 64 positions each, 2,048 products); the chains meet in FP32 atomics.
-// 65,536 samples' gradients of one sign came out 5.6e-5 (W2) and 2.3e-5 (W1) low with a chain over all of a CTA's
-// samples, 3.0e-6 and 2.0e-6 with these. Up to 32 samples a CTA (9,472 on 148 SMs) it is one chain, as it was; 16,384
-// samples' backward pass takes 482 us instead of 447 (chains of 16: 527, for 1.0e-6 instead of 2.4e-6).
+// theirs is at most kChain samples (for W2, with 64 positions each, 2,048 products). Up to 32 samples a CTA (9,472 on
+// 148 SMs) that is all of them; CHAINS, for more, puts the sums down every 32 and starts anew, and they meet in the FP32
+// atomics: 65,536 samples' gradients of one sign 5.6e-5 (W2) and 2.3e-5 (W1) low with one chain, 3.0e-6 and 2.0e-6
+// with these; 16,384 samples' backward pass 447 -> 507 us. (One kernel for both costs a step on 4,096 samples 2 us of
+// 269; a launch for every 9,472 samples in its place takes 530.)
 constexpr int kChain = 32;
 struct BackSmem {
   bf16 w2[32 * kSw2], w3[32 * kSw3];
@@ -441,6 +444,7 @@ struct BackSmem {
   float bias[16 + 32 + 32];
 };
 
+template <bool CHAINS>
 __global__ void __launch_bounds__(kNnThreads, 2) k_conv_backward(const float* __restrict__ P, const float* __restrict__ xs,
                                                                  const float* __restrict__ a1g, const float* __restrict__ a2g,
                                                                  const float* __restrict__ dz3g, int batch, float* G) {
@@ -457,9 +461,10 @@ __global__ void __launch_bounds__(kNnThreads, 2) k_conv_backward(const float* __
   // this warp's share: weight gradients of 16 output channels (m2) and a run of 8-column tiles
   const int m2 = warp & 1, q = warp >> 1, t2 = q < 2 ? 5 * q : 10 + 4 * (q - 2), n2 = q < 2 ? 5 : 4;
   float s3[2] = {}, s2[2] = {}, s1[4] = {};  // bias sums
-  for (int b = blockIdx.x; b < batch;) {
+  int b = blockIdx.x;
+  do {
   float g3[9][4] = {}, g2[5][4] = {}, g1[2][4] = {};
-  for (int i = 0; i < kChain && b < batch; i++, b += gridDim.x) {
+  for (int i = 0; (!CHAINS || i < kChain) && b < batch; i++, b += gridDim.x) {
     __syncthreads();  // the sample before is done with
     {
       const float4* v = reinterpret_cast<const float4*>(a1g + (long long)b * kA1);
@@ -594,6 +599,7 @@ __global__ void __launch_bounds__(kNnThreads, 2) k_conv_backward(const float* __
       mma16816(g1[1], a, w[2], w[3]);
     }
   }
+  __syncthreads();
   // the chain's sums into the gradient vector
 #pragma unroll
   for (int e = 0; e < 4; e++) {
@@ -607,8 +613,7 @@ __global__ void __launch_bounds__(kNnThreads, 2) k_conv_backward(const float* __
     atomicAdd(G + kW1 + m1 * 9 + c, g1[0][e]);
     if (c == 0) atomicAdd(G + kW1 + m1 * 9 + 8, g1[1][e]);
   }
-  }
-  __syncthreads();  // S.bias starts at zero
+  } while (CHAINS && b < batch);
   atomicAdd(&S.bias[48 + 2 * (tid & 15)], s3[0]), atomicAdd(&S.bias[48 + 2 * (tid & 15) + 1], s3[1]);
   atomicAdd(&S.bias[16 + (warp & 3) * 8 + 2 * t], s2[0]), atomicAdd(&S.bias[16 + (warp & 3) * 8 + 2 * t + 1], s2[1]);
 #pragma unroll
@@ -682,8 +687,13 @@ void backward(const float* P, int batch, const float* acts, const float* dlogits
                                                                                        G + kW4, G + kB4);
   k_dense_weights<<<dim3(1, (batch + p5 - 1) / p5), kNnThreads, 0, st>>>(dlogits, kOut, c.a4, 64, batch, p5, G + kW5,
                                                                           G + kB5);
-  const int grid = resident(k_conv_backward, sizeof(BackSmem), batch);
-  k_conv_backward<<<grid, kNnThreads, sizeof(BackSmem), st>>>(P, c.xs, c.a1, c.a2, dz3, batch, G);
+  const auto conv = [&](auto kernel) {
+    const int grid = resident(kernel, sizeof(BackSmem), batch);
+    kernel<<<grid, kNnThreads, sizeof(BackSmem), st>>>(P, c.xs, c.a1, c.a2, dz3, batch, G);
+  };
+  const int full = resident(k_conv_backward<false>, sizeof(BackSmem), INT_MAX);
+  if (batch <= (long long)full * kChain) conv(k_conv_backward<false>);
+  else conv(k_conv_backward<true>);
 }
 
 }  // namespace nn
