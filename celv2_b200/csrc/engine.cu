@@ -25,6 +25,7 @@
 #include <cstdio>
 #include <cstring>
 #include <mutex>
+#include <new>
 #include <stdexcept>
 #include <string>
 #include <vector>
@@ -70,7 +71,10 @@ int celv2cu::persistent_grid(const void* kernel, int threads, size_t smem, int u
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const int full = (per_sm < 1 ? 1 : per_sm) * sms;
-  g_grid_cache.push_back({GridKey{kernel, dev, threads, smem}, full});
+  try {
+    g_grid_cache.push_back({GridKey{kernel, dev, threads, smem}, full});
+  } catch (const std::bad_alloc&) {  // asked again next time (C entry points call this outside guarded())
+  }
   return units < full ? units : full;
 }
 
@@ -271,7 +275,6 @@ struct celv2_engine {
   std::vector<int> order;
   int row_streams = 1;
   bool pending = false;
-  int last_nrefs = 0;
   int fail_slice = -1;  // celv2_debug_fail: run() fails before it queues this slice
   FrameJob* djobs = nullptr;     // kMaxJobs + 1 device descriptors (the last: prepare's)
   // Descriptors go to the device from a ring of pinned buffers: an asynchronous copy from pageable
@@ -935,9 +938,9 @@ struct celv2_engine {
   }
 
   // The stages of a batch on st, its descriptors and zeroed queues already queued there (put_batch; graph:
-  // each wave's part up to its slices replayed as a CUDA graph). before(v) queues on st what wave v's jobs wait for; done(i,
-  // stream) is called once slice i's records are queued on `stream` -- to queue their copies. Several slices: their inter stages go to two streams in turn, so
-  // one's CTAs take the SMs that the drained launch before it leaves (in one stream eight slices of five
+  // each wave's part up to its slices replayed as a CUDA graph). before(v) queues on st what wave v's jobs
+  // wait for; done(i, stream) is called once slice i's records are queued on `stream` -- to queue their
+  // copies. Several slices: their inter stages go to two streams in turn, so one's CTAs take the SMs that the drained launch before it leaves (in one stream eight slices of five
   // 1080p leaves spent 2.07 ms in the stage that takes 1.60 in one launch), and their finalize to a third
   // of higher priority; st waits for the last finalize.
   template <typename B, typename F>
@@ -1123,7 +1126,6 @@ struct celv2_engine {
       // st stands behind the launch as a whole, its records' copies among it (one slice's are on it anyway)
       if (slices.size() > 1) CK(cudaStreamWaitEvent(st, row_done[order.back()], 0));
       mark_used(used, nrefs, st);
-      last_nrefs = nrefs;
       last_out = dest;
       pending = true;
     } catch (...) {
@@ -1365,7 +1367,8 @@ struct celv2_engine {
     }
   }
 
-  // ---- CUDA graphs: a batch's whole stage sequence captured once per shape, then replayed ----
+  // ---- CUDA graphs: a wave's stages up to its slices (of a batch in one slice: all) captured once per
+  // shape, then replayed ----
   // The descriptors are not part of the graph: each replay is preceded by their copy into djobs
   // through the pinned ring (stream order puts it after the previous batch's kernels), so a replay
   // never waits on the host for an earlier replay of the same graph.

@@ -115,7 +115,7 @@ struct WholeSmem {
   int tab[kTab];                // hash table of the cells' MVs
   unsigned char tidx[kTab];     // per table entry: its MV's index in D
   int D[kNb];                   // distinct MVs
-  int2 win[kNb + 1];            // per MV of D: its window's first row in the phase plane << 4 | phase; the first
+  int2 win[kNb];                // per MV of D: its window's first row in the phase plane << 4 | phase; the first
                                 // byte of its rows (from the row's start, a multiple of 16) | the prediction's
                                 // first byte in them (-1: not all inside the margin, or no MV)
   unsigned char dmap[kNb];      // neighbourhood cell -> its MV's index in D
@@ -357,10 +357,9 @@ __global__ void __launch_bounds__(kInterThreads* G, 4 / G) k_inter(const FrameJo
   __syncthreads();
   if (tid < kNb) S.dmap[tid] = S.tidx[h];
   const int nd = S.nd, steps = (nd + M - 1) / M;
-  if (tid == 0) S.win[nd].y = -1;
   if (tid == 0 && job.stats) atomicAdd(job.stats + kStatInterMvs, (unsigned long long)nd * 256);
 
-  __syncthreads();  // dmap and the end of win complete
+  __syncthreads();  // dmap complete
   // step s's windows into ring slot `to`, by one thread, once every warp is done with the step that had
   // the slot before; round: the parity of the step's own round (a wait that runs out marks the batch and
   // leaves the step without windows, which ends every thread's own wait for them the same way)

@@ -124,7 +124,4 @@ void launch_infer(const NetList& l, cudaStream_t st);
 size_t infer_weight_elems();
 void infer_weights(const float* params, void* wb, cudaStream_t st);
 
-// Set-up of the constant tables (once per device).
-cudaError_t init_tables();
-
 }  // namespace celv2cu

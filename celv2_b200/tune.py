@@ -4,7 +4,8 @@ The decisions never depend on these knobs (the tests check every one against the
 speed does. For one resolution it times the stage kernels under every combination of
   - motion-search cells per CTA (15 or 30),
   - persistent queue-draining grid or one CTA per unit,
-  - inter MV chunk (32 or 64),
+  - inter MV chunk (32 or 64: one setting to launches of more than four units an SM without keep
+    words, whose passes hold 30 at most; either may then be kept),
 on a representative job (a frame and its references already in the engine's store), with the
 engine's CUDA-event stage timing, and keeps for each stage its fastest setting: the cells per
 pyramid level, the persistent mask per stage, the inter chunk. Results can be cached in a JSON file

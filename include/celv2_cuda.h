@@ -187,15 +187,18 @@ long long celv2_kernel_launches(const celv2_engine* e);
  * How the stages run; none of it changes a decision.
  *  CELV2_CFG_PERSISTENT: 1 (default) -- each stage is one persistent kernel whose CTAs drain a
  *    device-side queue of the batch's work units (superblocks, cell groups); 0 -- one CTA per unit.
- *  CELV2_CFG_GRAPHS: 1 -- celv2_launch_group captures a batch's whole stage sequence (descriptor
- *    copy, queue resets, stage kernels) as a CUDA graph once per batch shape (the jobs' reference
- *    counts) and replays it, the record copies following it; 0 (default) -- launches stage by
- *    stage.
+ *  CELV2_CFG_GRAPHS: 1 -- celv2_launch_group captures a batch's stage kernels as a CUDA graph once
+ *    per batch shape (the jobs' reference counts, keep words and pruner use) and replays it behind
+ *    the descriptors' copy; of a batch decided in slices the kernels before them, each wave its own
+ *    graph, the slices and the record copies following. 0 (default) -- launches stage by stage.
  *  CELV2_CFG_PERSISTENT_OFF: a bit mask of stages that run one CTA per unit even when
  *    CELV2_CFG_PERSISTENT is on (bit l: motion-search level l, 5 intra, 6 inter, 7 finalize,
  *    8 level 0's quarter-pel refinement).
- *  CELV2_CFG_INTER_CHUNK: distinct MVs per pass of the inter stage at most, 8..64 (default 64; the
- *    whole-superblock kernel holds at most 30 where it runs four CTAs an SM).
+ *  CELV2_CFG_INTER_CHUNK: distinct MVs per pass of the inter stage, 8..64 (default 64). The region
+ *    pass takes at most that many. The whole-superblock kernel takes whole rounds of its window
+ *    ring: with four CTAs an SM 6, 12 .. 30 (so 30 from 30 on), with two (launches of up to four
+ *    units an SM) 12, 24 .. 60, with one (up to a unit an SM) 24 or 48; the largest of these within the
+ *    setting, at least the first.
  *  CELV2_CFG_ME_CELLS_L0 + l: 8x8 cells per motion-search CTA at pyramid level l, 15 or 30
  *    (default 30); levels too small to fill the GPU with CTAs of seven take seven.
  *  CELV2_CFG_FEATURES: 1 -- every inter frame's learned-pruner features are kept for

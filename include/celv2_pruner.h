@@ -44,7 +44,8 @@ extern "C" {
 #define CELV2_PRUNER_FEATURES 376
 #define CELV2_PRUNER_OUTPUTS 24
 #define CELV2_PRUNER_PARAMS 56120
-/* Forward activation cache, floats per sample; the logits are its last batch * 24 floats. */
+/* Forward activation cache, floats per sample; the logits are its last batch * 24 floats. (Both sizes are
+ * part of the interface; the kernels touch about 7,100 and 580 of them.) */
 #define CELV2_PRUNER_ACTS 23504
 /* Backward workspace, floats per sample. */
 #define CELV2_PRUNER_WORK 20544
