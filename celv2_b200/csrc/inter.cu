@@ -361,16 +361,14 @@ __global__ void __launch_bounds__(kInterThreads* G, 4 / G) k_inter(const FrameJo
 
   __syncthreads();  // dmap complete
   // step s's windows into ring slot `to`, by one thread, once every warp is done with the step that had
-  // the slot before; round: the parity of the step's own round (a wait that runs out marks the batch and
-  // leaves the step without windows, which ends every thread's own wait for them the same way)
+  // the slot before; round: the parity of the step's own round (a wait that runs out leaves the
+  // step without windows, which ends every thread's own wait for them; the batch is marked there alone: the loop
+  // over its jobs in each of these copies was 1.3 of 33 us of a 416x240 frame's stage)
   const void* map = job.map + r;
   auto load_step = [&](int s, unsigned to, unsigned round) {
     if (s >= steps) return;
     const unsigned bar = full_s + 8 * to;
-    if (!mbar_wait(empty_s + 8 * to, round ^ 1)) {
-      mark_fault(jobs, w);
-      return;
-    }
+    if (!mbar_wait(empty_s + 8 * to, round ^ 1)) return;
     int2 e[M];
     unsigned bytes = 0;
 #pragma unroll
