@@ -4,8 +4,10 @@ The decisions never depend on these knobs (the tests check every one against the
 speed does. For one resolution it times the stage kernels under every combination of
   - motion-search cells per CTA (15 or 30),
   - persistent queue-draining grid or one CTA per unit,
-  - inter MV chunk (32 or 64: one setting to launches of more than four units an SM without keep
-    words, whose passes hold 30 at most; either may then be kept),
+  - inter MV chunk (32 or 64; 64 only where it is faster by more than a run differs from the next:
+    without keep words a launch of more than four units an SM runs the same passes with both, while the
+    region pass of pruned batches, which the job need not have, is the faster with 32 -- 20.2 against 22.3 ms
+    of a pruned step of six 1080p mini-GOPs),
 on a representative job (a frame and its references already in the engine's store), with the
 engine's CUDA-event stage timing, and keeps for each stage its fastest setting: the cells per
 pyramid level, the persistent mask per stage, the inter chunk. Results can be cached in a JSON file
@@ -69,7 +71,8 @@ def autotune_run(eng: E.CudaEngine, run, reps: int = 3) -> dict:
         if b and not b[1]:
             chosen["persistent_off"] |= 1 << bit
         if stage == "inter" and b:
-            chosen["inter_chunk"] = b[2]
+            ms = {c: min(t[stage][0] for s, t in results if s[2] == c) for c in (32, 64)}
+            chosen["inter_chunk"] = 64 if ms[64] < 0.98 * ms[32] else 32
     for stage in STAGES_ME + ["me_refine", "intra", "inter", "finalize"]:
         chosen["stage_ms"][stage] = min(r[1][stage][0] for r in results) / reps
     apply(eng, chosen)
